@@ -169,7 +169,8 @@ def profile_traffic(kernel: str, cells: int) -> float | None:
     of the launch's region (the region depends on the CPML-band shape the
     autotuner keeps; traffic grows with it in proportion) times `cells`, or
     the per-launch figure when the summary has no per-cell one."""
-    name = ("step_tmat2_8192_production.md" if kernel.startswith("step_tmat2") else
+    name = ("step_tile_8192_production.md" if kernel.startswith("step_tmat_kernel<tile") else
+            "step_tmat2_8192_production.md" if kernel.startswith("step_tmat2") else
             "step_tmat_8192_production.md" if kernel.startswith("step_tmat") else "step_tma_8192_production.md")
     f = ROOT / "profiles" / name
     if not f.exists():

@@ -485,7 +485,7 @@ std::map<ChoiceKey, KernelChoice> g_choice;
 ChoiceKey choice_key(const fdtd2d_ctx* c, int device, const char* what) {
   std::string env = what;
   for (const char* v : {"FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_TMA", "FDTD2D_TMA_AUTOTUNE", "FDTD2D_TMAT_AUTOTUNE",
-                        "FDTD2D_KERNEL", "FDTD2D_PERSIST"}) {
+                        "FDTD2D_KERNEL", "FDTD2D_PERSIST", "FDTD2D_TILE"}) {
     const char* x = std::getenv(v);
     env += '|';
     env += x ? x : "-";
@@ -817,6 +817,117 @@ int setup_persist(fdtd2d_ctx* c, int device) {
                   c->medium == FDTD2D_MEDIUM_UNIFORM ? 0 : 1);
   }
   return FDTD2D_OK;
+}
+
+// The descriptor of a tile launch for steps after step n - 1: the current
+// state's buffers as slot 0 and psi, the others as slot 1.
+DevShot tile_view(const fdtd2d_ctx* c, int n) {
+  const int a = (n - 1) & 1;
+  DevShot t = c->h;
+  t.fb[0] = c->h.fb[a];
+  t.fb[1] = c->h.fb[a ^ 1];
+  t.psi = c->h.psi + a * c->h.psi_buf;
+  t.psi_buf = a ? -c->h.psi_buf : c->h.psi_buf;
+  return t;
+}
+
+// Four steps per pass on register tiles (step_tile.cu): every uniform-medium
+// shot whose CPML fits a tile's shared memory, unless a wave-front tracker
+// reads every step's field.  Measured on GB300 against the two-step path and
+// the persistent kernel, Gcell/s: 1024^2 180 (85), 2048^2 327 (165), 4096^2
+// 457 (249), 8192^2 553 (315), F16 4096^2 471 (281), 8192^2 585 (413).
+// The compiled shapes are timed at create (a trial reads one buffer set and
+// writes the other, as a step does) and the choice kept per class.
+// FDTD2D_TILE=0: never; FDTD2D_TILE=R: the shape with R rows per warp.  Not
+// taken when another path is forced by name.
+int setup_tile(fdtd2d_ctx* c, int device) {
+  const char* env = std::getenv("FDTD2D_TILE");
+  if (env && std::strcmp(env, "0") == 0) return FDTD2D_OK;
+  for (const char* v : {"FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_KERNEL"})
+    if (std::getenv(v)) return FDTD2D_OK;
+  if (const char* v = std::getenv("FDTD2D_PERSIST"); v && std::atoi(v) == 1) return FDTD2D_OK;
+  if (c->n_rc > 0) return FDTD2D_OK;
+  int forced = -1;
+  for (int k = 0; k < tile_shape_count(); ++k) {
+    if (!tile_fits(c->h, k, device)) return FDTD2D_OK;
+    if (env && std::atoi(env) == tile_shape_rows(k)) forced = k;
+  }
+  const ChoiceKey key = choice_key(c, device, "tile");
+  KernelChoice ch;
+  bool have = forced < 0 && find_choice(key, &ch) && ch.k >= 0 && ch.k < tile_shape_count();
+  if (have) note_choice(c, have, ch);
+  if (!have && forced < 0 && c->untimed) {
+    ch.k = c->h.store == FDTD2D_STORE_F32 ? 0 : 1;   // the shapes the timing keeps most often
+    c->choice_src = std::max(c->choice_src, 3);
+    have = true;
+  }
+  if (forced >= 0) ch.k = forced;
+  const bool timed = !have && forced < 0;
+  std::vector<int4> best;
+  int4* d_best = nullptr;
+  float best_ms = 0.f;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (timed) {
+    e = cudaEventCreate(&e0);
+    if (e == cudaSuccess) e = cudaEventCreate(&e1);
+  }
+  auto done = [&](cudaError_t x) {
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    return x == cudaSuccess ? (int)FDTD2D_OK : fail_cuda(c, x);
+  };
+  if (e != cudaSuccess) return done(e);
+  // about 0.4 ms of passes per shape, at least 3
+  const int reps = (int)std::max<int64_t>(3, std::min<int64_t>(20, (int64_t)(0.4e-3 / (1e-11 * (double)c->nx * c->ny)) + 1));
+  DevShot t = tile_view(c, 1);
+  t.record = 0;
+  t.dft = nullptr;
+  for (int k = 0; k < tile_shape_count(); ++k) {
+    if (!timed && k != ch.k) continue;
+    const std::vector<int4> tiles = make_tiles(c->h, k);
+    int4* d = nullptr;
+    e = dalloc(c, &d, tiles.size());
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(d, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) return done(e);
+    float ms = 0.f;
+    if (timed) {
+      const size_t smem = tile_smem(c->h, k);
+      const int steps = std::min(kTileSteps, c->n_steps);
+      for (int r = 0; r <= reps && e == cudaSuccess; ++r) {
+        if (r == 1) e = cudaEventRecord(e0, c->stream);
+        if (e == cudaSuccess)
+          e = launch_step_tile(k, t, d, (int)tiles.size(), smem, t.base_n + 1, steps, c->stream);
+      }
+      if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
+      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+      if (e != cudaSuccess) return done(e);
+    }
+    if (!d_best || ms < best_ms) {
+      std::swap(d, d_best);
+      best_ms = ms;
+      ch.k = k;
+      c->n_tiles = (int)tiles.size();
+    }
+    if (d) {
+      cudaFreeAsync(d, c->stream);
+      c->allocs.erase(std::find(c->allocs.begin(), c->allocs.end(), (void*)d));
+    }
+  }
+  if (timed) {
+    ch.q = 0;
+    ch.lv = kTileSteps;
+    keep_choice(key, ch);
+  }
+  c->d_tiles = d_best;
+  c->tile_shape = ch.k;
+  c->tile_smem = tile_smem(c->h, ch.k);
+  c->tile = true;
+  std::snprintf(c->kernel_name, sizeof c->kernel_name, "step_tmat_kernel<tile,%d>", tile_shape_rows(ch.k));
+  return done(cudaSuccess);
 }
 
 int setup_tmat(fdtd2d_ctx* c, int device) {
@@ -1389,7 +1500,7 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
     for (const Pt& p : pts) row_start[p.j + 1]++;
     for (int j = 0; j < ny; ++j) row_start[j + 1] += row_start[j];
     std::vector<int4> dp(std::max<size_t>(1, pts.size()));
-    for (size_t q = 0; q < pts.size(); ++q) dp[q] = make_int4(pts[q].i, pts[q].kind, pts[q].idx, 0);
+    for (size_t q = 0; q < pts.size(); ++q) dp[q] = make_int4(pts[q].i, pts[q].kind, pts[q].idx, pts[q].j);
     int* d_rs;
     int4* d_pts;
     CK(dalloc(c, &d_rs, row_start.size()));
@@ -1480,7 +1591,10 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
   }
   CK(dalloc(c, &c->d_err, 1));
   std::vector<int4> units;
-  if (c->tma) {
+  if (c->tma && !member) CK_RC(setup_tile(c, device));
+  if (c->tile) {
+    // its own tiles
+  } else if (c->tma) {
     // FDTD2D_TMA="W,ST" picks a compiled launch shape (W warps, ST stages);
     // otherwise the shapes are timed on this shot and the fastest is kept,
     // unless FDTD2D_TMA_AUTOTUNE=0 (then shape 0).
@@ -1561,10 +1675,10 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
   }
   c->n_units = (int)units.size();
   CK(dalloc(c, &c->d_units, units.size()));
-  CK(cudaMemcpyAsync(c->d_units, units.data(), units.size() * sizeof(int4), cudaMemcpyHostToDevice,
-                     c->stream));
-  if (c->tma && !member) CK_RC(setup_tmat(c, device));
-  if (!member && !solo) CK_RC(setup_persist(c, device));
+  if (!units.empty())
+    CK(cudaMemcpyAsync(c->d_units, units.data(), units.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
+  if (c->tma && !member && !c->tile) CK_RC(setup_tmat(c, device));
+  if (!member && !solo && !c->tile) CK_RC(setup_persist(c, device));
   CK(dalloc(c, &c->d_flag, 1));
   CK(cudaStreamSynchronize(c->stream));
 #undef CK
@@ -1626,6 +1740,35 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
       ++c->launches;
       c->step = m;
       n = m + 1;
+    }
+    return FDTD2D_OK;
+  }
+  if (c->tile) {
+    for (int32_t n = n_first; n <= n_last;) {
+      // single steps where something reads the fields after each of them
+      int k = std::min(kTileSteps, n_last - n + 1);
+      if (c->line_n > 0 && n <= c->line_last && n + k > c->line_first) k = n < c->line_first ? c->line_first - n : 1;
+      cudaEvent_t p0 = prof_mark(c, nullptr, 0, k);
+      cudaError_t e = launch_step_tile(c->tile_shape, tile_view(c, n), c->d_tiles, c->n_tiles, c->tile_smem, n, k,
+                                       c->stream);
+      if (p0) prof_mark(c, p0, (int64_t)c->nx * c->ny, k);
+      if (e != cudaSuccess) return fail_cuda(c, e);
+      ++c->launches;
+      if (k % 2 == 0) {
+        // an even number of steps: the buffers trade places, so that the
+        // state after step n is in slot n & 1 as everywhere else
+        std::swap(c->h.fb[0], c->h.fb[1]);
+        c->h.psi += c->h.psi_buf;
+        c->h.psi_buf = -c->h.psi_buf;
+      }
+      n += k;
+      c->step = n - 1;
+      if (c->line_n > 0 && c->step >= c->line_first && c->step <= c->line_last) {
+        e = launch_line(field_ptr(c->h, kEz, c->step & 1), c->pitch, c->line_j, c->line_i0, c->line_n,
+                        c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
+        if (e != cudaSuccess) return fail_cuda(c, e);
+        ++c->launches;
+      }
     }
     return FDTD2D_OK;
   }

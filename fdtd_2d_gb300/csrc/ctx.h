@@ -67,6 +67,11 @@ struct fdtd2d_ctx {
   // test parameters of its grid barrier (PersistAux::wait_ns, bar_extra)
   unsigned long long wait_ns = 0;
   int bar_extra = 0;
+  // several steps per pass on register tiles (step_tile.cu)
+  bool tile = false;
+  int tile_shape = 0, n_tiles = 0;
+  size_t tile_smem = 0;
+  int4* d_tiles = nullptr;
   // the CPML-band kernel runs on a second stream beside the interior one:
   // ev_t marks the interior kernel of the last step, ev_e the CPML kernel,
   // ev_m the shot stream's work before a run

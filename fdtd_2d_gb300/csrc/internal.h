@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <new>
+#include <vector>
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -55,7 +56,9 @@ struct DevShot {
   // and fb[1] (state n) on the ring cells its neighbours read.
   float* fb[4];
   int64_t cells;
-  // CPML psi slab [2 ping-pong buffers][psi_buf]; within a buffer (side s = 0
+  // CPML psi slab [2 ping-pong buffers][psi_buf] (the tile path, where an even
+  // number of steps may separate two states, lets the buffers trade places:
+  // psi then points at the second one and psi_buf is negative); within a buffer (side s = 0
   // low edge, 1 high edge):
   //   o_hxy: [s][r][pitch]  r in [0,P-2]   (Hx, y strips)
   //   o_ezy: [s][r][pitch]  r in [0,P-1]   (Ez, y strips; r = 0 unused)
@@ -80,7 +83,7 @@ struct DevShot {
 
   // sources and detectors, by row
   const int* row_start;       // [ny+1] offsets into pts
-  const int4* pts;            // (col, kind, element index, 0)
+  const int4* pts;            // (col, kind, element index, row)
   // Source waveform s_e(n) and DFT twiddles are tabulated per step by
   // build_source_tables (FP64 math, once per shot) so the step kernel does no
   // transcendental work.
@@ -252,6 +255,20 @@ cudaError_t launch_step_tmat2(int shape, const DevShot& shot, const TensorMaps& 
 // Sets *ctr = 0.
 cudaError_t launch_frame(const DevShot& shot, int ci0, int ci1, int ri0, int ri1, int n_global, int* ctr,
                          cudaStream_t stream);
+// Several steps per pass on register tiles (step_tile.cu), in shapes that
+// differ in the rows of a plain tile: tiles (flags, c0, r0, u1) of 128 columns
+// from c0 and a band of rows from r0, storing rows up to u1.  A launch reads
+// state n_global-1 from fb[0] and psi, writes state n_global-1+steps (steps <=
+// kTileSteps) to fb[1] and psi + psi_buf.  smem: tile_smem of the shot.
+constexpr int kTileSteps = 4;
+enum TileFlags : int { kTilePlain = 1 };   // no CPML and no border in the tile
+int tile_shape_count();
+int tile_shape_rows(int shape);   // rows per warp of its plain tiles
+std::vector<int4> make_tiles(const DevShot& s, int shape);
+size_t tile_smem(const DevShot& s, int shape);
+bool tile_fits(const DevShot& s, int shape, int device);
+cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
+                             int steps, cudaStream_t stream);
 // Launches the instantiation for shot.store.
 cudaError_t launch_step_tma(int shape, const DevShot& shot, const int4* units, int n_units, int n_global,
                             int max_ctas, int* err, cudaStream_t stream);

@@ -1,0 +1,309 @@
+// Several time steps per pass over the fields, a tile at a time in registers
+// (uniform medium, the CPML included).
+//
+// step_tmat_kernel<Tile<R>, ...>: a CTA of 8 warps loads a tile of 128 columns
+// x 8 R rows of state n, steps it up to kTileSteps = 4 times in registers
+// (tile_common.cuh) and stores state n+4 of the part that no step has eaten
+// into: a cell at distance d from the tile's edge is right for d steps, so 4
+// columns and 4 rows on every side are read again by the neighbouring tiles.
+// Tiles read one buffer and write the other, so nothing orders them but the
+// launch: one launch per four steps, where the two-step path took four per
+// two (interior, CPML bands twice, frame).
+//
+// Why this shape: 4 columns of halo are one lane, so every access stays a
+// whole vector; the rows are what registers allow at 2 CTAs per SM (128 per
+// thread: while one CTA loads or stores, the other computes), which with Jz in
+// shared memory is 7 (FP32) or 5 to 7 (16-bit, whose rounding takes registers).  Tiles
+// with CPML work keep 4 rows per warp and their psi in shared memory.
+//
+// Bytes: 20 x (halo) + 16 per stored cell and 4 steps, 10.1 B per cell-update
+// with R = 7 (the two-step path 18).  Measured on GB300 against that path,
+// Gcell/s: 8192^2 FP32 553 (315), F16 585 (413); 4096^2 457 (249) and 471
+// (281); 2048^2 327 (165).  R = 4 (Jz in registers) 504, 5 491, 6 520, 8 485
+// at 8192^2 FP32.  FP32 moves 5.6 TB/s of tile traffic there, 0.82 of the copy
+// peak; 16-bit storage is bound by its instructions.
+#include <algorithm>
+
+#include "internal.h"
+#include "tile_common.cuh"
+
+namespace fdtd2d {
+
+namespace {
+
+constexpr int kHalo = kTileSteps;                 // columns and rows around the stored part
+constexpr int kUse = kTileCols - 2 * kHalo;       // stored columns of a tile
+constexpr int kWarps = 8;
+constexpr int kREdge = 4;                         // rows per warp of a tile with CPML work
+constexpr int kRowsEdge = kREdge * kWarps;
+// Rows per warp of the plain tiles, by shape (Jz in shared memory).
+constexpr int kShapes[] = {7, 5};
+constexpr int kNumShapes = 2;
+
+// psi of the tile from (store = false) or to the slab, the owned cells only
+// when stored: columns of lanes [l0, l1], rows [u0, u1).
+template <int R, bool STORE>
+__device__ __forceinline__ void tile_psi_io(const DevShot& S, float* slab, const TilePos& p, const TilePsi& psi, int rows,
+                                            int row0, int warp, int lane, bool own, int u0, int u1) {
+  const int nx = S.nx, ny = S.ny, P = S.npml;
+  const int64_t pitch = S.pitch;
+#pragma unroll
+  for (int r = -1; r < R; ++r) {
+    const int j = p.j0 + r;
+    if (j < 0 || j > ny - 1 || (STORE && (r < 0 || j < u0 || j >= u1 || !own))) continue;
+    // x strips: Hy, Ez
+    if (r >= 0 && (p.xh | p.xe)) {
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        float4* ps = psi.x + (f * rows + row0 + r) * p.nxl + p.xslot;
+        float v[4];
+        if (STORE) get4(v, *ps); else zero4(v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (!((f ? p.xe : p.xh) >> k & 1)) continue;
+          const int c = p.i + k;
+          const int side = c >= P ? 1 : 0, q = side ? nx - (f ? 1 : 2) - c : c;
+          float* g = slab + (f ? S.o_ezx : S.o_hyx) + ((int64_t)side * ny + j) * P + q;
+          if (STORE) *g = v[k]; else v[k] = __ldcg(g);
+        }
+        if (!STORE) *ps = put4(v);
+      }
+    }
+    // y strips: Hx, Ez (a thread left of column 0 holds no strip cell)
+    const bool in = p.i >= 0 && p.i < nx;
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      if (r < 0 && f) continue;
+      if (!(f ? y_strip_e(j, ny, P) : y_strip_h(j, ny, P))) continue;
+      const int side = j >= P ? 1 : 0, q = side ? ny - (f ? 1 : 2) - j : j;
+      float* g = slab + (f ? S.o_ezy + ((int64_t)side * P + q) * pitch : ((int64_t)side * (P - 1) + q) * pitch) + p.i;
+      float4* ps = r < 0 ? psi.b + warp * 32 + lane : psi.y + (f * p.nyl + j - (j < P ? p.ylo : p.yhi)) * 32 + lane;
+      if (STORE) {
+        if (in) *reinterpret_cast<float4*>(g) = *ps;
+      } else {
+        *ps = in ? __ldcg(reinterpret_cast<const float4*>(g)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+  }
+}
+
+template <class T>
+__device__ __forceinline__ void load4(float (&d)[4], const T* p, bool in) {
+  if (in) {
+    Sto<T>::ldg4(d, p);
+  } else {
+    zero4(d);
+  }
+}
+
+template <int R, int NW, bool JS, bool LOSSLESS, bool PLAIN, class T>
+__device__ __forceinline__ void tile_pass(const DevShot& S, const int4 tile, int n, int steps, float4* smem) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int rows = NW * R, threads = NW * 32;
+  const int c0 = tile.y, r0 = tile.z, u0 = max(r0 + kHalo, 0), u1 = tile.w;
+  const int nx = S.nx, ny = S.ny;
+  const int64_t pitch = S.pitch;
+  const int row0 = warp * R, j0 = r0 + row0;
+  const TilePos p = tile_pos(S, c0, r0, rows, j0, lane, PLAIN);
+  const Coef<T> C(S);
+  float4* ex = smem;                                   // [2][NW][2][32]
+  float4* kps = ex + 4 * NW * 32 + tid;                // [R][threads]
+  float4* jzs = kps + R * threads;                     // [R][threads] where JS
+  float4* rest = ex + 4 * NW * 32 + (JS ? 2 : 1) * R * threads;
+  const TilePsi psi = tile_psi(rest, p, rows);
+  float* tc = PLAIN ? nullptr : reinterpret_cast<float*>(psi.b + NW * 32);
+  float* tr = PLAIN ? nullptr : tc + kTcRows * kTileCols;
+
+  TileRegs<R, JS> s;
+  {
+    const bool in = PLAIN || (p.i >= 0 && p.i < nx);
+    const T* ez = field_ptr_t<T>(S, kEz, 0) + p.i;
+    const T* hx = field_ptr_t<T>(S, kHx, 0) + p.i;
+    const T* hy = field_ptr_t<T>(S, kHy, 0) + p.i;
+    const T* jz = field_ptr_t<T>(S, kJz, 0) + p.i;
+    const T* kp = reinterpret_cast<const T*>(S.kp);
+    load4(s.hx[0], hx + (int64_t)(j0 - 1) * pitch, in && (PLAIN || (j0 >= 1 && j0 <= ny)));
+    float kv[R][4], jv[JS ? R : 1][4];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = j0 + r;
+      const bool ok = in && (PLAIN || (j >= 0 && j < ny));
+      const int64_t o = (int64_t)j * pitch;
+      load4(s.ez[r + 1], ez + o, ok);
+      load4(s.hx[r + 1], hx + o, ok);
+      load4(s.hy[r], hy + o, ok);
+      if (JS) load4(jv[r], jz + o, ok); else load4(s.jz[JS ? 0 : r], jz + o, ok);
+      load4(kv[r], kp + p.i + o, ok && kp != nullptr);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (sizeof(T) == 2) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) kv[r][k] = __fmul_rn(kv[r][k], C.rk);
+      }
+      kps[r * threads] = put4(kv[r]);
+      if (JS) jzs[r * threads] = put4(jv[JS ? r : 0]);
+    }
+  }
+  if (!PLAIN) {
+    tile_tables(S, tc, tr, c0, r0, rows, tid, threads);
+    tile_psi_io<R, false>(S, S.psi, p, psi, rows, row0, warp, lane, false, 0, 0);
+  }
+  // lanes whose columns are stored
+  const bool own = lane >= kHalo / 4 && lane < 32 - kHalo / 4 && p.i < nx;
+  int p0 = 0, p1 = 0;
+  if (j0 + R > 0 && j0 < ny) {
+    p0 = __ldg(S.row_start + max(j0, 0));
+    p1 = __ldg(S.row_start + min(j0 + R, ny));
+  }
+  for (int t = 0; t < steps; ++t) {
+    float4* e = ex + (t & 1) * 2 * NW * 32;
+    e[(2 * warp) * 32 + lane] = put4(s.ez[1]);
+    e[(2 * warp + 1) * 32 + lane] = put4(s.ez[R]);
+    __syncthreads();
+    // the tile's first and last rows have no neighbour here: any value does
+    get4(s.ez[0], e[(warp > 0 ? 2 * warp - 1 : 0) * 32 + lane]);
+    get4(s.ez[R + 1], e[(warp < NW - 1 ? 2 * warp + 2 : 2 * warp + 1) * 32 + lane]);
+    tile_step<R, JS, LOSSLESS, PLAIN, T>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, threads, warp, lane);
+    if (p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, own, u0, u1);
+    tile_round<R, JS, T>(s);
+  }
+  if (own) {
+    T* ez = field_ptr_t<T>(S, kEz, 1) + p.i;
+    T* hx = field_ptr_t<T>(S, kHx, 1) + p.i;
+    T* hy = field_ptr_t<T>(S, kHy, 1) + p.i;
+    T* jz = field_ptr_t<T>(S, kJz, 1) + p.i;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = j0 + r;
+      if (j < u0 || j >= u1) continue;
+      const int64_t o = (int64_t)j * pitch;
+      Sto<T>::stcs4(ez + o, s.ez[r + 1]);
+      Sto<T>::stcs4(hx + o, s.hx[r + 1]);
+      Sto<T>::stcs4(hy + o, s.hy[r]);
+      if (JS) {
+        float v[4];
+        get4(v, jzs[r * threads]);
+        Sto<T>::stcs4(jz + o, v);
+      } else {
+        Sto<T>::stcs4(jz + o, s.jz[JS ? 0 : r]);
+      }
+    }
+  }
+  if (!PLAIN) tile_psi_io<R, true>(S, S.psi + S.psi_buf, p, psi, rows, row0, warp, lane, own, u0, u1);
+}
+
+template <int RP>
+struct Tile {
+  static constexpr int kRows = RP;
+};
+
+template <class Shape, bool LOSSLESS, class T>
+__global__ void __launch_bounds__(kWarps * 32, 2)
+step_tmat_kernel(const __grid_constant__ DevShot S, const int4* __restrict__ tiles, int n_global, int steps) {
+  extern __shared__ float4 smem[];
+  const int4 tile = __ldg(tiles + blockIdx.x);
+  const int n = n_global - S.base_n;
+  if (tile.x & kTilePlain) {
+    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, T>(S, tile, n, steps, smem);
+  } else {
+    tile_pass<kREdge, kWarps, false, LOSSLESS, false, T>(S, tile, n, steps, smem);
+  }
+}
+
+bool lossless(const DevShot& s) { return s.ca == 1.f && s.da == 1.f; }
+
+template <int RP, class T>
+const void* tile_kernel(const DevShot& s) {
+  return lossless(s) ? (const void*)step_tmat_kernel<Tile<RP>, true, T> : (const void*)step_tmat_kernel<Tile<RP>, false, T>;
+}
+template <int RP>
+const void* tile_kernel(const DevShot& s) {
+  return s.store == 0 ? tile_kernel<RP, float>(s) : s.store == 1 ? tile_kernel<RP, __half>(s) : tile_kernel<RP, __nv_bfloat16>(s);
+}
+const void* tile_kernel(int shape, const DevShot& s) {
+  return shape == 0 ? tile_kernel<kShapes[0]>(s) : tile_kernel<kShapes[1]>(s);
+}
+
+// Strip lanes of a 128-column tile at c0, and strip rows of `rows` rows from r0.
+int strip_lanes(const DevShot& s, int c0) {
+  int n = 0;
+  for (int l = 0; l < 32; ++l) {
+    bool any = false;
+    for (int k = 0; k < 4; ++k) {
+      const int c = c0 + 4 * l + k;
+      any = any || (c >= 0 && c <= s.npml - 1) || (c >= s.nx - s.npml && c <= s.nx - 2);
+    }
+    n += any;
+  }
+  return n;
+}
+int strip_rows(const DevShot& s, int r0, int rows) {
+  int n = 0;
+  for (int j = r0; j < r0 + rows; ++j) n += (j >= 0 && j <= s.npml - 1) || (j >= s.ny - s.npml && j <= s.ny - 2);
+  return n;
+}
+
+}  // namespace
+
+int tile_shape_count() { return kNumShapes; }
+int tile_shape_rows(int shape) { return kShapes[shape]; }
+
+// Tiles over the grid: plain ones where a whole tile and its halo lie inside
+// the CPML, the others (slower: first) over the rest.
+std::vector<int4> make_tiles(const DevShot& s, int shape) {
+  const int nx = s.nx, ny = s.ny, P = s.npml, ue = kRowsEdge - 2 * kHalo, up = kShapes[shape] * kWarps - 2 * kHalo;
+  std::vector<int4> edge, plain;
+  auto add = [&](std::vector<int4>& v, int f, int ca, int cb, int ra, int rb, int use_r) {
+    for (int r = ra; r < rb; r += use_r)
+      for (int c = ca; c < cb; c += kUse) v.push_back(make_int4(f, c - kHalo, r - kHalo, std::min(r + use_r, rb)));
+  };
+  // plain columns [xa, xb): tiles whose 128 columns have no CPML; plain rows
+  // [ya, yb) likewise (a tile reads one row below its first)
+  const int xa = (P + kHalo + kUse - 1) / kUse * kUse;
+  const int nxp = (nx - P - kHalo - xa) / kUse;
+  const int ya = P + 1 + kHalo, yb = ny - P - kHalo;
+  if (!s.den_uniform || nxp < 1 || yb - ya < up) {
+    add(edge, 0, 0, nx, 0, ny - 1, ue);
+    return edge;
+  }
+  const int xb = xa + nxp * kUse;
+  const int yc = ya + (yb - ya) / up * up;   // whole plain tiles only: a short one would read into the strip
+  add(edge, 0, 0, nx, 0, ya, ue);
+  add(edge, 0, 0, nx, yc, ny - 1, ue);
+  add(edge, 0, 0, xa, ya, yc, ue);
+  add(edge, 0, xb, nx, ya, yc, ue);
+  add(plain, kTilePlain, xa, xb, ya, yc, up);
+  edge.insert(edge.end(), plain.begin(), plain.end());
+  return edge;
+}
+
+size_t tile_smem(const DevShot& s, int shape) {
+  int nxl = 0, nyl = 0;
+  for (int c = 0; c < s.nx; c += kUse) nxl = std::max(nxl, strip_lanes(s, c - kHalo));
+  for (int r = 0; r < s.ny - 1; ++r) nyl = std::max(nyl, strip_rows(s, r - kHalo, kRowsEdge));
+  const size_t ex = 4 * kWarps * 32;
+  const size_t edge = ex + kREdge * kWarps * 32 + 2 * (size_t)kRowsEdge * nxl + 2 * (size_t)nyl * 32 + kWarps * 32;
+  const size_t plain = ex + 2 * (size_t)kShapes[shape] * kWarps * 32;
+  return std::max(edge * 16 + ((size_t)kTcRows * kTileCols + (size_t)kTcRows * (kRowsEdge + 1)) * 4, plain * 16);
+}
+
+bool tile_fits(const DevShot& s, int shape, int device) {
+  int most = 0;
+  cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  // (Hx and Hy share one scale: the stored-unit arithmetic takes it so)
+  return (s.store == 0 || s.sc[1] == s.sc[2]) && tile_smem(s, shape) <= (size_t)most;
+}
+
+cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
+                             int steps, cudaStream_t stream) {
+  if (steps < 1 || steps > kTileSteps || n_tiles <= 0) return cudaErrorInvalidValue;
+  const void* fn = tile_kernel(shape, shot);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  DevShot s = shot;
+  void* args[] = {&s, (void*)&tiles, &n_global, &steps};
+  return cudaLaunchKernel(fn, dim3(n_tiles), dim3(kWarps * 32), args, smem, stream);
+}
+
+}  // namespace fdtd2d

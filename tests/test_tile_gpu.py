@@ -1,0 +1,86 @@
+"""The register-tile kernel (several time steps per pass, csrc/step_tile.cu)
+against the one-row kernel: the same bits in every field, psi array, trace and
+DFT sum.  Grids: no plain tile at all, exactly one, widths and heights around
+whole tiles, CPMLs of 2 to 40 cells, no plasma, lossy media; points on tile
+edges; run calls of 1 to 32 steps (odd and even, so the buffers trade places)."""
+import numpy as np
+import pytest
+
+import fdtd_2d_gb300 as F
+from helpers import FIELDS, PSI_FIELDS, load_state, random_state
+
+pytestmark = pytest.mark.gpu
+
+CHUNKS = (1, 4, 2, 11, 3, 8, 32)
+STEPS = sum(CHUNKS)
+
+
+def _stepped(gpu, prob, st, chunks):
+    with F.Shot(prob, gpu) as shot:
+        name = shot.kernel_name()
+        load_state([shot], st)
+        n = 1
+        for c in chunks:
+            shot.run(n, n + c - 1)
+            n += c
+        out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+        out["det"] = shot.traces()["det_ez"]
+        out["dft"] = shot.dft()
+        shot.synchronize()
+    return name, out
+
+
+@pytest.mark.parametrize("rows", ["7", "5"])
+@pytest.mark.parametrize("nx,ny,P,store,profile,ca", [
+    (40, 40, 2, 0, 1, 1.0), (120, 25, 3, 0, 1, 1.0), (121, 24, 4, 0, 0, 1.0), (203, 157, 7, 0, 1, 0.999),
+    (371, 75, 3, 0, 1, 1.0), (372, 76, 3, 0, 3, 1.0), (1100, 90, 9, 0, 1, 1.0), (500, 400, 40, 0, 1, 1.0),
+    (777, 601, 17, 0, 3, 0.998), (640, 330, 24, 1, 1, 1.0), (333, 257, 16, 2, 1, 0.999), (900, 700, 32, 1, 3, 1.0)])
+def test_tile_equals_one_row(gpu, monkeypatch, rows, nx, ny, P, store, profile, ca):
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST"):
+        monkeypatch.delenv(v, raising=False)
+    prob = F.Problem.from_spec(nx=nx, ny=ny, npml=P, n_steps=STEPS, profile=profile, x_lo=nx // 3, x_hi=nx - 3,
+                               x_center=nx / 2, width=nx / 8, grf_rms=0.05, grf_corr=8, ne_peak=2e19, nu=3e9, n_elem=5,
+                               src_i=nx // 2 - 6, src_j=ny // 2, src_di=3, src_dj=1, n_det=6, det_i=nx // 2 - 8,
+                               det_j=ny // 2 - 2, det_di=2, det_dj=1, storage=store, field_max=16.0)
+    prob.setup.ca = prob.setup.da = ca
+    st = random_state(None, nx, ny, P, np.random.default_rng(nx))
+    monkeypatch.setenv("FDTD2D_TILE", rows)
+    name, got = _stepped(gpu, prob, st, CHUNKS)
+    assert name == f"step_tmat_kernel<tile,{rows}>", name
+    monkeypatch.delenv("FDTD2D_TILE")
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv("FDTD2D_TMA", "4,3")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = _stepped(gpu, prob, st, (STEPS,))
+    assert name == "step_tma_kernel<4,3>", name
+    for k in ref:
+        assert np.array_equal(ref[k], got[k]), k
+
+
+def test_tile_line_probe_and_components(gpu, monkeypatch):
+    """A line-probe window opening and closing inside passes, and component
+    detectors: single steps where the probe reads, four at a time elsewhere."""
+    nx, ny, P = 400, 301, 11
+    prob = F.Problem.from_spec(nx=nx, ny=ny, npml=P, n_steps=50, x_lo=nx // 3, x_hi=nx - 3, src_i=200, src_j=150,
+                               det_i=203, det_j=151, n_det=3, det_di=5)
+    s = prob.setup
+    s.line_n, s.line_i0, s.line_j, s.line_first, s.line_last = 300, 50, 140, 15, 22
+    s.n_comp, s.comp = s.n_det, s.det
+
+    def stepped():
+        with F.Shot(prob, gpu) as shot:
+            shot.run(1, 33)
+            shot.run(34, 50)
+            return shot.kernel_name(), [shot.line(15, 22)] + list(shot.traces().values()) + [shot.read_field("ez")]
+
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST"):
+        monkeypatch.delenv(v, raising=False)
+    monkeypatch.setenv("FDTD2D_TILE", "7")
+    name, got = stepped()
+    assert name == "step_tmat_kernel<tile,7>"
+    monkeypatch.setenv("FDTD2D_TILE", "0")
+    monkeypatch.setenv("FDTD2D_KERNEL", "stream")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    _, ref = stepped()
+    for a, b in zip(got, ref):
+        assert np.array_equal(a, b)
