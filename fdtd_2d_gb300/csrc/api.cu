@@ -708,6 +708,8 @@ bool material_as_uniform(const fdtd2d_setup* s, double beta, float* ca, float* c
 constexpr int64_t kPersistMaxCells = int64_t(1) << 22;
 // Steps per persistent launch (a launch of a few tens of ms at most).
 constexpr int kPersistSteps = 4096;
+// Steps from which a run call is worth loading the shot on chip.
+constexpr int kResidentSteps = 8;
 
 // Persistent launches of every shot of this process on a device run one at a
 // time: each waits for the previous one (on whichever stream it ran) and
@@ -716,8 +718,9 @@ constexpr int kPersistSteps = 4096;
 std::mutex g_persist_mu;
 cudaEvent_t g_persist_last[64] = {};
 
-cudaError_t launch_persist_ordered(fdtd2d_ctx* c, const DevShot& t, int32_t n, int32_t m, int repeat,
-                                   const PersistAux& A) {
+// One persistent launch after the device's earlier ones.
+template <class Launch>
+cudaError_t launch_ordered(fdtd2d_ctx* c, const Launch& launch) {
   if (c->device < 0 || c->device >= 64) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(g_persist_mu);
   cudaEvent_t& last = g_persist_last[c->device];
@@ -727,11 +730,17 @@ cudaError_t launch_persist_ordered(fdtd2d_ctx* c, const DevShot& t, int32_t n, i
   } else {
     e = cudaStreamWaitEvent(c->stream, last, 0);
   }
-  if (e == cudaSuccess)
-    e = launch_step_persist(t, c->d_punits, c->n_punits, n, m, repeat, A, c->medium, c->persist_ctas, c->d_bar,
-                            c->d_err, c->stream);
+  if (e == cudaSuccess) e = launch();
   if (e == cudaSuccess) e = cudaEventRecord(last, c->stream);
   return e;
+}
+
+cudaError_t launch_persist_ordered(fdtd2d_ctx* c, const DevShot& t, int32_t n, int32_t m, int repeat,
+                                   const PersistAux& A) {
+  return launch_ordered(c, [&] {
+    return launch_step_persist(t, c->d_punits, c->n_punits, n, m, repeat, A, c->medium, c->persist_ctas, c->d_bar,
+                               c->d_err, c->stream);
+  });
 }
 
 // The persistent form: FP32 single shots of at most kPersistMaxCells cells
@@ -831,6 +840,26 @@ DevShot tile_view(const fdtd2d_ctx* c, int n) {
   return t;
 }
 
+// The whole shot on chip (step_resident.cu) for run calls of at least
+// kResidentSteps steps, wherever it fits (FP32, up to ~1.6 M cells): faster than
+// the tile passes at every size that fits (4.16 against 6.19 us per step at 500 x
+// 3000, 2.87 against 5.12 at 1024^2).  Not for a batch's solo members, whose
+// launches share the GPU.  FDTD2D_RESIDENT=0 (or FDTD2D_PERSIST=0, or FDTD2D_TILE
+// naming the tiles): never; FDTD2D_RESIDENT=R: with R rows per warp only.
+int setup_resident(fdtd2d_ctx* c, int device) {
+  const char* env = std::getenv("FDTD2D_RESIDENT");
+  if (c->solo || std::getenv("FDTD2D_PERSIST") || std::getenv("FDTD2D_TILE")) return FDTD2D_OK;
+  for (const int R : resident_rows()) {
+    if (env && std::atoi(env) != R) continue;
+    if (!resident_plan(c->h, c->points, R, device, &c->rplan)) continue;
+    const cudaError_t e = dalloc(c, &c->d_link, (size_t)c->rplan.link_words);
+    if (e != cudaSuccess) return fail_cuda(c, e);
+    c->resident = true;
+    break;
+  }
+  return FDTD2D_OK;
+}
+
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
 // shot whose CPML fits a tile's shared memory, unless a wave-front tracker
 // reads every step's field.  Measured on GB300 against the two-step path and
@@ -852,10 +881,17 @@ int setup_tile(fdtd2d_ctx* c, int device) {
     if (!tile_fits(c->h, k, device)) return FDTD2D_OK;
     if (env && std::atoi(env) == tile_shape_rows(k)) forced = k;
   }
+  const int rc = setup_resident(c, device);
+  if (rc) return rc;
   const ChoiceKey key = choice_key(c, device, "tile");
   KernelChoice ch;
-  bool have = forced < 0 && find_choice(key, &ch) && ch.k >= 0 && ch.k < tile_shape_count();
+  // (a resident shot's tiles serve its short run calls only: not timed)
+  bool have = forced < 0 && !c->resident && find_choice(key, &ch) && ch.k >= 0 && ch.k < tile_shape_count();
   if (have) note_choice(c, have, ch);
+  if (c->resident) {
+    ch.k = 0;
+    have = true;
+  }
   if (!have && forced < 0 && c->untimed) {
     ch.k = c->h.store == FDTD2D_STORE_F32 ? 0 : 1;   // the shapes the timing keeps most often
     c->choice_src = std::max(c->choice_src, 3);
@@ -926,7 +962,10 @@ int setup_tile(fdtd2d_ctx* c, int device) {
   c->tile_shape = ch.k;
   c->tile_smem = tile_smem(c->h, ch.k);
   c->tile = true;
-  std::snprintf(c->kernel_name, sizeof c->kernel_name, "step_tmat_kernel<tile,%d>", tile_shape_rows(ch.k));
+  if (c->resident)
+    std::snprintf(c->kernel_name, sizeof c->kernel_name, "step_persist_kernel<0>/tile<%d>", c->rplan.R);
+  else
+    std::snprintf(c->kernel_name, sizeof c->kernel_name, "step_tmat_kernel<tile,%d>", tile_shape_rows(ch.k));
   return done(cudaSuccess);
 }
 
@@ -1496,6 +1535,7 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
       if (a.kind != b.kind) return a.kind < b.kind;
       return a.i < b.i;
     });
+    for (const Pt& p : pts) c->points.push_back(make_int3(p.i, p.j, p.kind));
     std::vector<int> row_start(ny + 1, 0);
     for (const Pt& p : pts) row_start[p.j + 1]++;
     for (int j = 0; j < ny; ++j) row_start[j + 1] += row_start[j];
@@ -1746,11 +1786,17 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
   if (c->tile) {
     for (int32_t n = n_first; n <= n_last;) {
       // single steps where something reads the fields after each of them
-      int k = std::min(kTileSteps, n_last - n + 1);
+      int k = n_last - n + 1;
       if (c->line_n > 0 && n <= c->line_last && n + k > c->line_first) k = n < c->line_first ? c->line_first - n : 1;
+      const bool resident = c->resident && k >= kResidentSteps;
+      k = std::min(k, resident ? kPersistSteps : kTileSteps);
       cudaEvent_t p0 = prof_mark(c, nullptr, 0, k);
-      cudaError_t e = launch_step_tile(c->tile_shape, tile_view(c, n), c->d_tiles, c->n_tiles, c->tile_smem, n, k,
-                                       c->stream);
+      const DevShot t = tile_view(c, n);
+      const cudaError_t e =
+          resident ? launch_ordered(c, [&] {
+            return launch_resident(t, c->rplan, n, k, c->d_link, c->d_err, c->wait_ns, c->bar_extra, c->stream);
+          })
+                   : launch_step_tile(c->tile_shape, t, c->d_tiles, c->n_tiles, c->tile_smem, n, k, c->stream);
       if (p0) prof_mark(c, p0, (int64_t)c->nx * c->ny, k);
       if (e != cudaSuccess) return fail_cuda(c, e);
       ++c->launches;
@@ -1764,9 +1810,9 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
       n += k;
       c->step = n - 1;
       if (c->line_n > 0 && c->step >= c->line_first && c->step <= c->line_last) {
-        e = launch_line(field_ptr(c->h, kEz, c->step & 1), c->pitch, c->line_j, c->line_i0, c->line_n,
-                        c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
-        if (e != cudaSuccess) return fail_cuda(c, e);
+        const cudaError_t x = launch_line(field_ptr(c->h, kEz, c->step & 1), c->pitch, c->line_j, c->line_i0, c->line_n,
+                                          c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
+        if (x != cudaSuccess) return fail_cuda(c, x);
         ++c->launches;
       }
     }

@@ -72,6 +72,11 @@ struct fdtd2d_ctx {
   int tile_shape = 0, n_tiles = 0;
   size_t tile_smem = 0;
   int4* d_tiles = nullptr;
+  // the whole shot on chip for a run call's steps (step_resident.cu), beside the tiles
+  bool resident = false;
+  fdtd2d::ResidentPlan rplan{};
+  uint64_t* d_link = nullptr;
+  std::vector<int3> points;   // (column, row, kind) of the shot's sources and detectors
   // the CPML-band kernel runs on a second stream beside the interior one:
   // ev_t marks the interior kernel of the last step, ev_e the CPML kernel,
   // ev_m the shot stream's work before a run

@@ -269,6 +269,27 @@ size_t tile_smem(const DevShot& s, int shape);
 bool tile_fits(const DevShot& s, int shape, int device);
 cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
                              int steps, cudaStream_t stream);
+// The whole shot in the SMs' registers for many steps (step_resident.cu): nb
+// bands of w columns, each cut into strips of groups of R rows (a warp's).
+// The first and last band, whose columns hold the x strips, and the others
+// have their own cuts: strip k of a band is groups [start[t][k],
+// start[t][k+1]), t = 0 for the edge bands.  A launch reads state n_global-1
+// and writes state n_global-1+steps as launch_step_tile does.  link:
+// link_words words of the shot's own.  tag_add != 0 makes every wait run out
+// after wait_ns (the test of that).
+constexpr int kMaxStrips = 256;
+struct ResidentPlan {
+  int R, nb, w, groups, nw, smem;       // nw: most groups in a strip
+  int point_warps;                      // most warps of a CTA with sources or detectors
+  int ns[2];                            // strips per band
+  uint16_t start[2][kMaxStrips + 1];
+  int64_t link_words;
+};
+const std::vector<int>& resident_rows();
+// points: (column, row, PointKind) of the shot's sources and detectors.
+bool resident_plan(const DevShot& s, const std::vector<int3>& points, int R, int device, ResidentPlan* out);
+cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n_global, int steps, uint64_t* link, int* err,
+                            unsigned long long wait_ns, int tag_add, cudaStream_t stream);
 // Launches the instantiation for shot.store.
 cudaError_t launch_step_tma(int shape, const DevShot& shot, const int4* units, int n_units, int n_global,
                             int max_ctas, int* err, cudaStream_t stream);

@@ -40,53 +40,6 @@ constexpr int kRowsEdge = kREdge * kWarps;
 constexpr int kShapes[] = {7, 5};
 constexpr int kNumShapes = 2;
 
-// psi of the tile from (store = false) or to the slab, the owned cells only
-// when stored: columns of lanes [l0, l1], rows [u0, u1).
-template <int R, bool STORE>
-__device__ __forceinline__ void tile_psi_io(const DevShot& S, float* slab, const TilePos& p, const TilePsi& psi, int rows,
-                                            int row0, int warp, int lane, bool own, int u0, int u1) {
-  const int nx = S.nx, ny = S.ny, P = S.npml;
-  const int64_t pitch = S.pitch;
-#pragma unroll
-  for (int r = -1; r < R; ++r) {
-    const int j = p.j0 + r;
-    if (j < 0 || j > ny - 1 || (STORE && (r < 0 || j < u0 || j >= u1 || !own))) continue;
-    // x strips: Hy, Ez
-    if (r >= 0 && (p.xh | p.xe)) {
-#pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        float4* ps = psi.x + (f * rows + row0 + r) * p.nxl + p.xslot;
-        float v[4];
-        if (STORE) get4(v, *ps); else zero4(v);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (!((f ? p.xe : p.xh) >> k & 1)) continue;
-          const int c = p.i + k;
-          const int side = c >= P ? 1 : 0, q = side ? nx - (f ? 1 : 2) - c : c;
-          float* g = slab + (f ? S.o_ezx : S.o_hyx) + ((int64_t)side * ny + j) * P + q;
-          if (STORE) *g = v[k]; else v[k] = __ldcg(g);
-        }
-        if (!STORE) *ps = put4(v);
-      }
-    }
-    // y strips: Hx, Ez (a thread left of column 0 holds no strip cell)
-    const bool in = p.i >= 0 && p.i < nx;
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      if (r < 0 && f) continue;
-      if (!(f ? y_strip_e(j, ny, P) : y_strip_h(j, ny, P))) continue;
-      const int side = j >= P ? 1 : 0, q = side ? ny - (f ? 1 : 2) - j : j;
-      float* g = slab + (f ? S.o_ezy + ((int64_t)side * P + q) * pitch : ((int64_t)side * (P - 1) + q) * pitch) + p.i;
-      float4* ps = r < 0 ? psi.b + warp * 32 + lane : psi.y + (f * p.nyl + j - (j < P ? p.ylo : p.yhi)) * 32 + lane;
-      if (STORE) {
-        if (in) *reinterpret_cast<float4*>(g) = *ps;
-      } else {
-        *ps = in ? __ldcg(reinterpret_cast<const float4*>(g)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-  }
-}
-
 template <class T>
 __device__ __forceinline__ void load4(float (&d)[4], const T* p, bool in) {
   if (in) {
@@ -104,15 +57,15 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const int4 tile, int
   const int nx = S.nx, ny = S.ny;
   const int64_t pitch = S.pitch;
   const int row0 = warp * R, j0 = r0 + row0;
-  const TilePos p = tile_pos(S, c0, r0, rows, j0, lane, PLAIN);
+  const TilePos p = tile_pos(S, c0, r0, R, warp, lane);
   const Coef<T> C(S);
   float4* ex = smem;                                   // [2][NW][2][32]
   float4* kps = ex + 4 * NW * 32 + tid;                // [R][threads]
   float4* jzs = kps + R * threads;                     // [R][threads] where JS
   float4* rest = ex + 4 * NW * 32 + (JS ? 2 : 1) * R * threads;
-  const TilePsi psi = tile_psi(rest, p, rows);
-  float* tc = PLAIN ? nullptr : reinterpret_cast<float*>(psi.b + NW * 32);
-  float* tr = PLAIN ? nullptr : tc + kTcRows * kTileCols;
+  float* tc = reinterpret_cast<float*>(rest);          // the tables and psi of a tile with CPML work
+  float* tr = tc + kTcRows * kTileCols;
+  const TilePsi psi = tile_psi(rest + tile_table_f4(rows), p, rows, R, lane);
 
   TileRegs<R, JS> s;
   {
@@ -146,28 +99,35 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const int4 tile, int
     }
   }
   if (!PLAIN) {
-    tile_tables(S, tc, tr, c0, r0, rows, tid, threads);
-    tile_psi_io<R, false>(S, S.psi, p, psi, rows, row0, warp, lane, false, 0, 0);
+    tile_tables<T>(S, C, tc, tr, c0, r0, rows, tid, threads);
+    tile_psi_io<R, false, true>(S, S.psi, p, psi, rows, row0, 0, 0, 0);
   }
   // lanes whose columns are stored
-  const bool own = lane >= kHalo / 4 && lane < 32 - kHalo / 4 && p.i < nx;
+  const unsigned own = lane >= kHalo / 4 && lane < 32 - kHalo / 4 && p.i < nx ? 15u : 0u;
   int p0 = 0, p1 = 0;
   if (j0 + R > 0 && j0 < ny) {
     p0 = __ldg(S.row_start + max(j0, 0));
     p1 = __ldg(S.row_start + min(j0 + R, ny));
   }
-  for (int t = 0; t < steps; ++t) {
-    float4* e = ex + (t & 1) * 2 * NW * 32;
-    e[(2 * warp) * 32 + lane] = put4(s.ez[1]);
-    e[(2 * warp + 1) * 32 + lane] = put4(s.ez[R]);
-    __syncthreads();
-    // the tile's first and last rows have no neighbour here: any value does
-    get4(s.ez[0], e[(warp > 0 ? 2 * warp - 1 : 0) * 32 + lane]);
-    get4(s.ez[R + 1], e[(warp < NW - 1 ? 2 * warp + 2 : 2 * warp + 1) * 32 + lane]);
-    tile_step<R, JS, LOSSLESS, PLAIN, T>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, threads, warp, lane);
-    if (p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, own, u0, u1);
-    tile_round<R, JS, T>(s);
-  }
+  // the loop in the form the warp needs (its barriers pair across the forms)
+  auto loop = [&](auto x, auto y) {
+    for (int t = 0; t < steps; ++t) {
+      float4* e = ex + (t & 1) * 2 * NW * 32;
+      e[(2 * warp) * 32 + lane] = put4(s.ez[1]);
+      e[(2 * warp + 1) * 32 + lane] = put4(s.ez[R]);
+      cta_sync();
+      // the tile's first and last rows have no neighbour here: any value does
+      get4(s.ez[0], e[(warp > 0 ? 2 * warp - 1 : 0) * 32 + lane]);
+      get4(s.ez[R + 1], e[(warp < NW - 1 ? 2 * warp + 2 : 2 * warp + 1) * 32 + lane]);
+      tile_step<R, JS, LOSSLESS, decltype(x)::value, decltype(y)::value, T>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, threads, lane);
+      if (p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, own, u0, u1);
+      tile_round<R, JS, T>(s);
+    }
+  };
+  if (PLAIN || !(p.x || p.y)) loop(No{}, No{});
+  else if (!p.y) loop(Yes{}, No{});
+  else if (!p.x) loop(No{}, Yes{});
+  else loop(Yes{}, Yes{});
   if (own) {
     T* ez = field_ptr_t<T>(S, kEz, 1) + p.i;
     T* hx = field_ptr_t<T>(S, kHx, 1) + p.i;
@@ -190,7 +150,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const int4 tile, int
       }
     }
   }
-  if (!PLAIN) tile_psi_io<R, true>(S, S.psi + S.psi_buf, p, psi, rows, row0, warp, lane, own, u0, u1);
+  if (!PLAIN) tile_psi_io<R, true, true>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, u0, u1);
 }
 
 template <int RP>
@@ -223,25 +183,6 @@ const void* tile_kernel(const DevShot& s) {
 }
 const void* tile_kernel(int shape, const DevShot& s) {
   return shape == 0 ? tile_kernel<kShapes[0]>(s) : tile_kernel<kShapes[1]>(s);
-}
-
-// Strip lanes of a 128-column tile at c0, and strip rows of `rows` rows from r0.
-int strip_lanes(const DevShot& s, int c0) {
-  int n = 0;
-  for (int l = 0; l < 32; ++l) {
-    bool any = false;
-    for (int k = 0; k < 4; ++k) {
-      const int c = c0 + 4 * l + k;
-      any = any || (c >= 0 && c <= s.npml - 1) || (c >= s.nx - s.npml && c <= s.nx - 2);
-    }
-    n += any;
-  }
-  return n;
-}
-int strip_rows(const DevShot& s, int r0, int rows) {
-  int n = 0;
-  for (int j = r0; j < r0 + rows; ++j) n += (j >= 0 && j <= s.npml - 1) || (j >= s.ny - s.npml && j <= s.ny - 2);
-  return n;
 }
 
 }  // namespace
@@ -279,13 +220,14 @@ std::vector<int4> make_tiles(const DevShot& s, int shape) {
 }
 
 size_t tile_smem(const DevShot& s, int shape) {
-  int nxl = 0, nyl = 0;
+  int nxl = 0, yw = 0;
   for (int c = 0; c < s.nx; c += kUse) nxl = std::max(nxl, strip_lanes(s, c - kHalo));
-  for (int r = 0; r < s.ny - 1; ++r) nyl = std::max(nyl, strip_rows(s, r - kHalo, kRowsEdge));
+  for (int r = 0; r < s.ny - 1; ++r) yw = std::max(yw, y_warps(s, r - kHalo, kWarps, kREdge));
   const size_t ex = 4 * kWarps * 32;
-  const size_t edge = ex + kREdge * kWarps * 32 + 2 * (size_t)kRowsEdge * nxl + 2 * (size_t)nyl * 32 + kWarps * 32;
+  const size_t edge = ex + kREdge * kWarps * 32 + tile_table_f4(kRowsEdge) + tile_psi_x(kRowsEdge, nxl) +
+                      (size_t)yw * (2 * kREdge + 1) * 32;
   const size_t plain = ex + 2 * (size_t)kShapes[shape] * kWarps * 32;
-  return std::max(edge * 16 + ((size_t)kTcRows * kTileCols + (size_t)kTcRows * (kRowsEdge + 1)) * 4, plain * 16);
+  return std::max(edge, plain) * 16;
 }
 
 bool tile_fits(const DevShot& s, int shape, int device) {

@@ -26,6 +26,13 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
+struct Yes { static constexpr bool value = true; };
+struct No { static constexpr bool value = false; };
+
+// The CTA's barrier, from any point of the code: the warps of a tile run
+// differently specialised loops that meet at it.
+__device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 0;" ::: "memory"); }
+
 // Column and row tables of a tile that is not plain, in shared memory.
 // Columns: b and c/d of the Hy and Ez recursions (the column's strip), and
 // the denominators; rows likewise for Hx and Ez.
@@ -75,68 +82,82 @@ struct TileRegs {
 };
 
 // Where a thread and its warp sit in the grid, and what of the CPML they hold.
+// x: the tile touches a border or a strip in x (the same for its whole CTA);
+// y: the warp's rows, or the row below them, do in y.  Elsewhere the update
+// needs no masks, no psi and no tables.
 struct TilePos {
   int i, j0;          // first column and row
-  unsigned mh, me;    // columns (bits 0-3) whose H / Ez are updated
-  unsigned xh, xe;    // columns in an x strip for Hy / Ez
+  bool x, y;
+  // columns whose H (bits 0-3) and Ez (4-7) are updated, that lie in an x strip
+  // for Hy (8-11) and for Ez (12-15)
+  unsigned mask;
   int xslot, nxl;     // the thread's slot among the row's strip lanes, their number
-  int ylo, yhi, nyl;  // strip rows: slot of row j is j - ylo (j < npml) or j - yhi; their number
+  int yslot;          // the warp's slot among the CTA's y warps
+  __device__ __forceinline__ bool mh(int k) const { return mask >> k & 1; }
+  __device__ __forceinline__ bool me(int k) const { return mask >> (4 + k) & 1; }
+  __device__ __forceinline__ bool xh(int k) const { return mask >> (8 + k) & 1; }
+  __device__ __forceinline__ bool xe(int k) const { return mask >> (12 + k) & 1; }
+  __device__ __forceinline__ bool strip() const { return mask >> 8; }
 };
 
-// psi of a tile in shared memory.
+// psi of a tile in shared memory: x strips [Hy, Ez][rows][nxl]; y strips, per y
+// warp, R + 1 rows of Hx (the row below first) and R of Ez, a float4 per lane.
 struct TilePsi {
-  float4* x;   // [Hy, Ez][rows][nxl]
-  float4* y;   // [Hx, Ez][nyl][32]
-  float4* b;   // [warps][32]: Hx of the row below each warp
+  float4 *x, *y;      // y: this thread's first
 };
 
 __device__ __forceinline__ void get4(float (&d)[4], const float4& v) { d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w; }
 __device__ __forceinline__ float4 put4(const float (&d)[4]) { return make_float4(d[0], d[1], d[2], d[3]); }
 
-// Strip row of Hx (side -1: none): rows 0 .. P-2 and ny-P .. ny-2.
-__device__ __forceinline__ bool y_strip_h(int j, int ny, int P) { return (j >= 0 && j <= P - 2) || (j >= ny - P && j <= ny - 2); }
-// Strip row of Ez: rows 1 .. P-1 and ny-P .. ny-2.
-__device__ __forceinline__ bool y_strip_e(int j, int ny, int P) { return (j >= 1 && j <= P - 1) || (j >= ny - P && j <= ny - 2); }
+// Strip rows of Hx: 0 .. P-2 and ny-P .. ny-2.
+__host__ __device__ __forceinline__ bool y_strip_h(int j, int ny, int P) { return (j >= 0 && j <= P - 2) || (j >= ny - P && j <= ny - 2); }
+// Strip rows of Ez: 1 .. P-1 and ny-P .. ny-2.
+__host__ __device__ __forceinline__ bool y_strip_e(int j, int ny, int P) { return (j >= 1 && j <= P - 1) || (j >= ny - P && j <= ny - 2); }
+// Whether rows j0-1 .. j0+R-1 need the y form, columns c0 .. c0+127 the x form.
+__host__ __device__ __forceinline__ bool tile_y(const DevShot& s, int j0, int R) {
+  return !s.den_uniform || j0 - 1 < s.npml || j0 + R - 1 >= s.ny - s.npml;
+}
+__host__ __device__ __forceinline__ bool tile_x(const DevShot& s, int c0) {
+  return !s.den_uniform || c0 < s.npml || c0 + kTileCols - 1 >= s.nx - s.npml;
+}
 
-// Geometry of a thread in the tile at (c0, r0) of `rows` rows; `plain` tiles
-// have no CPML and no border.
-__device__ __forceinline__ TilePos tile_pos(const DevShot& S, int c0, int r0, int rows, int j0, int lane, bool plain) {
+__device__ __forceinline__ TilePos tile_pos(const DevShot& S, int c0, int r0, int R, int warp, int lane) {
   TilePos p{};
   p.i = c0 + 4 * lane;
-  p.j0 = j0;
-  if (plain) return p;
-  const int nx = S.nx, ny = S.ny, P = S.npml;
+  p.j0 = r0 + warp * R;
+  p.x = tile_x(S, c0);
+  p.y = tile_y(S, p.j0, R);
+  const int nx = S.nx, P = S.npml;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int c = p.i + k;
-    if (c >= 0 && c <= nx - 2) p.mh |= 1u << k;
-    if (c >= 1 && c <= nx - 2) p.me |= 1u << k;
-    if ((c >= 0 && c <= P - 2) || (c >= nx - P && c <= nx - 2)) p.xh |= 1u << k;
-    if ((c >= 1 && c <= P - 1) || (c >= nx - P && c <= nx - 2)) p.xe |= 1u << k;
+    if (c >= 0 && c <= nx - 2) p.mask |= 1u << k;
+    if (c >= 1 && c <= nx - 2) p.mask |= 16u << k;
+    if ((c >= 0 && c <= P - 2) || (c >= nx - P && c <= nx - 2)) p.mask |= 256u << k;
+    if ((c >= 1 && c <= P - 1) || (c >= nx - P && c <= nx - 2)) p.mask |= 4096u << k;
   }
-  const unsigned m = __ballot_sync(kFull, (p.xh | p.xe) != 0);
-  p.xslot = __popc(m & ((1u << lane) - 1));
+  const unsigned m = __ballot_sync(kFull, p.strip());
+  p.xslot = p.strip() ? __popc(m & ((1u << lane) - 1)) : 0;
   p.nxl = __popc(m);
-  const int top = r0 + rows;                      // one past the tile's last row
-  const int lo0 = max(r0, 0), lo = max(0, min(top, P) - lo0);
-  const int hi0 = max(r0, ny - P), hi = max(0, min(top, ny - 1) - hi0);
-  p.ylo = lo0;
-  p.yhi = hi0 - lo;
-  p.nyl = lo + hi;
+  for (int w = 0; w < warp; ++w) p.yslot += tile_y(S, r0 + w * R, R) ? 1 : 0;
   return p;
 }
 
-__device__ __forceinline__ TilePsi tile_psi(float4* base, const TilePos& p, int rows) {
+// float4s of a tile's tables and of its x psi
+__host__ __device__ __forceinline__ int tile_table_f4(int rows) { return kTcRows * (kTileCols + rows + 4) / 4; }
+__host__ __device__ __forceinline__ int tile_psi_x(int rows, int nxl) { return 2 * rows * nxl; }
+__device__ __forceinline__ TilePsi tile_psi(float4* base, const TilePos& p, int rows, int R, int lane) {
   TilePsi s;
   s.x = base;
-  s.y = s.x + 2 * rows * p.nxl;
-  s.b = s.y + 2 * p.nyl * 32;
+  s.y = base + tile_psi_x(rows, p.nxl) + p.yslot * (2 * R + 1) * 32 + lane;
   return s;
 }
 
-// The tables of a tile that is not plain: tc[kTcRows][128] by column, tr[kTcRows][rows+1] by row (row r0-1 first).
-__device__ __forceinline__ void tile_tables(const DevShot& S, float* tc, float* tr, int c0, int r0, int rows, int tid,
-                                            int threads) {
+// The tables of a tile with borders or strips: tc[kTcRows][128] by column,
+// tr[kTcRows][rows+1] by row (row r0-1 first); c/d in stored units.
+template <class T>
+__device__ __forceinline__ void tile_tables(const DevShot& S, const Coef<T>& C, float* tc, float* tr, int c0, int r0,
+                                            int rows, int tid, int threads) {
   const int nx = S.nx, ny = S.ny, P = S.npml;
   for (int t = tid; t < kTileCols + rows + 1; t += threads) {
     const bool col = t < kTileCols;
@@ -151,151 +172,251 @@ __device__ __forceinline__ void tile_tables(const DevShot& S, float* tc, float* 
     if (c >= 1 && c <= P - 1) { be = S.cpml[e0 * P + c]; ce = S.cpml[(e0 + 1) * P + c]; }
     else if (c >= n - P && c <= n - 2) { be = S.cpml[(e0 + 2) * P + n - 1 - c]; ce = S.cpml[(e0 + 3) * P + n - 1 - c]; }
     if (c >= 0 && c < n - 1) { de = (col ? S.den_ex : S.den_ey)[c]; dh = (col ? S.den_hx : S.den_hy)[c]; }
-    out[kTcBh * st] = bh; out[kTcCh * st] = ch; out[kTcBe * st] = be; out[kTcCe * st] = ce;
+    out[kTcBh * st] = bh; out[kTcCh * st] = __fmul_rn(ch, C.sE); out[kTcBe * st] = be; out[kTcCe * st] = __fmul_rn(ce, C.sH);
     out[kTcDe * st] = de; out[kTcDh * st] = dh;
+  }
+}
+
+// psi of the tile from (STORE false) or to the slab; stored: the columns of
+// the mask `own` in rows [u0, u1).  ALIGNED: the thread's first column is a
+// multiple of 4 (then `own` is all or none).
+template <int R, bool STORE, bool ALIGNED>
+__device__ __forceinline__ void tile_psi_io(const DevShot& S, float* slab, const TilePos& p, const TilePsi& psi, int rows,
+                                            int row0, unsigned own, int u0, int u1) {
+  const int nx = S.nx, ny = S.ny, P = S.npml;
+  const int64_t pitch = S.pitch;
+#pragma unroll 1
+  for (int r = -1; r < R; ++r) {
+    const int j = p.j0 + r;
+    if (STORE && (r < 0 || j < u0 || j >= u1 || !own)) continue;
+    const bool row = j >= 0 && j <= ny - 1;
+    // x strips: Hy, Ez
+    if (r >= 0 && p.strip()) {
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        float4* ps = psi.x + (f * rows + row0 + r) * p.nxl + p.xslot;
+        float v[4];
+        if (STORE) get4(v, *ps); else zero4(v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (!row || !(f ? p.xe(k) : p.xh(k)) || (STORE && !(own >> k & 1))) continue;
+          const int c = p.i + k;
+          const int side = c >= P ? 1 : 0, q = side ? nx - (f ? 1 : 2) - c : c;
+          float* g = slab + (f ? S.o_ezx : S.o_hyx) + ((int64_t)side * ny + j) * P + q;
+          if (STORE) *g = v[k]; else v[k] = __ldcg(g);
+        }
+        if (!STORE) *ps = put4(v);
+      }
+    }
+    // y strips: Hx, Ez
+    if (!p.y) continue;
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      if (r < 0 && f) continue;
+      const bool strip = f ? y_strip_e(j, ny, P) : y_strip_h(j, ny, P);
+      if (STORE && !strip) continue;
+      const int side = j >= P ? 1 : 0, q = side ? ny - (f ? 1 : 2) - j : j;
+      float* g = slab + (f ? S.o_ezy + ((int64_t)side * P + q) * pitch : ((int64_t)side * (P - 1) + q) * pitch) + p.i;
+      float4* ps = psi.y + (f ? R + 1 + r : r + 1) * 32;
+      if (ALIGNED) {   // a thread left of column 0 holds no strip cell
+        const bool in = p.i >= 0 && p.i < nx;
+        if (STORE) {
+          if (in) *reinterpret_cast<float4*>(g) = *ps;
+        } else {
+          *ps = strip && in ? __ldcg(reinterpret_cast<const float4*>(g)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      } else {
+        float v[4];
+        if (STORE) get4(v, *ps);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const bool in = p.i + k >= 0 && p.i + k < nx;
+          if (STORE) {
+            if (in && (own >> k & 1)) g[k] = v[k];
+          } else {
+            v[k] = strip && in ? __ldcg(g + k) : 0.f;
+          }
+        }
+        if (!STORE) *ps = put4(v);
+      }
+    }
   }
 }
 
 // One time step of the thread's cells up to Ez, without sources, detectors
 // and the rounding to the storage type; s.ez[0] and s.ez[R+1] hold the rows
-// around the thread's.  PLAIN: no CPML, no border, the denominators are the shot's
-// constants.  kp: the thread's drive, `stride` float4 from row to row.
-template <int R, bool JS, bool LOSSLESS, bool PLAIN, class T>
+// around the thread's.  X, Y: the tile's and the warp's forms (TilePos).  The
+// body has no branches (a strip row or lane is a select, every psi slot of an
+// X tile or Y warp is read and written) and stores to shared memory only
+// after several rows' loads, which the compiler may not move across a store,
+// so that the rows' chains overlap: with a branch per strip row a warp took
+// ~1800 cycles a row, and the tiles in the corners of the grid set the step
+// time of all.
+// kp: the thread's drive, js its Jz where JS, `stride` float4 from row to row.
+template <int R, bool JS, bool LOSSLESS, bool X, bool Y, class T>
 __device__ __forceinline__ void tile_step(TileRegs<R, JS>& s, const DevShot& S, const Coef<T>& C, const TilePos& p,
                                           const TilePsi& psi, const float* tc, const float* tr, int rows, int row0,
-                                          const float4* kp, float4* js, int stride, int warp, int lane) {
+                                          const float4* kp, float4* js, int stride, int lane) {
   const int ny = S.ny, P = S.npml;
-  const float dhx_c = S.den_c[1], dhy_c = S.den_c[3], dex_c = S.den_c[0], dey_c = S.den_c[2];
   const int ts = rows + 1;             // row tables start at row r0 - 1
+  const float* trw = tr + row0;        // this warp's: entry r is row j0 - 1 + r
   // ---- Hx: row j0 - 1 (the warp below owns it), then the thread's rows
+  constexpr int kBatch = 2;   // rows whose psi is held before it is stored
+  float pq[kBatch][4];
 #pragma unroll
   for (int r = 0; r <= R; ++r) {
-    const float den = PLAIN ? dhy_c : tr[kTcDh * ts + row0 + r];
-    const int j = p.j0 - 1 + r;
-    if (!PLAIN && !(j >= 0 && j <= ny - 2)) continue;
-    const bool strip = !PLAIN && y_strip_h(j, ny, P);
-    float4* ps = r == 0 ? psi.b + warp * 32 + lane : psi.y + (j - (j < P ? p.ylo : p.yhi)) * 32 + lane;
-    float pn[4] = {0.f, 0.f, 0.f, 0.f};
-    if (strip) get4(pn, *ps);
-    const float b = strip ? tr[kTcBh * ts + row0 + r] : 0.f;
-    const float c = strip ? __fmul_rn(tr[kTcCh * ts + row0 + r], C.sE) : 0.f;
+    const float den = Y ? trw[kTcDh * ts + r] : S.den_c[3];
+    float (&pn)[4] = pq[r % kBatch];
+    float b = 0.f, c = 0.f;
+    bool strip = false;
+    if (Y) {
+      get4(pn, psi.y[r * 32]);
+      b = trw[kTcBh * ts + r];
+      c = trw[kTcCh * ts + r];
+      strip = y_strip_h(p.j0 - 1 + r, ny, P);
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const bool in = PLAIN || (p.mh >> k & 1);
+      const bool in = !X || p.mh(k);
       float v = tile_h<LOSSLESS>(C.da, s.hx[r][k], C.db, s.ez[r][k], s.ez[r + 1][k], den);
-      if (strip) {
+      if (Y) {
         const float q = upd_psi(b, pn[k], c, s.ez[r][k], s.ez[r + 1][k]);
-        v = __fmaf_rn(C.pdb, q, v);
-        pn[k] = in ? q : pn[k];
+        const float w = __fmaf_rn(C.pdb, q, v);
+        v = strip ? w : v;
+        pn[k] = strip && in ? q : pn[k];
       }
       s.hx[r][k] = in ? v : s.hx[r][k];
     }
-    if (strip) *ps = put4(pn);
+    if (Y && (r % kBatch == kBatch - 1 || r == R)) {
+#pragma unroll
+      for (int q = r - r % kBatch; q <= r; ++q) psi.y[q * 32] = put4(pq[q % kBatch]);
+    }
   }
   // ---- Hy
-  float dhx[4], dex[4];
-  if (PLAIN) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) { dhx[k] = dhx_c; dex[k] = dex_c; }
-  } else {
+  float dhx[4], b[4], c[4];
+  if (X) {
     lds4f(dhx, tc + kTcDh * kTileCols + 4 * lane);
-    lds4f(dex, tc + kTcDe * kTileCols + 4 * lane);
+    lds4f(b, tc + kTcBh * kTileCols + 4 * lane);
+    lds4f(c, tc + kTcCh * kTileCols + 4 * lane);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dhx[k] = S.den_c[1];
   }
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const float e4 = __shfl_down_sync(kFull, s.ez[r + 1][0], 1);
     const float er[4] = {s.ez[r + 1][1], s.ez[r + 1][2], s.ez[r + 1][3], e4};
+    float (&pn)[4] = pq[r % kBatch];
+    if (X) get4(pn, psi.x[(row0 + r) * p.nxl + p.xslot]);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float v = tile_h<LOSSLESS>(C.da, s.hy[r][k], C.db, er[k], s.ez[r + 1][k], dhx[k]);
-      s.hy[r][k] = PLAIN || (p.mh >> k & 1) ? v : s.hy[r][k];
-    }
-    if (!PLAIN && p.xh) {
-      float b[4], c[4], pn[4];
-      lds4f(b, tc + kTcBh * kTileCols + 4 * lane);
-      lds4f(c, tc + kTcCh * kTileCols + 4 * lane);
-      float4* ps = psi.x + (row0 + r) * p.nxl + p.xslot;
-      get4(pn, *ps);
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-      {
-        const bool in = p.xh >> k & 1;
-        const float q = upd_psi(b[k], pn[k], __fmul_rn(c[k], C.sE), er[k], s.ez[r + 1][k]);
-        const float v = __fmaf_rn(C.pdb, q, s.hy[r][k]);
-        pn[k] = in ? q : pn[k];
-        s.hy[r][k] = in ? v : s.hy[r][k];
+      float v = tile_h<LOSSLESS>(C.da, s.hy[r][k], C.db, er[k], s.ez[r + 1][k], dhx[k]);
+      if (X) {
+        const bool strip = p.xh(k);
+        const float q = upd_psi(b[k], pn[k], c[k], er[k], s.ez[r + 1][k]);
+        const float w = __fmaf_rn(C.pdb, q, v);
+        v = strip ? w : v;
+        pn[k] = strip ? q : pn[k];
       }
-      *ps = put4(pn);
+      s.hy[r][k] = !X || p.mh(k) ? v : s.hy[r][k];
+    }
+    if (X && p.strip() && (r % kBatch == kBatch - 1 || r == R - 1)) {
+#pragma unroll
+      for (int q = r - r % kBatch; q <= r; ++q) psi.x[(row0 + q) * p.nxl + p.xslot] = put4(pq[q % kBatch]);
     }
   }
   // ---- Jz and Ez
+  float dex[4];
+  if (X) {
+    lds4f(dex, tc + kTcDe * kTileCols + 4 * lane);
+    lds4f(b, tc + kTcBe * kTileCols + 4 * lane);
+    lds4f(c, tc + kTcCe * kTileCols + 4 * lane);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dex[k] = S.den_c[0];
+  }
+  float pxq[kBatch][4], pyq[kBatch][4], jq[kBatch][4];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const float hl = __shfl_up_sync(kFull, s.hy[r][3], 1);
     const float hyl[4] = {hl, s.hy[r][0], s.hy[r][1], s.hy[r][2]};
     const int j = p.j0 + r;
-    if (!PLAIN && !(j >= 1 && j <= ny - 2)) continue;
+    const bool row_in = !Y || (j >= 1 && j <= ny - 2);
+    float (&px)[4] = pxq[r % kBatch], (&py)[4] = pyq[r % kBatch], (&jv)[4] = jq[r % kBatch];
     float kv[4];
     get4(kv, kp[r * stride]);
+    if (JS) get4(jv, js[r * stride]);
     float (&jz)[4] = s.jz[JS ? 0 : r];
-    if (JS) get4(jz, js[r * stride]);
-    const float dey = PLAIN ? dey_c : tr[kTcDe * ts + row0 + 1 + r];
-    float ep[4] = {0.f, 0.f, 0.f, 0.f};
-    if (!PLAIN && p.xe) {
-      float b[4], c[4];
-      lds4f(b, tc + kTcBe * kTileCols + 4 * lane);
-      lds4f(c, tc + kTcCe * kTileCols + 4 * lane);
-      float4* ps = psi.x + (rows + row0 + r) * p.nxl + p.xslot;
-      get4(ep, *ps);
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-      {
-        const float q = upd_psi(b[k], ep[k], __fmul_rn(c[k], C.sH), s.hy[r][k], hyl[k]);
-        ep[k] = p.xe >> k & 1 ? q : ep[k];
-      }
-      *ps = put4(ep);
+    const float dey = Y ? trw[kTcDe * ts + r + 1] : S.den_c[2];
+    float yb = 0.f, yc = 0.f;
+    bool ystrip = false;
+    if (X) get4(px, psi.x[(rows + row0 + r) * p.nxl + p.xslot]);
+    if (Y) {
+      get4(py, psi.y[(R + 1 + r) * 32]);
+      yb = trw[kTcBe * ts + r + 1];
+      yc = trw[kTcCe * ts + r + 1];
+      ystrip = y_strip_e(j, ny, P);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const bool in = PLAIN || (p.me >> k & 1);
-      const float jn = upd_j(C.ja, jz[k], kv[k], s.ez[r + 1][k]);
-      float v = tile_e<LOSSLESS, T>(C, s.ez[r + 1][k], __fsub_rn(s.hy[r][k], hyl[k]), dex[k], __fsub_rn(s.hx[r][k], s.hx[r + 1][k]), dey, jn);
-      if (!PLAIN && p.xe) {
-        const float w = __fmaf_rn(C.pcb, ep[k], v);
-        v = p.xe >> k & 1 ? w : v;
+      const bool in = row_in && (!X || p.me(k));
+      const float jo = JS ? jv[k] : jz[k];
+      const float jn = upd_j(C.ja, jo, kv[k], s.ez[r + 1][k]);
+      float v = tile_e<LOSSLESS, T>(C, s.ez[r + 1][k], __fsub_rn(s.hy[r][k], hyl[k]), dex[k], __fsub_rn(s.hx[r][k], s.hx[r + 1][k]),
+                                    dey, jn);
+      if (X) {
+        const bool strip = p.xe(k) && row_in;
+        const float q = upd_psi(b[k], px[k], c[k], s.hy[r][k], hyl[k]);
+        const float w = __fmaf_rn(C.pcb, q, v);
+        v = strip ? w : v;
+        px[k] = strip ? q : px[k];
       }
-      jz[k] = in ? jn : jz[k];
+      if (Y) {
+        const float q = upd_psi(yb, py[k], yc, s.hx[r][k], s.hx[r + 1][k]);
+        const float w = __fmaf_rn(C.pcb, q, v);
+        v = ystrip ? w : v;
+        py[k] = ystrip && in ? q : py[k];
+      }
+      if (JS) jv[k] = in ? jn : jo; else jz[k] = in ? jn : jo;
       s.ez[r + 1][k] = in ? v : s.ez[r + 1][k];
     }
-    if (JS) {
-      if (sizeof(T) == 2) Sto<T>::rt4(jz, jz);
-      js[r * stride] = put4(jz);
-    }
-    if (!PLAIN && y_strip_e(j, ny, P)) {
-      const float b = tr[kTcBe * ts + row0 + 1 + r], c = __fmul_rn(tr[kTcCe * ts + row0 + 1 + r], C.sH);
-      float4* ps = psi.y + (p.nyl + j - (j < P ? p.ylo : p.yhi)) * 32 + lane;
-      float pn[4];
-      get4(pn, *ps);
+    if (JS && sizeof(T) == 2) Sto<T>::rt4(jv, jv);
+    if (r % kBatch == kBatch - 1 || r == R - 1) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-      {
-        const bool in = p.me >> k & 1;
-        const float q = upd_psi(b, pn[k], c, s.hx[r][k], s.hx[r + 1][k]);
-        const float v = __fmaf_rn(C.pcb, q, s.ez[r + 1][k]);
-        pn[k] = in ? q : pn[k];
-        s.ez[r + 1][k] = in ? v : s.ez[r + 1][k];
+      for (int q = r - r % kBatch; q <= r; ++q) {
+        if (X && p.strip()) psi.x[(rows + row0 + q) * p.nxl + p.xslot] = put4(pxq[q % kBatch]);
+        if (Y) psi.y[(R + 1 + q) * 32] = put4(pyq[q % kBatch]);
+        if (JS) js[q * stride] = put4(jq[q % kBatch]);
       }
-      *ps = put4(pn);
     }
   }
 }
 
+// Strip lanes of the 128 columns at c0, y warps among `warps` of R rows from r0.
+inline int strip_lanes(const DevShot& s, int c0) {
+  int n = 0;
+  for (int l = 0; l < 32; ++l) {
+    bool any = false;
+    for (int k = 0; k < 4; ++k) {
+      const int c = c0 + 4 * l + k;
+      any = any || (c >= 0 && c <= s.npml - 1) || (c >= s.nx - s.npml && c <= s.nx - 2);
+    }
+    n += any;
+  }
+  return n;
+}
+inline int y_warps(const DevShot& s, int r0, int warps, int R) {
+  int n = 0;
+  for (int w = 0; w < warps; ++w) n += tile_y(s, r0 + w * R, R) ? 1 : 0;
+  return n;
+}
+
 // Sources, then detectors, of the thread's rows at step n (points [p0, p1) of
-// the shot's table are those of the warp's rows).  Detectors record where
-// `own`; rows [u0, u1) are the ones this tile answers for.
+// the shot's table are those of the warp's rows).  Detectors record in the
+// columns of the mask `own` and rows [u0, u1), the ones this tile answers for.
 template <int R, bool JS, class T>
 __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S, const TilePos& p, int p0, int p1, int n,
-                                            bool own, int u0, int u1) {
+                                            unsigned own, int u0, int u1) {
   constexpr bool sc = sizeof(T) == 2;
   for (int q = p0; q < p1; ++q) {
     const int4 pt = __ldg(S.pts + q);
@@ -312,7 +433,7 @@ __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S
 #pragma unroll
       for (int t = 0; t < 4 * R; ++t)
         if (t == at) s.ez[t / 4 + 1][t % 4] = e;
-    } else if (!own || pt.w < u0 || pt.w >= u1) {
+    } else if (!(own >> k & 1) || pt.w < u0 || pt.w >= u1) {
       continue;
     } else if (pt.y == kPointDetEz) {
       if (sc) e = __fmul_rn(e, S.sc[0]);

@@ -30,6 +30,18 @@ def _stepped(gpu, prob, st, chunks):
     return name, out
 
 
+def _one_row(gpu, monkeypatch, prob, st, steps):
+    """The one-row kernel's results."""
+    for v in ("FDTD2D_TILE", "FDTD2D_RESIDENT"):
+        monkeypatch.delenv(v, raising=False)
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv("FDTD2D_TMA", "4,3")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = _stepped(gpu, prob, st, (steps,))
+    assert name == "step_tma_kernel<4,3>", name
+    return ref
+
+
 @pytest.mark.parametrize("rows", ["7", "5"])
 @pytest.mark.parametrize("nx,ny,P,store,profile,ca", [
     (40, 40, 2, 0, 1, 1.0), (120, 25, 3, 0, 1, 1.0), (121, 24, 4, 0, 0, 1.0), (203, 157, 7, 0, 1, 0.999),
@@ -47,14 +59,80 @@ def test_tile_equals_one_row(gpu, monkeypatch, rows, nx, ny, P, store, profile, 
     monkeypatch.setenv("FDTD2D_TILE", rows)
     name, got = _stepped(gpu, prob, st, CHUNKS)
     assert name == f"step_tmat_kernel<tile,{rows}>", name
-    monkeypatch.delenv("FDTD2D_TILE")
-    monkeypatch.setenv("FDTD2D_TMAT", "0")
-    monkeypatch.setenv("FDTD2D_TMA", "4,3")
-    monkeypatch.setenv("FDTD2D_PERSIST", "0")
-    name, ref = _stepped(gpu, prob, st, (STEPS,))
-    assert name == "step_tma_kernel<4,3>", name
+    ref = _one_row(gpu, monkeypatch, prob, st, STEPS)
     for k in ref:
         assert np.array_equal(ref[k], got[k]), k
+
+
+@pytest.mark.parametrize("rows", [2, 4, 6, 8])
+@pytest.mark.parametrize("nx,ny,P,profile,ca", [
+    (10, 9, 2, 1, 1.0), (126, 40, 3, 1, 1.0), (127, 41, 5, 0, 1.0), (252, 33, 4, 1, 0.999), (253, 97, 12, 1, 1.0),
+    (203, 157, 7, 1, 1.0), (64, 260, 12, 3, 1.0), (1100, 90, 9, 1, 1.0), (500, 400, 40, 1, 0.998), (777, 601, 17, 3, 1.0)])
+def test_resident_equals_one_row(gpu, monkeypatch, rows, nx, ny, P, profile, ca):
+    """The whole shot on chip: one band of columns, two, several; strips down to
+    a single warp; component detectors; the short run calls on the tile passes."""
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE"):
+        monkeypatch.delenv(v, raising=False)
+    n = 1 if nx < 40 else 5
+    prob = F.Problem.from_spec(nx=nx, ny=ny, npml=P, n_steps=STEPS, profile=profile, x_lo=nx // 3, x_hi=nx - 3,
+                               x_center=nx / 2, width=nx / 8, grf_rms=0.05, grf_corr=8, ne_peak=2e19, nu=3e9, n_elem=n,
+                               src_i=nx // 2 - 6 if nx > 40 else 4, src_j=ny // 2, src_di=3, src_dj=1, n_det=n,
+                               det_i=nx // 2 - 8 if nx > 40 else 5, det_j=ny // 2 - 2, det_di=2, det_dj=1)
+    s = prob.setup
+    s.ca = s.da = ca
+    s.n_comp, s.comp = s.n_det, s.det
+    st = random_state(None, nx, ny, P, np.random.default_rng(nx))
+    monkeypatch.setenv("FDTD2D_RESIDENT", str(rows))
+    name, got = _stepped(gpu, prob, st, CHUNKS)
+    assert name == f"step_persist_kernel<0>/tile<{rows}>", name
+    ref = _one_row(gpu, monkeypatch, prob, st, STEPS)
+    for k in ref:
+        assert np.array_equal(ref[k], got[k]), k
+
+
+def test_resident_default_and_limits(gpu, monkeypatch):
+    """A small shot runs on chip by default; one with more points than a warp's
+    list holds, with two sources in a cell, or too large, on tile passes."""
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE", "FDTD2D_RESIDENT"):
+        monkeypatch.delenv(v, raising=False)
+    base = dict(ny=160, npml=10, n_steps=40, src_i=60, src_j=80, det_i=62, det_j=80)
+
+    def name_and_check(**kw):
+        prob = F.Problem.from_spec(**{**base, **kw})
+        st = random_state(None, prob.nx, prob.ny, prob.setup.npml, np.random.default_rng(3))
+        with monkeypatch.context() as m:
+            name, got = _stepped(gpu, prob, st, (40,))
+            ref = _one_row(gpu, m, prob, st, 40)
+        for k in ref:
+            assert np.array_equal(ref[k], got[k]), (name, k)
+        return name
+
+    assert name_and_check(nx=200).startswith("step_persist_kernel<0>/tile<")
+    assert name_and_check(nx=200, n_det=60, det_i=63, det_di=1).startswith("step_tmat_kernel<tile")
+    assert name_and_check(nx=200, n_elem=2).startswith("step_tmat_kernel<tile")   # both elements in one cell
+    assert name_and_check(nx=1300, ny=1300).startswith("step_tmat_kernel<tile")
+
+
+def test_resident_wait_runs_out(gpu, monkeypatch):
+    """A neighbour's edge that never carries the expected tag: the poll gives up
+    after its bound, the run reports it, the next shot runs as usual."""
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE", "FDTD2D_RESIDENT"):
+        monkeypatch.delenv(v, raising=False)
+    prob = F.Problem.from_spec(nx=256, ny=192, n_steps=200, x_lo=128, x_hi=246, src_i=30, src_j=96, det_i=34, det_j=96)
+    monkeypatch.setenv("FDTD2D_WAIT_NS", "1000000")
+    monkeypatch.setenv("FDTD2D_TEST_BARRIER_EXTRA", "1")
+    with F.Shot(prob, gpu) as shot:
+        assert shot.kernel_name().startswith("step_persist_kernel<0>/tile<")
+        shot.run(1, 100)
+        with pytest.raises(F.FdtdError) as e:
+            shot.synchronize()
+        assert e.value.status == F.ERR_TIMEOUT
+    monkeypatch.delenv("FDTD2D_WAIT_NS")
+    monkeypatch.delenv("FDTD2D_TEST_BARRIER_EXTRA")
+    with F.Shot(prob, gpu) as shot:
+        shot.run(1, 200)
+        shot.synchronize()
+        assert shot.check_finite()
 
 
 def test_tile_line_probe_and_components(gpu, monkeypatch):
