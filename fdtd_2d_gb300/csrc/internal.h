@@ -320,7 +320,11 @@ cudaError_t launch_line(const float* ez, int64_t pitch, int j, int i0, int n, fl
 // Count non-finite values in n floats (atomic count into *flag).
 cudaError_t launch_nonfinite(const float* a, int64_t n, int* flag, cudaStream_t stream);
 cudaError_t launch_nonfinite16(const uint16_t* a, int64_t n, bool bf16, int* flag, cudaStream_t stream);
-// n FP32 values to F16 (store 1) or BF16 (store 2) elements, times isc.
+// rows x cols F16 (store 1) or BF16 (store 2) elements, rows `pitch` apart, to
+// contiguous FP32 values, times sc.
+cudaError_t launch_from_storage(const void* src, int64_t pitch, float* dst, int rows, int cols, int store, float sc,
+                                cudaStream_t stream);
+// n FP32 values to elements of the storage type, times isc.
 cudaError_t launch_to_storage(const float* src, void* dst, int64_t n, int store, float isc, cudaStream_t stream);
 
 }  // namespace fdtd2d

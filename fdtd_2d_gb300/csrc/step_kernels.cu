@@ -27,6 +27,7 @@
 #include "step_common.cuh"
 #include "tma_common.cuh"
 
+#include <algorithm>
 #include <cstdio>
 
 namespace fdtd2d {
@@ -653,6 +654,25 @@ cudaError_t launch_to_storage(const float* src, void* dst, int64_t n, int store,
     to_half_kernel<<<1024, 256, 0, stream>>>(src, static_cast<__half*>(dst), n, isc);
   else
     to_bf16_kernel<<<1024, 256, 0, stream>>>(src, static_cast<__nv_bfloat16*>(dst), n, isc);
+  return cudaGetLastError();
+}
+
+// Elements of the storage type to FP32 values: dst[j][i] = src[j][i] * sc.
+template <class T>
+__global__ void from_storage_kernel(const T* __restrict__ src, int64_t pitch, float* __restrict__ dst, int rows, int cols,
+                                    float sc) {
+  for (int j = blockIdx.y; j < rows; j += gridDim.y)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cols; i += gridDim.x * blockDim.x)
+      dst[(int64_t)j * cols + i] = static_cast<float>(src[j * pitch + i]) * sc;
+}
+
+cudaError_t launch_from_storage(const void* src, int64_t pitch, float* dst, int rows, int cols, int store, float sc,
+                                cudaStream_t stream) {
+  const dim3 grid((cols + 255) / 256, std::min(rows, 2048));
+  if (store == 1)
+    from_storage_kernel<<<grid, 256, 0, stream>>>(static_cast<const __half*>(src), pitch, dst, rows, cols, sc);
+  else
+    from_storage_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(src), pitch, dst, rows, cols, sc);
   return cudaGetLastError();
 }
 
