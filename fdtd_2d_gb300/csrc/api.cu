@@ -888,26 +888,80 @@ int setup_resident(fdtd2d_ctx* c, int device) {
   return FDTD2D_OK;
 }
 
+// The tracker and the line probe on the tile paths (FP32): the kernels record
+// the tracked columns of every step (a history of up to 64 MB) and the probe's
+// row.  False when they cannot (16-bit storage, too many columns, a probe on the
+// last row, which no tile stores); an allocation that fails is no error.
+bool setup_aux(fdtd2d_ctx* c, const std::vector<int32_t>& scan_i, const std::vector<int32_t>& max_i) {
+  if (c->n_rc == 0 && c->line_n == 0) return true;
+  if (c->h.store != FDTD2D_STORE_F32 || (c->line_n > 0 && c->line_j >= c->ny - 1)) return false;
+  TileAux a{};
+  if (c->n_rc > 0) {
+    std::vector<int> cols(scan_i.begin(), scan_i.end());
+    cols.insert(cols.end(), max_i.begin(), max_i.end());
+    std::sort(cols.begin(), cols.end());
+    cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
+    a.n_cols = (int)cols.size();
+    a.rows = (c->ny + 31) / 32 * 32;
+    const int64_t per = (int64_t)a.n_cols * a.rows * 4;
+    c->rc_chunk = (int)std::min<int64_t>(256, (int64_t(64) << 20) / per);
+    if (a.n_cols > kMaxTracked || c->rc_chunk < kResidentSteps) return false;
+    auto slot = [&](int32_t i) { return (int)(std::lower_bound(cols.begin(), cols.end(), (int)i) - cols.begin()); };
+    std::vector<int> all(cols);   // columns, then each line's slots
+    for (const int32_t i : scan_i) all.push_back(slot(i));
+    for (const int32_t i : max_i) all.push_back(slot(i));
+    int* d = nullptr;
+    void* hist = nullptr;
+    cudaError_t e = dalloc(c, &d, all.size());
+    if (e == cudaSuccess) e = dalloc(c, &c->d_cand, (size_t)c->rc_chunk * c->n_rc);
+    if (e == cudaSuccess) e = cudaMallocAsync(&hist, (size_t)c->rc_chunk * per, c->stream);
+    if (e == cudaSuccess) c->allocs.push_back(hist);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    a.cols = d;
+    c->d_scan_slot = d + a.n_cols;
+    c->d_max_slot = c->d_scan_slot + c->n_rc;
+    a.hist = static_cast<float*>(hist);
+  }
+  if (c->line_n > 0) {
+    a.line_n = c->line_n;
+    a.line_j = c->line_j;
+    a.line_i0 = c->line_i0;
+    a.line_first = c->line_first;
+    a.line_last = c->line_last;
+    a.line = c->d_line;
+  }
+  c->taux = a;
+  c->aux = true;
+  return true;
+}
+
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
-// shot whose CPML fits a tile's shared memory, unless a wave-front tracker
-// reads every step's field.  Measured on GB300 against the two-step path and
+// shot whose CPML fits a tile's shared memory.  Measured on GB300 against the two-step path and
 // the persistent kernel, Gcell/s: 1024^2 180 (85), 2048^2 327 (165), 4096^2
 // 457 (249), 8192^2 553 (315), F16 4096^2 471 (281), 8192^2 585 (413).
 // The compiled shapes are timed at create (a trial reads one buffer set and
 // writes the other, as a step does) and the choice kept per class.
 // FDTD2D_TILE=0: never; FDTD2D_TILE=R: the shape with R rows per warp.  Not
 // taken when another path is forced by name.
-int setup_tile(fdtd2d_ctx* c, int device) {
+int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
   const char* env = std::getenv("FDTD2D_TILE");
   if (env && std::strcmp(env, "0") == 0) return FDTD2D_OK;
   for (const char* v : {"FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_KERNEL"})
     if (std::getenv(v)) return FDTD2D_OK;
   if (const char* v = std::getenv("FDTD2D_PERSIST"); v && std::atoi(v) == 1) return FDTD2D_OK;
-  if (c->n_rc > 0) return FDTD2D_OK;
   int forced = -1;
   for (int k = 0; k < tile_shape_count(); ++k) {
     if (!tile_fits(c->h, k, device)) return FDTD2D_OK;
     if (env && std::atoi(env) == tile_shape_rows(k)) forced = k;
+  }
+  {
+    const std::vector<int32_t> scan(s->rc_scan_i, s->rc_scan_i + c->n_rc), most(s->rc_max_i, s->rc_max_i + c->n_rc);
+    if (!setup_aux(c, scan, most) && c->n_rc > 0) return FDTD2D_OK;   // (the probe alone: single steps in its window)
   }
   const int rc = setup_resident(c, device);
   if (rc) return rc;
@@ -963,7 +1017,7 @@ int setup_tile(fdtd2d_ctx* c, int device) {
       for (int r = 0; r <= reps && e == cudaSuccess; ++r) {
         if (r == 1) e = cudaEventRecord(e0, c->stream);
         if (e == cudaSuccess)
-          e = launch_step_tile(k, t, d, (int)tiles.size(), smem, t.base_n + 1, steps, c->stream);
+          e = launch_step_tile(k, t, d, (int)tiles.size(), smem, t.base_n + 1, steps, nullptr, c->stream);
       }
       if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
       if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -1659,7 +1713,7 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
   }
   CK(dalloc(c, &c->d_err, 1));
   std::vector<int4> units;
-  if (c->tma && !member) CK_RC(setup_tile(c, device));
+  if (c->tma && !member) CK_RC(setup_tile(c, s, device));
   if (c->tile) {
     // its own tiles
   } else if (c->tma) {
@@ -1812,37 +1866,53 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
     return FDTD2D_OK;
   }
   if (c->tile) {
+    // launches up to `stop`: until the tracker's history is full, or the line
+    // probe's window opens or closes where the kernels do not record it
     for (int32_t n = n_first; n <= n_last;) {
-      // single steps where something reads the fields after each of them
-      int k = n_last - n + 1;
-      if (c->line_n > 0 && n <= c->line_last && n + k > c->line_first) k = n < c->line_first ? c->line_first - n : 1;
-      const bool resident = c->resident && k >= kResidentSteps;
-      k = std::min(k, resident ? kPersistSteps : kTileSteps);
-      cudaEvent_t p0 = prof_mark(c, nullptr, 0, k);
-      const DevShot t = tile_view(c, n);
-      const cudaError_t e =
-          resident ? launch_ordered(c, [&] {
-            return launch_resident(t, c->rplan, n, k, c->d_link, c->d_err, c->wait_ns, c->bar_extra, c->stream);
-          })
-                   : launch_step_tile(c->tile_shape, t, c->d_tiles, c->n_tiles, c->tile_smem, n, k, c->stream);
-      if (p0) prof_mark(c, p0, (int64_t)c->nx * c->ny, k);
-      if (e != cudaSuccess) return fail_cuda(c, e);
-      ++c->launches;
-      if (k % 2 == 0) {
-        // an even number of steps: the buffers trade places, so that the
-        // state after step n is in slot n & 1 as everywhere else
-        std::swap(c->h.fb[0], c->h.fb[1]);
-        c->h.psi += c->h.psi_buf;
-        c->h.psi_buf = -c->h.psi_buf;
+      int32_t stop = n_last + 1;
+      const bool probe = c->line_n > 0 && !c->aux;
+      if (probe && n <= c->line_last && stop > c->line_first) stop = n < c->line_first ? c->line_first : n + 1;
+      if (c->n_rc > 0) stop = (int32_t)std::min<int64_t>(stop, (int64_t)n + c->rc_chunk);
+      const int32_t n0 = n;
+      TileAux aux = c->taux;
+      aux.n0 = n0;
+      while (n < stop) {
+        int k = stop - n;
+        const bool resident = c->resident && k >= kResidentSteps;
+        k = std::min(k, resident ? kPersistSteps : kTileSteps);
+        cudaEvent_t p0 = prof_mark(c, nullptr, 0, k);
+        const DevShot t = tile_view(c, n);
+        const TileAux* a = c->aux ? &aux : nullptr;
+        const cudaError_t e =
+            resident ? launch_ordered(c, [&] {
+              return launch_resident(t, c->rplan, n, k, a, c->d_link, c->d_err, c->wait_ns, c->bar_extra, c->stream);
+            })
+                     : launch_step_tile(c->tile_shape, t, c->d_tiles, c->n_tiles, c->tile_smem, n, k, a, c->stream);
+        if (p0) prof_mark(c, p0, (int64_t)c->nx * c->ny, k);
+        if (e != cudaSuccess) return fail_cuda(c, e);
+        ++c->launches;
+        if (k % 2 == 0) {
+          // an even number of steps: the buffers trade places, so that the
+          // state after step n is in slot n & 1 as everywhere else
+          std::swap(c->h.fb[0], c->h.fb[1]);
+          c->h.psi += c->h.psi_buf;
+          c->h.psi_buf = -c->h.psi_buf;
+        }
+        n += k;
+        c->step = n - 1;
       }
-      n += k;
-      c->step = n - 1;
-      if (c->line_n > 0 && c->step >= c->line_first && c->step <= c->line_last) {
-        const cudaError_t x = launch_line(field_ptr(c->h, kEz, c->step & 1), c->pitch, c->line_j, c->line_i0, c->line_n,
-                                          c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
-        if (x != cudaSuccess) return fail_cuda(c, x);
+      cudaError_t e = cudaSuccess;
+      if (c->n_rc > 0) {
+        e = launch_rc_steps(aux, c->ny, n - n0, c->n_rc, c->d_scan_slot, c->d_max_slot, c->rc_j_cut, c->rc_level, c->d_edge,
+                            c->d_cand, c->d_spd + (size_t)(n0 - 1) * c->n_rc, c->stream);
+        c->launches += 3;
+      }
+      if (e == cudaSuccess && probe && c->step >= c->line_first && c->step <= c->line_last) {
+        e = launch_line(field_ptr(c->h, kEz, c->step & 1), c->pitch, c->line_j, c->line_i0, c->line_n,
+                        c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
         ++c->launches;
       }
+      if (e != cudaSuccess) return fail_cuda(c, e);
     }
     return FDTD2D_OK;
   }

@@ -72,6 +72,13 @@ struct fdtd2d_ctx {
   int tile_shape = 0, n_tiles = 0;
   size_t tile_smem = 0;
   int4* d_tiles = nullptr;
+  // the tracker and the line probe recorded by the tile kernels: the history
+  // holds rc_chunk steps, worked off after them
+  bool aux = false;
+  fdtd2d::TileAux taux{};
+  int rc_chunk = 0;
+  int *d_scan_slot = nullptr, *d_max_slot = nullptr;
+  float* d_cand = nullptr;
   // the whole shot on chip for a run call's steps (step_resident.cu), beside the tiles
   bool resident = false;
   fdtd2d::ResidentPlan rplan{};

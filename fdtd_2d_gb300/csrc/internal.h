@@ -255,6 +255,24 @@ cudaError_t launch_step_tmat2(int shape, const DevShot& shot, const TensorMaps& 
 // Sets *ctr = 0.
 cudaError_t launch_frame(const DevShot& shot, int ci0, int ci1, int ri0, int ri1, int n_global, int* ctr,
                          cudaStream_t stream);
+// What the tile kernels record after every step beside the detectors: the
+// columns the wave-front tracker reads, whole, into `hist` ([step n - n0][n_cols]
+// [rows]; launch_rc_steps works them off after the launch), and the line probe's
+// row while its window is open.  Zero counts: nothing.
+struct TileAux {
+  int n_cols, rows, n0;       // rows: floats per column
+  const int* cols;            // [n_cols] distinct columns, at most kMaxTracked
+  float* hist;
+  int line_n, line_j, line_i0, line_first, line_last;
+  float* line;                // [n - line_first][line_n]
+};
+constexpr int kMaxTracked = 254;
+// The tracker over steps n0 .. n0+steps-1 of a column history: line l takes its
+// maximum from history column max_slot[l] and its scan from scan_slot[l]; cand:
+// steps * n_rc floats of scratch; spd: row of step n0.  launch_rc's values.
+cudaError_t launch_rc_steps(const TileAux& A, int ny, int steps, int n_rc, const int* scan_slot, const int* max_slot,
+                            int j_cut, float level, float* edge, float* cand, int* spd, cudaStream_t stream);
+
 // Several steps per pass on register tiles (step_tile.cu), in shapes that
 // differ in the rows of a plain tile: tiles (flags, c0, r0, u1) of 128 columns
 // from c0 and a band of rows from r0, storing rows up to u1.  A launch reads
@@ -267,8 +285,9 @@ int tile_shape_rows(int shape);   // rows per warp of its plain tiles
 std::vector<int4> make_tiles(const DevShot& s, int shape);
 size_t tile_smem(const DevShot& s, int shape);
 bool tile_fits(const DevShot& s, int shape, int device);
+// aux: null, or what to record (FP32 storage).
 cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
-                             int steps, cudaStream_t stream);
+                             int steps, const TileAux* aux, cudaStream_t stream);
 // The whole shot in the SMs' registers for many steps (step_resident.cu): nb
 // bands of w columns, each cut into strips of groups of R rows (a warp's).
 // The first and last band, whose columns hold the x strips, and the others
@@ -288,8 +307,8 @@ struct ResidentPlan {
 const std::vector<int>& resident_rows();
 // points: (column, row, PointKind) of the shot's sources and detectors.
 bool resident_plan(const DevShot& s, const std::vector<int3>& points, int R, int device, ResidentPlan* out);
-cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n_global, int steps, uint64_t* link, int* err,
-                            unsigned long long wait_ns, int tag_add, cudaStream_t stream);
+cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n_global, int steps, const TileAux* aux,
+                            uint64_t* link, int* err, unsigned long long wait_ns, int tag_add, cudaStream_t stream);
 // Launches the instantiation for shot.store.
 cudaError_t launch_step_tma(int shape, const DevShot& shot, const int4* units, int n_units, int n_global,
                             int max_ctas, int* err, cudaStream_t stream);

@@ -594,6 +594,85 @@ cudaError_t launch_rc(const float* ez, int64_t pitch, int ny, int n_rc, const in
   return cudaGetLastError();
 }
 
+// The tracker over many steps at once, from the columns the tile kernels
+// recorded.  A step's edge level is the running maximum of the candidates up to
+// it, so every (line, step) first forms its candidate, then takes the maximum
+// over the candidates before it and scans its column: two launches for a whole
+// run of steps, where rc_kernel took one of 8 us after every step.
+__global__ void __launch_bounds__(256) rc_max_steps_kernel(const TileAux A, int ny, const int* __restrict__ max_slot,
+                                                           int j_cut, float level, float* __restrict__ cand) {
+  __shared__ float s_max[8];
+  const int l = blockIdx.x, t = blockIdx.y, tid = threadIdx.x;
+  const float* col = A.hist + ((int64_t)t * A.n_cols + max_slot[l]) * A.rows;
+  float m = -INFINITY;
+#pragma unroll 4
+  for (int j = j_cut + tid; j < ny - 2; j += 256) m = fmaxf(m, col[j]);
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((tid & 31) == 0) s_max[tid >> 5] = m;
+  __syncthreads();
+  if (tid == 0) {
+    float temp = col[0];   // Dev_FindMax starts from row 0
+    for (int k = 0; k < 8; ++k)
+      if (s_max[k] > temp) temp = s_max[k];
+    cand[t * gridDim.x + l] = temp * level;
+  }
+}
+__global__ void __launch_bounds__(256) rc_scan_steps_kernel(const TileAux A, int ny, const int* __restrict__ scan_slot,
+                                                            const float* __restrict__ cand, const float* __restrict__ edge,
+                                                            int* __restrict__ spd) {
+  __shared__ float s_max[8];
+  __shared__ int s_best[8];
+  const int l = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, n_rc = gridDim.x;
+  float e = edge[l];
+  for (int q = tid; q <= t; q += 256) {
+    const float c = cand[q * n_rc + l];
+    if (c > e) e = c;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const float c = __shfl_xor_sync(0xffffffffu, e, o);
+    if (c > e) e = c;
+  }
+  if ((tid & 31) == 0) s_max[tid >> 5] = e;
+  __syncthreads();
+  for (int k = 0; k < 8; ++k)
+    if (s_max[k] > e) e = s_max[k];
+  const float* col = A.hist + ((int64_t)t * A.n_cols + scan_slot[l]) * A.rows;
+  int best = 0;
+#pragma unroll 4
+  for (int j = 1 + tid; j <= ny - 3; j += 256)
+    if (!(fabsf(col[j]) < e)) best = j;
+  for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if ((tid & 31) == 0) s_best[tid >> 5] = best;
+  __syncthreads();
+  if (tid == 0) {
+    for (int k = 1; k < 8; ++k) best = max(best, s_best[k]);
+    spd[t * n_rc + l] = best;
+  }
+}
+__global__ void rc_edge_steps_kernel(const float* __restrict__ cand, int steps, int n_rc, float* edge) {
+  for (int l = threadIdx.x >> 5; l < n_rc; l += blockDim.x >> 5) {
+    float e = edge[l];
+    for (int q = threadIdx.x & 31; q < steps; q += 32) {
+      const float c = cand[q * n_rc + l];
+      if (c > e) e = c;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float c = __shfl_xor_sync(0xffffffffu, e, o);
+      if (c > e) e = c;
+    }
+    if ((threadIdx.x & 31) == 0) edge[l] = e;
+  }
+}
+
+cudaError_t launch_rc_steps(const TileAux& A, int ny, int steps, int n_rc, const int* scan_slot, const int* max_slot,
+                            int j_cut, float level, float* edge, float* cand, int* spd, cudaStream_t stream) {
+  const dim3 grid(n_rc, steps);
+  rc_max_steps_kernel<<<grid, 256, 0, stream>>>(A, ny, max_slot, j_cut, level, cand);
+  rc_scan_steps_kernel<<<grid, 256, 0, stream>>>(A, ny, scan_slot, cand, edge, spd);
+  rc_edge_steps_kernel<<<1, 1024, 0, stream>>>(cand, steps, n_rc, edge);
+  return cudaGetLastError();
+}
+
 __global__ void line_kernel(const float* __restrict__ ez, int64_t pitch, int j, int i0, int n,
                             float* __restrict__ dst) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)

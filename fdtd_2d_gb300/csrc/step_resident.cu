@@ -332,8 +332,8 @@ struct ResPoints {
   }
 };
 
-template <int R, bool LOSSLESS>
-__device__ __forceinline__ void resident_run(const DevShot& S, const ResidentPlan& G, int n, int steps, uint64_t* link,
+template <int R, bool LOSSLESS, bool AUX>
+__device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A, const ResidentPlan& G, int n, int steps, uint64_t* link,
                                              const Waiter& wait, uint32_t tag_add, float4* smem, int* slots) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x;
   const int nx = S.nx, ny = S.ny;
@@ -426,6 +426,7 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const ResidentPla
   const bool take_l = l && b > 0, take_r = rr && b + 1 < G.nb;
   const int col_at = (rr ? rows : 0) + row0;
 
+  const unsigned tracked = AUX && work ? tile_tracked(A, p.i, own) : 0u;
   // the loop in the form the warp needs
   auto loop = [&](auto x, auto y) {
     for (int t = 0; t < steps; ++t) {
@@ -437,6 +438,7 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const ResidentPla
         for (int r = 0; r < R; ++r) E.col_out[col_at + r] = l ? s.ez[r + 1][1] : s.ez[r + 1][2];
       }
       bar_arrive(1, threads);
+      if (AUX && t > 0) tile_record<R, JS>(s, A, tracked, p, own, r0, min(r0 + rows, ny - 1), n + t - 1);
       if (pts.state) {
         if (t > 0) pts.detectors<R, JS>(s, S, n + t - 1, lane);
         pts.load_step<R>(S, n + t, lane);
@@ -468,6 +470,7 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const ResidentPla
     if (!p.y) loop(Yes{}, No{});
     else loop(Yes{}, Yes{});
   }
+  if (AUX) tile_record<R, JS>(s, A, tracked, p, own, r0, min(r0 + rows, ny - 1), n + steps - 1);
   if (pts.state) {
     pts.detectors<R, JS>(s, S, n + steps - 1, lane);
     pts.end<R>(S, lane);
@@ -491,29 +494,34 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const ResidentPla
   tile_psi_io<R, true, false>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, r0, min(r0 + rows, ny - 1));
 }
 
-template <int R, bool LOSSLESS>
+template <int R, bool LOSSLESS, bool AUX>
 __global__ void __launch_bounds__(all_warps(R) * 32, 1)
-step_persist_tile_kernel(const __grid_constant__ DevShot S, const __grid_constant__ ResidentPlan G, int n_global, int steps,
+step_persist_tile_kernel(const __grid_constant__ DevShot S, const __grid_constant__ TileAux A,
+                         const __grid_constant__ ResidentPlan G, int n_global, int steps,
                          uint64_t* link, int* err, unsigned long long wait_ns, int tag_add) {
   extern __shared__ float4 smem[];
   __shared__ int dead, slots;
   if (threadIdx.x == 0) dead = slots = 0;
   __syncthreads();
   const Waiter wait{&dead, err, wait_ns};
-  resident_run<R, LOSSLESS>(S, G, n_global - S.base_n, steps, link, wait, (uint32_t)tag_add, smem, &slots);
+  resident_run<R, LOSSLESS, AUX>(S, A, G, n_global - S.base_n, steps, link, wait, (uint32_t)tag_add, smem, &slots);
 }
 
-template <int R>
+template <int R, bool AUX>
 const void* resident_kernel(const DevShot& s) {
-  return s.ca == 1.f && s.da == 1.f ? (const void*)step_persist_tile_kernel<R, true>
-                                    : (const void*)step_persist_tile_kernel<R, false>;
+  return s.ca == 1.f && s.da == 1.f ? (const void*)step_persist_tile_kernel<R, true, AUX>
+                                    : (const void*)step_persist_tile_kernel<R, false, AUX>;
 }
-const void* resident_kernel(int R, const DevShot& s) {
+template <int R>
+const void* resident_kernel(const DevShot& s, bool aux) {
+  return aux ? resident_kernel<R, true>(s) : resident_kernel<R, false>(s);
+}
+const void* resident_kernel(int R, const DevShot& s, bool aux) {
   switch (R) {
-    case 8: return resident_kernel<8>(s);
-    case 6: return resident_kernel<6>(s);
-    case 4: return resident_kernel<4>(s);
-    default: return resident_kernel<2>(s);
+    case 8: return resident_kernel<8>(s, aux);
+    case 6: return resident_kernel<6>(s, aux);
+    case 4: return resident_kernel<4>(s, aux);
+    default: return resident_kernel<2>(s, aux);
   }
 }
 
@@ -651,9 +659,9 @@ int resident_ctas(const ResidentPlan& p) {
   return edges * p.ns[0] + (p.nb - edges) * p.ns[1];
 }
 
-cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n_global, int steps, uint64_t* link, int* err,
-                            unsigned long long wait_ns, int tag_add, cudaStream_t stream) {
-  const void* fn = resident_kernel(plan.R, shot);
+cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n_global, int steps, const TileAux* aux,
+                            uint64_t* link, int* err, unsigned long long wait_ns, int tag_add, cudaStream_t stream) {
+  const void* fn = resident_kernel(plan.R, shot, aux != nullptr);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem);
   // tags count from 1 in every launch: clear the words of earlier ones
   if (e == cudaSuccess) e = cudaMemsetAsync(link, 0, (size_t)plan.link_words * sizeof(uint64_t), stream);
@@ -661,7 +669,8 @@ cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n
   DevShot s = shot;
   ResidentPlan g = plan;
   if (wait_ns == 0) wait_ns = kWaitNs;
-  void* args[] = {&s, &g, &n_global, &steps, &link, &err, &wait_ns, &tag_add};
+  TileAux a = aux ? *aux : TileAux{};
+  void* args[] = {&s, &a, &g, &n_global, &steps, &link, &err, &wait_ns, &tag_add};
   return cudaLaunchCooperativeKernel(fn, dim3(resident_ctas(plan)), dim3((plan.nw + 1) * 32), args, (size_t)plan.smem, stream);
 }
 

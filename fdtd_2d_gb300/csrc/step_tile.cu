@@ -49,8 +49,8 @@ __device__ __forceinline__ void load4(float (&d)[4], const T* p, bool in) {
   }
 }
 
-template <int R, int NW, bool JS, bool LOSSLESS, bool PLAIN, class T>
-__device__ __forceinline__ void tile_pass(const DevShot& S, const int4 tile, int n, int steps, float4* smem) {
+template <int R, int NW, bool JS, bool LOSSLESS, bool PLAIN, bool AUX, class T>
+__device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, const int4 tile, int n, int steps, float4* smem) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int rows = NW * R, threads = NW * 32;
   const int c0 = tile.y, r0 = tile.z, u0 = max(r0 + kHalo, 0), u1 = tile.w;
@@ -109,6 +109,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const int4 tile, int
     p0 = __ldg(S.row_start + max(j0, 0));
     p1 = __ldg(S.row_start + min(j0 + R, ny));
   }
+  const unsigned slots = AUX ? tile_tracked(A, p.i, own) : 0u;
   // the loop in the form the warp needs (its barriers pair across the forms)
   auto loop = [&](auto x, auto y) {
     for (int t = 0; t < steps; ++t) {
@@ -121,6 +122,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const int4 tile, int
       get4(s.ez[R + 1], e[(warp < NW - 1 ? 2 * warp + 2 : 2 * warp + 1) * 32 + lane]);
       tile_step<R, JS, LOSSLESS, decltype(x)::value, decltype(y)::value, T>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, threads, lane);
       if (p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, own, u0, u1);
+      if (AUX) tile_record<R, JS>(s, A, slots, p, own, u0, u1, n + t);
       tile_round<R, JS, T>(s);
     }
   };
@@ -158,31 +160,33 @@ struct Tile {
   static constexpr int kRows = RP;
 };
 
-template <class Shape, bool LOSSLESS, class T>
+template <class Shape, bool LOSSLESS, bool AUX, class T>
 __global__ void __launch_bounds__(kWarps * 32, 2)
-step_tmat_kernel(const __grid_constant__ DevShot S, const int4* __restrict__ tiles, int n_global, int steps) {
+step_tmat_kernel(const __grid_constant__ DevShot S, const __grid_constant__ TileAux A, const int4* __restrict__ tiles, int n_global, int steps) {
   extern __shared__ float4 smem[];
   const int4 tile = __ldg(tiles + blockIdx.x);
   const int n = n_global - S.base_n;
   if (tile.x & kTilePlain) {
-    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, T>(S, tile, n, steps, smem);
+    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, AUX, T>(S, A, tile, n, steps, smem);
   } else {
-    tile_pass<kREdge, kWarps, false, LOSSLESS, false, T>(S, tile, n, steps, smem);
+    tile_pass<kREdge, kWarps, false, LOSSLESS, false, AUX, T>(S, A, tile, n, steps, smem);
   }
 }
 
 bool lossless(const DevShot& s) { return s.ca == 1.f && s.da == 1.f; }
 
-template <int RP, class T>
+template <int RP, bool AUX, class T>
 const void* tile_kernel(const DevShot& s) {
-  return lossless(s) ? (const void*)step_tmat_kernel<Tile<RP>, true, T> : (const void*)step_tmat_kernel<Tile<RP>, false, T>;
+  return lossless(s) ? (const void*)step_tmat_kernel<Tile<RP>, true, AUX, T> : (const void*)step_tmat_kernel<Tile<RP>, false, AUX, T>;
 }
 template <int RP>
-const void* tile_kernel(const DevShot& s) {
-  return s.store == 0 ? tile_kernel<RP, float>(s) : s.store == 1 ? tile_kernel<RP, __half>(s) : tile_kernel<RP, __nv_bfloat16>(s);
+const void* tile_kernel(const DevShot& s, bool aux) {
+  if (aux) return s.store == 0 ? tile_kernel<RP, true, float>(s) : nullptr;
+  return s.store == 0 ? tile_kernel<RP, false, float>(s)
+       : s.store == 1 ? tile_kernel<RP, false, __half>(s) : tile_kernel<RP, false, __nv_bfloat16>(s);
 }
-const void* tile_kernel(int shape, const DevShot& s) {
-  return shape == 0 ? tile_kernel<kShapes[0]>(s) : tile_kernel<kShapes[1]>(s);
+const void* tile_kernel(int shape, const DevShot& s, bool aux) {
+  return shape == 0 ? tile_kernel<kShapes[0]>(s, aux) : tile_kernel<kShapes[1]>(s, aux);
 }
 
 }  // namespace
@@ -238,13 +242,15 @@ bool tile_fits(const DevShot& s, int shape, int device) {
 }
 
 cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
-                             int steps, cudaStream_t stream) {
+                             int steps, const TileAux* aux, cudaStream_t stream) {
   if (steps < 1 || steps > kTileSteps || n_tiles <= 0) return cudaErrorInvalidValue;
-  const void* fn = tile_kernel(shape, shot);
+  const void* fn = tile_kernel(shape, shot, aux != nullptr);
+  if (!fn) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   DevShot s = shot;
-  void* args[] = {&s, (void*)&tiles, &n_global, &steps};
+  TileAux a = aux ? *aux : TileAux{};
+  void* args[] = {&s, &a, (void*)&tiles, &n_global, &steps};
   return cudaLaunchKernel(fn, dim3(n_tiles), dim3(kWarps * 32), args, smem, stream);
 }
 

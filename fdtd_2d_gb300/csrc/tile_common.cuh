@@ -458,6 +458,47 @@ __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S
   }
 }
 
+// Slots of the thread's columns in the tracked list (TileAux::cols), 8 bits per
+// column, 0 for none: the columns of the mask `own`.
+__device__ __forceinline__ unsigned tile_tracked(const TileAux& A, int i, unsigned own) {
+  unsigned slots = 0;
+  for (int u = 0; u < A.n_cols; ++u) {
+    const int k = __ldg(A.cols + u) - i;
+    if (k >= 0 && k < 4 && (own >> k & 1)) slots |= (unsigned)(u + 1) << 8 * k;
+  }
+  return slots;
+}
+
+// Records state n of the rows [u0, u1) among the thread's: its tracked columns
+// and its part of the line probe.
+template <int R, bool JS>
+__device__ __forceinline__ void tile_record(const TileRegs<R, JS>& s, const TileAux& A, unsigned slots, const TilePos& p,
+                                            unsigned own, int u0, int u1, int n) {
+  if (slots) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int u = slots >> 8 * k & 255;
+      if (!u) continue;
+      float* h = A.hist + ((int64_t)(n - A.n0) * A.n_cols + u - 1) * A.rows + p.j0;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (p.j0 + r >= u0 && p.j0 + r < u1) h[r] = s.ez[r + 1][k];
+    }
+  }
+  if (A.line_n > 0 && n >= A.line_first && n <= A.line_last && A.line_j >= max(u0, p.j0) && A.line_j < min(u1, p.j0 + R)) {
+    float* dst = A.line + (int64_t)(n - A.line_first) * A.line_n;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (p.j0 + r != A.line_j) continue;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = p.i + k - A.line_i0;
+        if ((own >> k & 1) && c >= 0 && c < A.line_n) dst[c] = s.ez[r + 1][k];
+      }
+    }
+  }
+}
+
 // 16-bit storage: the values a store and a load would give back.
 template <int R, bool JS, class T>
 __device__ __forceinline__ void tile_round(TileRegs<R, JS>& s) {

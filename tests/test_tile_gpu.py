@@ -162,3 +162,50 @@ def test_tile_line_probe_and_components(gpu, monkeypatch):
     _, ref = stepped()
     for a, b in zip(got, ref):
         assert np.array_equal(a, b)
+
+
+def test_tracker_and_probe_recorded(gpu, monkeypatch, tmp_path):
+    """The wave-front tracker and the line probe recorded by the tile kernels, on
+    chip and in passes (a Settings.ini shot of 500 x 1200 cells with 21 tracker
+    lines; run calls shorter and longer than the history): the streaming
+    kernel's rows, probe samples, traces and fields."""
+    import re
+    from pathlib import Path
+
+    ini = (Path(__file__).resolve().parent / "golden" / "sphere_fluc_chirp" / "Settings.ini").read_text()
+    for key, val in (("Imax", "250"), ("Jmax", "600"), ("Use_Exp_time", "0"), ("Max_time", "420")):
+        ini = re.sub(rf"(?m)^{key}\s*=.*$", f"{key} = {val}", ini)
+    path = tmp_path / "Settings.ini"
+    path.write_text(ini)
+    prob = F.Problem.from_ini(path)
+    s = prob.setup
+    assert (s.nx, s.ny) == (500, 1200) and s.n_rc > 0
+    s.line_n, s.line_i0, s.line_j, s.line_first, s.line_last = 400, 50, 700, 120, 180
+
+    def stepped():
+        with F.Shot(prob, gpu) as shot:
+            n = 1
+            for c in (1, 100, 7, 300, 12):
+                shot.run(n, n + c - 1)
+                n += c
+            out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+            out.update(shot.traces())
+            out["rc"], out["line"] = shot.rc(), shot.line(120, 180)
+            return shot.kernel_name(), out
+
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE", "FDTD2D_RESIDENT"):
+        monkeypatch.delenv(v, raising=False)
+    name, on_chip = stepped()
+    assert name.startswith("step_persist_kernel<0>/tile<"), name
+    monkeypatch.setenv("FDTD2D_TILE", "7")
+    name, passes = stepped()
+    assert name == "step_tmat_kernel<tile,7>", name
+    monkeypatch.setenv("FDTD2D_TILE", "0")
+    monkeypatch.setenv("FDTD2D_KERNEL", "stream")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = stepped()
+    assert name == "step_stream_kernel<0>", name
+    assert ref["rc"].max() > 0
+    for k in ref:
+        assert np.array_equal(ref[k], on_chip[k]), ("on chip", k)
+        assert np.array_equal(ref[k], passes[k]), ("passes", k)
