@@ -1714,8 +1714,8 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
   CK(dalloc(c, &c->d_err, 1));
   std::vector<int4> units;
   if (c->tma && !member) CK_RC(setup_tile(c, s, device));
-  if (c->tile) {
-    // its own tiles
+  if (c->tile || member) {
+    // its own tiles; a batch member is stepped by the batch's kernel
   } else if (c->tma) {
     // FDTD2D_TMA="W,ST" picks a compiled launch shape (W warps, ST stages);
     // otherwise the shapes are timed on this shot and the fastest is kept,
@@ -1723,9 +1723,7 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
     const int forced = tma_shape_parse(std::getenv("FDTD2D_TMA"));
     const char* at = std::getenv("FDTD2D_TMA_AUTOTUNE");
     KernelChoice known;
-    if (member) {
-      // batch members are stepped by the batch's kernel
-    } else if (forced >= 0) {
+    if (forced >= 0) {
       c->tma_shape = forced;
     } else if (!(at && std::strcmp(at, "0") == 0) && c->n_steps >= 1 &&
                find_choice(choice_key(c, device, "tma"), &known)) {

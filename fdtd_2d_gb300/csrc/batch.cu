@@ -3,18 +3,15 @@
 // The reference runs one shot per process (global state, FDTD_2D_Full/
 // kernel.cu:1928-2818).  A batch owns many shots, each a full fdtd2d_ctx
 // (fields, CPML state, tables, traces and DFT accumulators resident in HBM),
-// and advances all of them with one persistent launch per time step of the
-// staged kernel (step_tma_batch_kernel): units (shot, band, row range) of every
-// unfinished shot are handed out dynamically to the resident CTAs, and each
-// shot runs its own step n = global step - its admission step, so shots
-// admitted at different times advance together (continuous batching).  Steps
-// are issued in blocks of K launches captured once as a CUDA graph; the block
-// base lives in device memory and the graph's last node advances it, so the
-// same graph serves every block.  Admission is by a device-memory budget.
+// and advances all of them with one launch per pass of up to four time steps
+// (step_tile.cu's batch kernel): the register tiles of every unfinished shot in
+// one grid, each shot at its own step n = global step - its admission step, so
+// shots admitted at different times advance together (continuous batching).
+// Admission is by a device-memory budget.
 //
-// Host-side state changes (admit, finish, remove) take effect at block
-// boundaries: the unit list is rebuilt on the host and uploaded on the batch's
-// stream before the next block, which the same graph then reads.
+// Host-side state changes (admit, finish, remove) take effect between passes:
+// the tile list is rebuilt on the host and uploaded in the order of the batch's
+// stream before the next pass; nothing waits for the device.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -30,12 +27,6 @@ using namespace fdtd2d;
 namespace {
 
 constexpr int kMaxShots = 512;     // descriptor slots per batch
-constexpr int kBlockSteps = 16;    // launches per captured step block
-
-// Misc device words of a batch.
-enum Misc : int { kNUnits = 0, kGStep = 1, kCtr0 = 2, kCtr1 = 3, kErr = 4, kMiscWords = 8 };
-
-__global__ void advance_gstep(int* gstep, int k) { *gstep += k; }
 
 struct Member {
   fdtd2d_ctx* ctx = nullptr;
@@ -43,6 +34,9 @@ struct Member {
   int32_t base = 0;     // global steps issued before its first step
   bool live = false;
   bool done = false;    // all its steps issued
+  // its register tiles (a member of the batch kernel) and the passes issued
+  std::vector<int4> tiles;
+  int32_t passes = 0;
   // A solo member is a full single shot on its own streams (the tensor path:
   // two steps per pass where it wins), stepped by fdtd2d_run from the batch's
   // run calls; `ev` holds the events recorded after its recent run calls on
@@ -80,17 +74,21 @@ struct fdtd2d_batch {
   std::vector<Member> m;
   std::vector<DevShot> h_shots;        // host copies of the slots' descriptors
   DevShot* d_shots = nullptr;          // [kMaxShots]
-  DevShot* d_trial = nullptr;          // [kMaxShots] descriptors for launch-shape trials
-  int4* d_units = nullptr;
-  int unit_cap = 0, n_units = 0;
-  int* d_misc = nullptr;               // Misc words for the real steps
-  int* d_tmisc = nullptr;              // and for the trials
+  int4* d_tiles = nullptr;
+  int tile_cap = 0, n_tiles = 0;
+  // the list's host copies, pinned: two, so that one can be filled while the
+  // stream still copies from the other (its event marks that copy)
+  struct Staging {
+    int4* p = nullptr;
+    int cap = 0;
+    cudaEvent_t ev = nullptr;
+  } staging[2];
+  int next_staging = 0;
+  size_t smem = 0;
+  bool lossless = true;                // CA = DA = 1 in every member
   int32_t g = 0;                       // global steps issued
-  int shape = 0;
-  bool tuned = false;
-  int ctas = 0, max_pml = 1;
+  int32_t passes = 0;                  // and passes
   bool dirty = true;
-  std::map<int, cudaGraphExec_t> graphs;
   int64_t launches = 0;
   int last_cuda = 0;
   char name[64] = {0};
@@ -104,134 +102,73 @@ int fail(fdtd2d_batch* b, cudaError_t e) {
   return e == cudaErrorMemoryAllocation ? FDTD2D_ERR_NOMEM : FDTD2D_ERR_CUDA;
 }
 
-void drop_graphs(fdtd2d_batch* b) {
-  for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
-  b->graphs.clear();
-}
+// Shape of the members' plain tiles: 7 rows per warp (8192^2: 560 Gcell/s, 490
+// with 5).
+constexpr int kBatchShape = 0;
 
-// Units of one shot for band width `band` and `rows` rows per unit.
-void shot_units(std::vector<int4>& u, int slot, int nx, int ny, int band, int rows) {
-  const int bands = (nx + band - 1) / band;
-  const int total = ny - 1;
-  const int strips = std::max(1, (total + rows - 1) / rows);
-  for (int s = 0; s < strips; ++s) {
-    const int j0 = (int)((int64_t)total * s / strips), j1 = (int)((int64_t)total * (s + 1) / strips);
-    if (j1 <= j0) continue;
-    for (int c = 0; c < bands; ++c) u.push_back(make_int4(slot, c * band, j0, j1));
-  }
-}
-
-// Unit list of every live shot with steps left, for launch shape `shape`:
-// rows per unit chosen for about 6 units per resident CTA (16..512 rows).
-std::vector<int4> build_units(const fdtd2d_batch* b, int shape, int ctas) {
-  const int band = tma_band_cols(shape);
-  int64_t band_rows = 0;
-  for (const Member& x : b->m)
-    if (x.live && !x.done && !x.solo) band_rows += (int64_t)((x.ctx->nx + band - 1) / band) * (x.ctx->ny - 1);
-  int rows = (int)std::min<int64_t>(512, std::max<int64_t>(16, (band_rows + 6LL * ctas - 1) / (6LL * ctas)));
-  std::vector<int4> u;
+// The tile list of every live shot with steps left, tiles with CPML work (the
+// slower ones) of all shots first, uploaded in the stream's order.
+int upload_tiles(fdtd2d_batch* b) {
+  int n = 0;
+  b->smem = 0;
+  b->lossless = true;
   for (int k = 0; k < (int)b->m.size(); ++k) {
     const Member& x = b->m[k];
-    if (x.live && !x.done && !x.solo) shot_units(u, k, x.ctx->nx, x.ctx->ny, band, rows);
+    if (!x.live || x.done || x.solo) continue;
+    const DevShot& s = b->h_shots[k];
+    n += (int)x.tiles.size();
+    b->smem = std::max(b->smem, tile_smem(s, kBatchShape));
+    b->lossless = b->lossless && s.ca == 1.f && s.da == 1.f;
   }
-  return u;
-}
-
-int upload_units(fdtd2d_batch* b, const std::vector<int4>& u, int* misc) {
-  if ((int)u.size() > b->unit_cap) {
-    cudaStreamSynchronize(b->stream);
-    if (b->d_units) cudaFree(b->d_units);
-    b->d_units = nullptr;
-    const int cap = std::max<int>((int)u.size() * 2, 1024);
-    cudaError_t e = cudaMalloc(&b->d_units, (size_t)cap * sizeof(int4));
-    if (e != cudaSuccess) return fail(b, e);
-    b->unit_cap = cap;
-    drop_graphs(b);   // they hold the old pointer
-  }
-  static thread_local std::vector<int4> staging;
-  staging = u;   // pageable source: cudaMemcpyAsync stages it before returning
-  const int n = (int)u.size();
   cudaError_t e = cudaSuccess;
-  if (n) e = cudaMemcpyAsync(b->d_units, staging.data(), (size_t)n * sizeof(int4), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(misc + kNUnits, &n, sizeof(int), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);   // n lives on this stack frame
+  fdtd2d_batch::Staging& st = b->staging[b->next_staging];
+  if (!st.ev) e = cudaEventCreateWithFlags(&st.ev, cudaEventDisableTiming);
+  else e = cudaEventSynchronize(st.ev);   // the list before the last one has been copied
+  if (e == cudaSuccess && n > st.cap) {
+    if (st.p) cudaFreeHost(st.p);
+    st.p = nullptr;
+    st.cap = 0;
+    const int cap = std::max(n * 2, 4096);
+    e = cudaHostAlloc(&st.p, (size_t)cap * sizeof(int4), cudaHostAllocDefault);
+    if (e == cudaSuccess) st.cap = cap;
+  }
+  if (e == cudaSuccess && n > b->tile_cap) {
+    // (stream-ordered: the passes issued before still read the old list)
+    if (b->d_tiles) cudaFreeAsync(b->d_tiles, b->stream);
+    b->d_tiles = nullptr;
+    b->tile_cap = 0;
+    const int cap = std::max(n * 2, 4096);
+    e = cudaMallocAsync(&b->d_tiles, (size_t)cap * sizeof(int4), b->stream);
+    if (e == cudaSuccess) b->tile_cap = cap;
+  }
   if (e != cudaSuccess) return fail(b, e);
+  int at = 0;
+  for (int plain = 0; plain < 2; ++plain)
+    for (int k = 0; k < (int)b->m.size(); ++k) {
+      const Member& x = b->m[k];
+      if (!x.live || x.done || x.solo) continue;
+      for (const int4& t : x.tiles)
+        if (((t.x & kTilePlain) != 0) == (plain != 0)) st.p[at++] = make_int4(t.x | k << kTileSlot, t.y, t.z, t.w);
+    }
+  if (n) e = cudaMemcpyAsync(b->d_tiles, st.p, (size_t)n * sizeof(int4), cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess) e = cudaEventRecord(st.ev, b->stream);
+  if (e != cudaSuccess) return fail(b, e);
+  b->n_tiles = n;
+  b->next_staging ^= 1;
+  b->dirty = false;
   return FDTD2D_OK;
 }
 
-// Time every compiled launch shape on the batch's next step (traces and DFT
-// off; a step reads one buffer set and overwrites the other, so re-running
-// the next step leaves nothing behind) and keep the fastest.
-int autotune(fdtd2d_batch* b) {
-  std::vector<DevShot> t = b->h_shots;
-  for (DevShot& d : t) {
-    d.record = 0;
-    d.dft = nullptr;
-  }
-  cudaError_t e = cudaMemcpyAsync(b->d_trial, t.data(), t.size() * sizeof(DevShot), cudaMemcpyHostToDevice,
-                                  b->stream);
-  if (e != cudaSuccess) return fail(b, e);
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  float best = 0.f;
-  int best_k = 0;
-  int rc = FDTD2D_OK;
-  for (int k = 0; k < tma_shape_count() && rc == FDTD2D_OK; ++k) {
-    const int ctas = tma_batch_resident_ctas(k, b->max_pml, b->device);
-    const std::vector<int4> u = build_units(b, k, ctas);
-    rc = upload_units(b, u, b->d_tmisc);
-    if (rc) break;
-    const int g = b->g;
-    e = cudaMemcpyAsync(b->d_tmisc + kGStep, &g, sizeof(int), cudaMemcpyHostToDevice, b->stream);
-    for (int r = 0; r < 3 && e == cudaSuccess; ++r) {
-      if (r == 1) e = cudaEventRecord(e0, b->stream);
-      if (e == cudaSuccess)
-        e = launch_step_tma_batch(k, b->d_trial, b->d_units, b->d_tmisc + kNUnits, b->d_tmisc + kGStep, 0,
-                                  b->d_tmisc + kCtr0, b->max_pml, ctas, b->d_tmisc + kErr, b->stream);
-      // the trial re-runs the same step: clear its unit counter between runs
-      if (e == cudaSuccess) e = cudaMemsetAsync(b->d_tmisc + kCtr0, 0, 2 * sizeof(int), b->stream);
-    }
-    if (e == cudaSuccess) e = cudaEventRecord(e1, b->stream);
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-    float ms = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-    if (e != cudaSuccess) rc = fail(b, e);
-    if (rc == FDTD2D_OK && (k == 0 || ms < best)) {
-      best = ms;
-      best_k = k;
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (rc) return rc;
-  int err = 0;
-  e = cudaMemcpy(&err, b->d_tmisc + kErr, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return fail(b, e);
-  if (err) return FDTD2D_ERR_TIMEOUT;
-  b->shape = best_k;
-  b->tuned = true;
-  b->dirty = true;
-  drop_graphs(b);
-  return FDTD2D_OK;
-}
-
-cudaError_t capture_block(fdtd2d_batch* b, int K, cudaGraphExec_t* out) {
-  cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) return e;
-  for (int k = 0; k < K && e == cudaSuccess; ++k)
-    e = launch_step_tma_batch(b->shape, b->d_shots, b->d_units, b->d_misc + kNUnits, b->d_misc + kGStep, k,
-                              b->d_misc + kCtr0, b->max_pml, b->ctas, b->d_misc + kErr, b->stream);
-  if (e == cudaSuccess) {
-    advance_gstep<<<1, 1, 0, b->stream>>>(b->d_misc + kGStep, K);
-    e = cudaGetLastError();
-  }
-  const cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
-  if (e == cudaSuccess) e = ee;
-  if (e == cudaSuccess) e = cudaGraphInstantiate(out, graph, 0);
-  if (graph) cudaGraphDestroy(graph);
-  return e;
+// A member's host descriptor after a pass: the state after step n is in slot
+// n & 1 for the readers, whatever buffer its passes have left it in (slot
+// `passes & 1` of the descriptor it was admitted with, which the kernel reads).
+void settle(Member& x, const DevShot& s) {
+  DevShot& h = x.ctx->h;
+  const int at = x.passes & 1, slot = x.ctx->step & 1;
+  h.fb[slot] = s.fb[at];
+  h.fb[slot ^ 1] = s.fb[at ^ 1];
+  h.psi = at == slot ? s.psi : s.psi + s.psi_buf;
+  h.psi_buf = at == slot ? s.psi_buf : -s.psi_buf;
 }
 
 int add_solo(fdtd2d_batch* b, const fdtd2d_setup* s, int64_t bytes, int32_t* shot) {
@@ -351,14 +288,10 @@ int fdtd2d_batch_create(int device, int64_t hbm_budget_bytes, fdtd2d_batch** out
   std::memset(b->h_shots.data(), 0, kMaxShots * sizeof(DevShot));
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_shots, kMaxShots * sizeof(DevShot));
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_trial, kMaxShots * sizeof(DevShot));
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_misc, 2 * kMiscWords * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(b->d_misc, 0, 2 * kMiscWords * sizeof(int));
   if (e != cudaSuccess) {
     fdtd2d_batch_destroy(b);
     return e == cudaErrorMemoryAllocation ? FDTD2D_ERR_NOMEM : FDTD2D_ERR_CUDA;
   }
-  b->d_tmisc = b->d_misc + kMiscWords;
   *out = b;
   return FDTD2D_OK;
 }
@@ -406,17 +339,16 @@ static int fdtd2d_batch_add_body(fdtd2d_batch* b, const fdtd2d_setup* s, int32_t
   x.base = b->g;
   x.live = true;
   x.done = false;
+  x.passes = 0;
   c->h.base_n = b->g;
+  c->h.base_pass = b->passes;
+  x.tiles = make_tiles(c->h, kBatchShape);
   b->h_shots[slot] = c->h;
   cudaSetDevice(b->device);
   cudaError_t e = cudaMemcpyAsync(b->d_shots + slot, &b->h_shots[slot], sizeof(DevShot), cudaMemcpyHostToDevice,
                                   b->stream);
   if (e != cudaSuccess) return fail(b, e);
   b->used += bytes;
-  if (s->npml > b->max_pml) {
-    b->max_pml = s->npml;
-    drop_graphs(b);
-  }
   b->dirty = true;
   *shot = slot;
   return FDTD2D_OK;
@@ -440,50 +372,25 @@ static int fdtd2d_batch_run_body(fdtd2d_batch* b, int32_t n_steps) {
     bool any = false;
     for (const Member& x : b->m) any = any || (x.live && !x.done && !x.solo);
     if (!any) return FDTD2D_OK;
-    if (!b->tuned) {
-      const int forced = tma_shape_parse(std::getenv("FDTD2D_TMA"));
-      if (forced >= 0) {
-        b->shape = forced;
-        b->tuned = true;
-      } else {
-        const int rc = autotune(b);
-        if (rc) return rc;
-      }
-    }
-    const int ctas = tma_batch_resident_ctas(b->shape, b->max_pml, b->device);
-    if (ctas != b->ctas) {
-      b->ctas = ctas;
-      drop_graphs(b);
-    }
     if (b->dirty) {
-      const std::vector<int4> u = build_units(b, b->shape, b->ctas);
-      const int rc = upload_units(b, u, b->d_misc);
+      const int rc = upload_tiles(b);
       if (rc) return rc;
-      b->n_units = (int)u.size();
-      b->dirty = false;
-      // the shape's counters may hold a trial's values
-      cudaError_t e = cudaMemsetAsync(b->d_misc + kCtr0, 0, 2 * sizeof(int), b->stream);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_misc + kGStep, &b->g, sizeof(int), cudaMemcpyHostToDevice, b->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-      if (e != cudaSuccess) return fail(b, e);
     }
-    const int K = std::min<int>(n_steps, kBlockSteps);
-    auto it = b->graphs.find(K);
-    if (it == b->graphs.end()) {
-      cudaGraphExec_t ge = nullptr;
-      const cudaError_t e = capture_block(b, K, &ge);
-      if (e != cudaSuccess) return fail(b, e);
-      it = b->graphs.emplace(K, ge).first;
-    }
-    const cudaError_t e = cudaGraphLaunch(it->second, b->stream);
+    const int K = std::min<int>(n_steps, kTileSteps);
+    const cudaError_t e = launch_batch_tile(kBatchShape, b->lossless, b->d_shots, b->d_tiles, b->n_tiles, b->smem, b->g, K,
+                                            b->passes, b->stream);
     if (e != cudaSuccess) return fail(b, e);
     b->g += K;
-    b->launches += K;
+    ++b->passes;
+    ++b->launches;
     n_steps -= K;
-    for (Member& x : b->m) {
-      if (!x.live || x.solo) continue;
-      x.ctx->step = std::min(x.ctx->n_steps, std::max(0, b->g - x.base));
-      if (!x.done && x.ctx->step >= x.ctx->n_steps) {
+    for (int k = 0; k < (int)b->m.size(); ++k) {
+      Member& x = b->m[k];
+      if (!x.live || x.solo || x.done) continue;
+      x.ctx->step = std::min(x.ctx->n_steps, b->g - x.base);
+      ++x.passes;
+      settle(x, b->h_shots[k]);
+      if (x.ctx->step >= x.ctx->n_steps) {
         x.done = true;
         b->dirty = true;
       }
@@ -500,12 +407,8 @@ int fdtd2d_batch_synchronize(fdtd2d_batch* b) {
       const int rc = fdtd2d_synchronize(x.ctx);
       if (rc) return rc;
     }
-  cudaError_t e = cudaStreamSynchronize(b->stream);
-  if (e != cudaSuccess) return fail(b, e);
-  int err = 0;
-  e = cudaMemcpy(&err, b->d_misc + kErr, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return fail(b, e);
-  return err ? FDTD2D_ERR_TIMEOUT : FDTD2D_OK;
+  const cudaError_t e = cudaStreamSynchronize(b->stream);
+  return e == cudaSuccess ? FDTD2D_OK : fail(b, e);
 }
 
 fdtd2d_ctx* fdtd2d_batch_shot(fdtd2d_batch* b, int32_t shot) {
@@ -536,9 +439,7 @@ int64_t fdtd2d_batch_launch_count(const fdtd2d_batch* b) { return b ? b->launche
 
 const char* fdtd2d_batch_kernel_name(const fdtd2d_batch* b) {
   if (!b) return "";
-  int w = 0, st = 0;
-  tma_shape_dims(b->shape, &w, &st);
-  std::snprintf(const_cast<char*>(b->name), sizeof b->name, "step_tma_batch_kernel<%d,%d>", w, st);
+  std::snprintf(const_cast<char*>(b->name), sizeof b->name, "step_tma_batch_kernel<tile,%d>", tile_shape_rows(kBatchShape));
   return b->name;
 }
 
@@ -551,11 +452,12 @@ int fdtd2d_batch_destroy(fdtd2d_batch* b) {
       fdtd2d_destroy(x.ctx);
       release_events(x);
     }
-  drop_graphs(b);
-  if (b->d_units) cudaFree(b->d_units);
+  for (auto& st : b->staging) {
+    if (st.ev) cudaEventDestroy(st.ev);
+    if (st.p) cudaFreeHost(st.p);
+  }
+  if (b->d_tiles) cudaFreeAsync(b->d_tiles, b->stream);
   if (b->d_shots) cudaFree(b->d_shots);
-  if (b->d_trial) cudaFree(b->d_trial);
-  if (b->d_misc) cudaFree(b->d_misc);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return FDTD2D_OK;
@@ -635,23 +537,18 @@ int retire(fdtd2d_server* s, int* n_done) {
       continue;
     }
     fdtd2d_ctx* c = b->m[x.slot].ctx;
-    // A shot whose kernels gave up on a bounded wait has skipped work: its
-    // results are not handed out (the batch kernel's error word for its
-    // members, a solo member's own one), and the call reports the timeout.
-    // A solo member's word was allocated and zeroed on its own stream
-    // (stream-ordered, from the pool): it is read in that stream's order,
-    // which has completed.  The batch's word comes from cudaMalloc and a
-    // synchronous memset; reading it does not wait for the queued blocks.
-    int derr = 0;
-    cudaError_t re;
+    // A solo member whose kernels gave up on a bounded wait has skipped work:
+    // its results are not handed out, and the call reports the timeout (the
+    // batch's own kernel waits for nothing).  The word was allocated and zeroed
+    // on the member's own stream: it is read in that stream's order, which has
+    // completed.
     if (mem.solo) {
-      re = cudaMemcpyAsync(&derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+      int derr = 0;
+      cudaError_t re = cudaMemcpyAsync(&derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
       if (re == cudaSuccess) re = cudaStreamSynchronize(c->stream);
-    } else {
-      re = cudaMemcpy(&derr, b->d_misc + kErr, sizeof(int), cudaMemcpyDeviceToHost);
+      if (re != cudaSuccess) return fail(b, re);
+      if (derr) return FDTD2D_ERR_TIMEOUT;
     }
-    if (re != cudaSuccess) return fail(b, re);
-    if (derr) return FDTD2D_ERR_TIMEOUT;
     Finished f;
     f.tag = x.tag;
     f.n_det = c->n_det;
@@ -807,9 +704,6 @@ static int fdtd2d_server_step_body(fdtd2d_server* s) {
     rc = retire(s, &n_done);
     if (rc) return rc;
   }
-  int err = 0;
-  if (cudaMemcpy(&err, b->d_misc + kErr, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && err)
-    return FDTD2D_ERR_TIMEOUT;
   return n_done;
 }
 

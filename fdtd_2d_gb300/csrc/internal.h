@@ -34,6 +34,7 @@ struct DevShot {
   int nx, ny, pitch, npml;
   int n_steps;
   int base_n;                 // global step offset (batched/serving shots)
+  int base_pass;              // and pass offset (launch_batch_tile)
   float ca, cb, da, db;       // uniform medium coefficients
   float ja;                   // Jz decay (1 - nu dt/2)/(1 + nu dt/2)
   float dx, dy;               // the float dx, dy the reference passes to the psi kernels
@@ -288,6 +289,15 @@ bool tile_fits(const DevShot& s, int shape, int device);
 // aux: null, or what to record (FP32 storage).
 cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
                              int steps, const TileAux* aux, cudaStream_t stream);
+// A pass of a batch: every shot in `shots` (FP32) by up to `steps` steps after
+// global step g, shot s by its own steps g + 1 - base_n on, at most to its last
+// one.  tiles: (flags | slot << kTileSlot, c0, r0, u1).  pass: the batch's passes
+// before this one; a shot's state is in fb[q] and psi + q psi_buf, q the parity of
+// its own passes (pass - base_pass).  lossless: CA = DA = 1 in every shot.
+constexpr int kTileSlot = 8;
+cudaError_t launch_batch_tile(int shape, bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
+                              int g, int steps, int pass, cudaStream_t stream);
+
 // The whole shot in the SMs' registers for many steps (step_resident.cu): nb
 // bands of w columns, each cut into strips of groups of R rows (a warp's).
 // The first and last band, whose columns hold the x strips, and the others
@@ -312,14 +322,6 @@ cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n
 // Launches the instantiation for shot.store.
 cudaError_t launch_step_tma(int shape, const DevShot& shot, const int4* units, int n_units, int n_global,
                             int max_ctas, int* err, cudaStream_t stream);
-// Batched form: one launch advances every shot in `shots` by one step, units
-// (shot, c0, j0, j1) handed out dynamically; n_global = *gstep + k + 1.
-// counters: 2 ints, zero before the first launch.
-cudaError_t launch_step_tma_batch(int shape, const DevShot* shots, const int4* units, const int* n_units,
-                                  const int* gstep, int k, int* counters, int max_pml, int ctas, int* err,
-                                  cudaStream_t stream);
-int tma_batch_resident_ctas(int shape, int max_pml, int device);
-
 // Tabulate s_e(n) = scale*env[n]*cos(2*pi_c*(beta/2 t^2 + f0 t + phase_e)),
 // t = n*dt, for n = 0..n_steps, and the DFT twiddles, in FP64.
 cudaError_t build_source_tables(float* src_val, double2* twiddle, const float* env,

@@ -173,6 +173,35 @@ step_tmat_kernel(const __grid_constant__ DevShot S, const __grid_constant__ Tile
   }
 }
 
+// The same for the shots of a batch: the tile's shot from a device array, its
+// own step and the buffers its passes so far have left it in.
+template <class Shape, bool LOSSLESS>
+__global__ void __launch_bounds__(kWarps * 32, 2)
+step_tma_batch_kernel(const DevShot* __restrict__ shots, const int4* __restrict__ tiles, int g, int steps, int pass) {
+  extern __shared__ float4 smem[];
+  __shared__ __align__(16) DevShot S;
+  const int4 tile = __ldg(tiles + blockIdx.x);
+  const int* src = reinterpret_cast<const int*>(shots + (tile.x >> kTileSlot));
+  for (int t = threadIdx.x; t < (int)(sizeof(DevShot) / 4); t += kWarps * 32) reinterpret_cast<int*>(&S)[t] = __ldg(src + t);
+  __syncthreads();
+  if (threadIdx.x == 0 && ((pass - S.base_pass) & 1)) {
+    float* f = S.fb[0];
+    S.fb[0] = S.fb[1];
+    S.fb[1] = f;
+    S.psi += S.psi_buf;
+    S.psi_buf = -S.psi_buf;
+  }
+  __syncthreads();
+  const int n = g + 1 - S.base_n, k = min(steps, S.n_steps - n + 1);
+  if (k <= 0) return;
+  const TileAux none{};
+  if (tile.x & kTilePlain) {
+    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, false, float>(S, none, tile, n, k, smem);
+  } else {
+    tile_pass<kREdge, kWarps, false, LOSSLESS, false, false, float>(S, none, tile, n, k, smem);
+  }
+}
+
 bool lossless(const DevShot& s) { return s.ca == 1.f && s.da == 1.f; }
 
 template <int RP, bool AUX, class T>
@@ -251,6 +280,20 @@ cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, 
   DevShot s = shot;
   TileAux a = aux ? *aux : TileAux{};
   void* args[] = {&s, &a, (void*)&tiles, &n_global, &steps};
+  return cudaLaunchKernel(fn, dim3(n_tiles), dim3(kWarps * 32), args, smem, stream);
+}
+
+cudaError_t launch_batch_tile(int shape, bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
+                              int g, int steps, int pass, cudaStream_t stream) {
+  if (steps < 1 || steps > kTileSteps) return cudaErrorInvalidValue;
+  if (n_tiles <= 0) return cudaSuccess;
+  const void* fn = shape == 0 ? (lossless ? (const void*)step_tma_batch_kernel<Tile<kShapes[0]>, true>
+                                          : (const void*)step_tma_batch_kernel<Tile<kShapes[0]>, false>)
+                              : (lossless ? (const void*)step_tma_batch_kernel<Tile<kShapes[1]>, true>
+                                          : (const void*)step_tma_batch_kernel<Tile<kShapes[1]>, false>);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&shots, &tiles, &g, &steps, &pass};
   return cudaLaunchKernel(fn, dim3(n_tiles), dim3(kWarps * 32), args, smem, stream);
 }
 

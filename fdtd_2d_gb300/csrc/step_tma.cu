@@ -470,74 +470,13 @@ step_tma_kernel(const __grid_constant__ DevShot S, const int4* __restrict__ unit
   }
 }
 
-// Batched form: one launch advances every shot of a batch by one step.  The
-// shots' descriptors sit in a device array; units (shot, c0, j0, j1) are
-// handed out dynamically (one atomic counter per step parity, so CTAs that
-// drew short or fast units take more); each shot runs its own step
-// n = n_global - base_n, and units of shots outside [1, n_steps] are skipped,
-// so shots admitted at different times advance together.  n_global is read
-// from device memory (the step-block base, advanced by the graph's last node)
-// plus the launch's offset k within the block, so one captured graph of K
-// launches serves every block.
-template <class C>
-__global__ void __launch_bounds__(C::kThreads, C::kMinBlocks)
-step_tma_batch_kernel(const DevShot* __restrict__ shots, const int4* __restrict__ units,
-                      const int* __restrict__ n_units_p, const int* __restrict__ gstep_p, int k, int* counters,
-                      int* err) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t full[C::kStages], empty[C::kStages];
-  __shared__ __align__(16) DevShot sS;
-  __shared__ int s_unit;
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    for (int s = 0; s < C::kStages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], C::kWarps);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  const int n_global = *gstep_p + k + 1;
-  const int n_units = *n_units_p;
-  int* ctr = counters + (n_global & 1);
-  if (blockIdx.x == 0 && tid == 0) counters[(n_global + 1) & 1] = 0;   // the next step's counter
-  __syncthreads();
-  Ring R;
-  R.stage = smem;
-  R.full = full;
-  R.empty = empty;
-  float* cp = reinterpret_cast<float*>(smem + C::kStages * C::kStageBytes);   // CPML table of the current shot
-  int cur = -1;
-  for (;;) {
-    if (tid == 0) s_unit = *(volatile int*)err ? n_units : atomicAdd(ctr, 1);
-    __syncthreads();
-    const int u = s_unit;
-    if (u >= n_units) break;
-    const int4 ud = __ldg(units + u);
-    if (ud.x != cur) {
-      const int* src = reinterpret_cast<const int*>(shots + ud.x);
-      int* dst = reinterpret_cast<int*>(&sS);
-      for (int t = tid; t < (int)(sizeof(DevShot) / 4); t += C::kThreads) dst[t] = __ldg(src + t);
-      __syncthreads();
-      for (int t = tid; t < kCpmlRows * sS.npml; t += C::kThreads) cp[t] = sS.cpml[t];
-      cur = ud.x;
-      __syncthreads();
-    }
-    const int n = n_global - sS.base_n;
-    if (n >= 1 && n <= sS.n_steps) process_band<C>(sS, R, cp, ud.y, ud.z, ud.w, n, err);
-    __syncthreads();   // every thread has read s_unit (and sS) before the next unit overwrites them
-  }
-}
-
 using KernelFn = void (*)(DevShot, const int4*, int, int, int*);
-using BatchFn = void (*)(const DevShot*, const int4*, const int*, const int*, int, int*, int*);
 
-// One launch shape: the single-shot kernel per storage type (F32, F16,
-// BF16) and the batched kernel (F32 storage).
+// One launch shape: the kernel per storage type (F32, F16, BF16).
 struct ShapeEntry {
   int warps, stages;
   KernelFn fn[3];
   size_t smem[3];
-  BatchFn bfn;
 };
 
 template <int W, int ST>
@@ -546,7 +485,7 @@ constexpr ShapeEntry entry() {
   using C16 = Cfg<W, ST, __half>;
   using CB16 = Cfg<W, ST, __nv_bfloat16>;
   return {W, ST, {step_tma_kernel<C32>, step_tma_kernel<C16>, step_tma_kernel<CB16>},
-          {C32::kSmem, C16::kSmem, CB16::kSmem}, step_tma_batch_kernel<C32>};
+          {C32::kSmem, C16::kSmem, CB16::kSmem}};
 }
 
 // Compiled launch shapes; the first is the default.
@@ -598,26 +537,6 @@ cudaError_t launch_step_tma(int shape, const DevShot& shot, const int4* units, i
   e.fn[st]<<<ctas, e.warps * 32, smem_bytes(e.smem[st], shot.npml), stream>>>(shot, units, n_units, n_global,
                                                                             err);
   return cudaGetLastError();
-}
-
-cudaError_t launch_step_tma_batch(int shape, const DevShot* shots, const int4* units, const int* n_units,
-                                  const int* gstep, int k, int* counters, int max_pml, int ctas, int* err,
-                                  cudaStream_t stream) {
-  const ShapeEntry& e = kShapes[shape];
-  e.bfn<<<ctas, e.warps * 32, smem_bytes(e.smem[0], max_pml), stream>>>(shots, units, n_units, gstep, k, counters,
-                                                                         err);
-  return cudaGetLastError();
-}
-
-int tma_batch_resident_ctas(int shape, int max_pml, int device) {
-  const ShapeEntry& e = kShapes[shape];
-  const size_t smem = smem_bytes(e.smem[0], max_pml);
-  cudaFuncSetAttribute(e.bfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(e.smem[0], kTmaMaxPml));
-  int sms = 0, per_sm = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, e.bfn, e.warps * 32, smem);
-  if (per_sm < 1) per_sm = 1;
-  return sms * per_sm;
 }
 
 int tma_resident_ctas(int shape, int npml, int store, int device) {
