@@ -414,7 +414,8 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A,
       if (JS) jzs[r * wt] = put4(jv);
     }
   }
-  if (work) tile_psi_io<R, false, false>(S, S.psi, p, psi, rows, row0, 0, 0, 0);
+  if (work) tile_psi_load<R, false>(S, S.psi, p, psi, rows, row0);
+  copies_done();
   // rows around the strip that nobody sends (beyond the grid, or its last row) stay as loaded
   if (work && warp == 0 && k == 0) E.row_in[lane] = put4(s.ez[0]);
   if (work && warp == nw - 1 && !has_u) E.row_in[32 + lane] = put4(s.ez[R + 1]);
@@ -491,7 +492,7 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A,
       field_ptr(S, kJz, 1)[o] = JS ? jv[q] : s.jz[JS ? 0 : r][q];
     }
   }
-  tile_psi_io<R, true, false>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, r0, min(r0 + rows, ny - 1));
+  tile_psi_store<R, false>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, r0, min(r0 + rows, ny - 1));
 }
 
 template <int R, bool LOSSLESS, bool AUX>

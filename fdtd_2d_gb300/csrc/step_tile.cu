@@ -67,40 +67,54 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
   float* tr = tc + kTcRows * kTileCols;
   const TilePsi psi = tile_psi(rest + tile_table_f4(rows), p, rows, R, lane);
 
+  // Everything the tile reads is asked for together: drive, Jz (JS) and psi by
+  // copies into shared memory (FP32; 16-bit elements pass through registers to be
+  // converted), the fields into registers.
   TileRegs<R, JS> s;
-  {
-    const bool in = PLAIN || (p.i >= 0 && p.i < nx);
-    const T* ez = field_ptr_t<T>(S, kEz, 0) + p.i;
-    const T* hx = field_ptr_t<T>(S, kHx, 0) + p.i;
-    const T* hy = field_ptr_t<T>(S, kHy, 0) + p.i;
-    const T* jz = field_ptr_t<T>(S, kJz, 0) + p.i;
-    const T* kp = reinterpret_cast<const T*>(S.kp);
-    load4(s.hx[0], hx + (int64_t)(j0 - 1) * pitch, in && (PLAIN || (j0 >= 1 && j0 <= ny)));
-    float kv[R][4], jv[JS ? R : 1][4];
+  constexpr bool kCopy = sizeof(T) == 4;
+  const bool in = PLAIN || (p.i >= 0 && p.i < nx);
+  const T* ez = field_ptr_t<T>(S, kEz, 0) + p.i;
+  const T* hx = field_ptr_t<T>(S, kHx, 0) + p.i;
+  const T* hy = field_ptr_t<T>(S, kHy, 0) + p.i;
+  const T* jz = field_ptr_t<T>(S, kJz, 0) + p.i;
+  const T* kp = reinterpret_cast<const T*>(S.kp);
+  if (!PLAIN) tile_psi_load<R, true>(S, S.psi, p, psi, rows, row0);
+  float kv[kCopy ? 1 : R][4], jv[JS && !kCopy ? R : 1][4];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int j = j0 + r;
-      const bool ok = in && (PLAIN || (j >= 0 && j < ny));
-      const int64_t o = (int64_t)j * pitch;
-      load4(s.ez[r + 1], ez + o, ok);
-      load4(s.hx[r + 1], hx + o, ok);
-      load4(s.hy[r], hy + o, ok);
-      if (JS) load4(jv[r], jz + o, ok); else load4(s.jz[JS ? 0 : r], jz + o, ok);
-      load4(kv[r], kp + p.i + o, ok && kp != nullptr);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (sizeof(T) == 2) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) kv[r][k] = __fmul_rn(kv[r][k], C.rk);
-      }
-      kps[r * threads] = put4(kv[r]);
-      if (JS) jzs[r * threads] = put4(jv[JS ? r : 0]);
+  for (int r = 0; r < R; ++r) {
+    const int j = j0 + r;
+    const bool ok = in && (PLAIN || (j >= 0 && j < ny));
+    const int64_t o = (int64_t)j * pitch;
+    if (kCopy) {
+      const bool has = ok && kp != nullptr;
+      copy16(kps + r * threads, has ? (const void*)(kp + p.i + o) : (const void*)S.fb[0], has);
+      if (JS) copy16(jzs + r * threads, ok ? (const void*)(jz + o) : (const void*)S.fb[0], ok);
+    } else {
+      load4(kv[kCopy ? 0 : r], kp + p.i + o, ok && kp != nullptr);
+      if (JS) load4(jv[JS && !kCopy ? r : 0], jz + o, ok);
     }
   }
-  if (!PLAIN) {
-    tile_tables<T>(S, C, tc, tr, c0, r0, rows, tid, threads);
-    tile_psi_io<R, false, true>(S, S.psi, p, psi, rows, row0, 0, 0, 0);
+  load4(s.hx[0], hx + (int64_t)(j0 - 1) * pitch, in && (PLAIN || (j0 >= 1 && j0 <= ny)));
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int j = j0 + r;
+    const bool ok = in && (PLAIN || (j >= 0 && j < ny));
+    const int64_t o = (int64_t)j * pitch;
+    load4(s.ez[r + 1], ez + o, ok);
+    load4(s.hx[r + 1], hx + o, ok);
+    load4(s.hy[r], hy + o, ok);
+    if (!JS) load4(s.jz[JS ? 0 : r], jz + o, ok);
+  }
+  if (!PLAIN) tile_tables<T>(S, C, tc, tr, c0, r0, rows, tid, threads);
+  if (!kCopy) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float (&v)[4] = kv[kCopy ? 0 : r];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = __fmul_rn(v[k], C.rk);
+      kps[r * threads] = put4(v);
+      if (JS) jzs[r * threads] = put4(jv[JS && !kCopy ? r : 0]);
+    }
   }
   // lanes whose columns are stored
   const unsigned own = lane >= kHalo / 4 && lane < 32 - kHalo / 4 && p.i < nx ? 15u : 0u;
@@ -109,6 +123,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
     p0 = __ldg(S.row_start + max(j0, 0));
     p1 = __ldg(S.row_start + min(j0 + R, ny));
   }
+  copies_done();   // (a thread reads only what it copied)
   const unsigned slots = AUX ? tile_tracked(A, p.i, own) : 0u;
   // the loop in the form the warp needs (its barriers pair across the forms)
   auto loop = [&](auto x, auto y) {
@@ -131,28 +146,28 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
   else if (!p.x) loop(No{}, Yes{});
   else loop(Yes{}, Yes{});
   if (own) {
-    T* ez = field_ptr_t<T>(S, kEz, 1) + p.i;
-    T* hx = field_ptr_t<T>(S, kHx, 1) + p.i;
-    T* hy = field_ptr_t<T>(S, kHy, 1) + p.i;
-    T* jz = field_ptr_t<T>(S, kJz, 1) + p.i;
+    T* ez_w = field_ptr_t<T>(S, kEz, 1) + p.i;
+    T* hx_w = field_ptr_t<T>(S, kHx, 1) + p.i;
+    T* hy_w = field_ptr_t<T>(S, kHy, 1) + p.i;
+    T* jz_w = field_ptr_t<T>(S, kJz, 1) + p.i;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int j = j0 + r;
       if (j < u0 || j >= u1) continue;
       const int64_t o = (int64_t)j * pitch;
-      Sto<T>::stcs4(ez + o, s.ez[r + 1]);
-      Sto<T>::stcs4(hx + o, s.hx[r + 1]);
-      Sto<T>::stcs4(hy + o, s.hy[r]);
+      Sto<T>::stcs4(ez_w + o, s.ez[r + 1]);
+      Sto<T>::stcs4(hx_w + o, s.hx[r + 1]);
+      Sto<T>::stcs4(hy_w + o, s.hy[r]);
       if (JS) {
         float v[4];
         get4(v, jzs[r * threads]);
-        Sto<T>::stcs4(jz + o, v);
+        Sto<T>::stcs4(jz_w + o, v);
       } else {
-        Sto<T>::stcs4(jz + o, s.jz[JS ? 0 : r]);
+        Sto<T>::stcs4(jz_w + o, s.jz[JS ? 0 : r]);
       }
     }
   }
-  if (!PLAIN) tile_psi_io<R, true, true>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, u0, u1);
+  if (!PLAIN) tile_psi_store<R, true>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, u0, u1);
 }
 
 template <int RP>

@@ -165,79 +165,125 @@ __device__ __forceinline__ void tile_tables(const DevShot& S, const Coef<T>& C, 
     const int n = col ? nx : ny;
     float* out = col ? tc + t : tr + (t - kTileCols);
     const int st = col ? kTileCols : rows + 1;
-    float bh = 0.f, ch = 0.f, be = 0.f, ce = 0.f, de = 0.f, dh = 0.f;
+    // every entry's six loads are issued together, from a clamped place where
+    // there is none
     const int h0 = col ? kBhX1 : kBhY1, e0 = col ? kBeX1 : kBeY1;
-    if (c >= 0 && c <= P - 2) { bh = S.cpml[h0 * P + c]; ch = S.cpml[(h0 + 1) * P + c]; }
-    else if (c >= n - P && c <= n - 2) { bh = S.cpml[(h0 + 2) * P + n - 2 - c]; ch = S.cpml[(h0 + 3) * P + n - 2 - c]; }
-    if (c >= 1 && c <= P - 1) { be = S.cpml[e0 * P + c]; ce = S.cpml[(e0 + 1) * P + c]; }
-    else if (c >= n - P && c <= n - 2) { be = S.cpml[(e0 + 2) * P + n - 1 - c]; ce = S.cpml[(e0 + 3) * P + n - 1 - c]; }
-    if (c >= 0 && c < n - 1) { de = (col ? S.den_ex : S.den_ey)[c]; dh = (col ? S.den_hx : S.den_hy)[c]; }
+    const bool lo_h = c >= 0 && c <= P - 2, hi_h = c >= n - P && c <= n - 2;
+    const bool lo_e = c >= 1 && c <= P - 1, hi_e = hi_h, in = c >= 0 && c < n - 1;
+    const int qh = lo_h ? h0 * P + c : hi_h ? (h0 + 2) * P + n - 2 - c : 0;
+    const int qe = lo_e ? e0 * P + c : hi_e ? (e0 + 2) * P + n - 1 - c : 0;
+    const int qd = in ? c : 0;
+    float bh = __ldg(S.cpml + qh), ch = __ldg(S.cpml + qh + P), be = __ldg(S.cpml + qe), ce = __ldg(S.cpml + qe + P);
+    float de = __ldg((col ? S.den_ex : S.den_ey) + qd), dh = __ldg((col ? S.den_hx : S.den_hy) + qd);
+    if (!(lo_h || hi_h)) bh = ch = 0.f;
+    if (!(lo_e || hi_e)) be = ce = 0.f;
+    if (!in) de = dh = 0.f;
     out[kTcBh * st] = bh; out[kTcCh * st] = __fmul_rn(ch, C.sE); out[kTcBe * st] = be; out[kTcCe * st] = __fmul_rn(ce, C.sH);
     out[kTcDe * st] = de; out[kTcDh * st] = dh;
   }
 }
 
-// psi of the tile from (STORE false) or to the slab; stored: the columns of
-// the mask `own` in rows [u0, u1).  ALIGNED: the thread's first column is a
-// multiple of 4 (then `own` is all or none).
-template <int R, bool STORE, bool ALIGNED>
-__device__ __forceinline__ void tile_psi_io(const DevShot& S, float* slab, const TilePos& p, const TilePsi& psi, int rows,
-                                            int row0, unsigned own, int u0, int u1) {
+// Copies of 4 and 16 bytes into shared memory, without a register or a wait
+// (cp.async; the issuing thread waits for its own with copies_done()).  The
+// 16-byte form gives zeros where `in` is false and reads nothing.
+__device__ __forceinline__ void copy4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool in) {
+  const int n = in ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// psi of the tile from the slab, every slot of the thread (copies in flight at
+// return), and back: the columns of the mask `own` in rows [u0, u1).  ALIGNED:
+// the thread's first column is a multiple of 4 (then `own` is all or none).
+// (A load at a time in a loop, each waiting for the one before, made up half the
+// time of a pass's CPML tiles.)
+template <int R, bool ALIGNED>
+__device__ __forceinline__ void tile_psi_load(const DevShot& S, const float* slab, const TilePos& p, const TilePsi& psi,
+                                              int rows, int row0) {
   const int nx = S.nx, ny = S.ny, P = S.npml;
   const int64_t pitch = S.pitch;
-#pragma unroll 1
-  for (int r = -1; r < R; ++r) {
-    const int j = p.j0 + r;
-    if (STORE && (r < 0 || j < u0 || j >= u1 || !own)) continue;
-    const bool row = j >= 0 && j <= ny - 1;
-    // x strips: Hy, Ez
-    if (r >= 0 && p.strip()) {
+  if (p.strip()) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = p.j0 + r;
+      const bool row = j >= 0 && j <= ny - 1;
 #pragma unroll
       for (int f = 0; f < 2; ++f) {
-        float4* ps = psi.x + (f * rows + row0 + r) * p.nxl + p.xslot;
-        float v[4];
-        if (STORE) get4(v, *ps); else zero4(v);
+        float* ps = reinterpret_cast<float*>(psi.x + (f * rows + row0 + r) * p.nxl + p.xslot);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          if (!row || !(f ? p.xe(k) : p.xh(k)) || (STORE && !(own >> k & 1))) continue;
           const int c = p.i + k;
           const int side = c >= P ? 1 : 0, q = side ? nx - (f ? 1 : 2) - c : c;
-          float* g = slab + (f ? S.o_ezx : S.o_hyx) + ((int64_t)side * ny + j) * P + q;
-          if (STORE) *g = v[k]; else v[k] = __ldcg(g);
+          if (row && (f ? p.xe(k) : p.xh(k))) copy4(ps + k, slab + (f ? S.o_ezx : S.o_hyx) + ((int64_t)side * ny + j) * P + q);
+          else ps[k] = 0.f;
         }
-        if (!STORE) *ps = put4(v);
       }
     }
-    // y strips: Hx, Ez
-    if (!p.y) continue;
+  }
+  if (p.y) {
 #pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      if (r < 0 && f) continue;
-      const bool strip = f ? y_strip_e(j, ny, P) : y_strip_h(j, ny, P);
-      if (STORE && !strip) continue;
-      const int side = j >= P ? 1 : 0, q = side ? ny - (f ? 1 : 2) - j : j;
-      float* g = slab + (f ? S.o_ezy + ((int64_t)side * P + q) * pitch : ((int64_t)side * (P - 1) + q) * pitch) + p.i;
-      float4* ps = psi.y + (f ? R + 1 + r : r + 1) * 32;
-      if (ALIGNED) {   // a thread left of column 0 holds no strip cell
-        const bool in = p.i >= 0 && p.i < nx;
-        if (STORE) {
-          if (in) *reinterpret_cast<float4*>(g) = *ps;
+    for (int r = -1; r < R; ++r) {
+      const int j = p.j0 + r;
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        if (r < 0 && f) continue;
+        const bool strip = f ? y_strip_e(j, ny, P) : y_strip_h(j, ny, P);
+        const int side = j >= P ? 1 : 0, q = side ? ny - (f ? 1 : 2) - j : j;
+        const float* g = slab + (strip ? (f ? S.o_ezy + ((int64_t)side * P + q) * pitch : ((int64_t)side * (P - 1) + q) * pitch) + p.i : 0);
+        float4* ps = psi.y + (f ? R + 1 + r : r + 1) * 32;
+        if (ALIGNED) {   // a thread left of column 0 holds no strip cell
+          const bool in = strip && p.i >= 0 && p.i < nx;
+          copy16(ps, in ? g : slab, in);
         } else {
-          *ps = strip && in ? __ldcg(reinterpret_cast<const float4*>(g)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      } else {
-        float v[4];
-        if (STORE) get4(v, *ps);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const bool in = p.i + k >= 0 && p.i + k < nx;
-          if (STORE) {
-            if (in && (own >> k & 1)) g[k] = v[k];
-          } else {
-            v[k] = strip && in ? __ldcg(g + k) : 0.f;
+          for (int k = 0; k < 4; ++k) {
+            if (strip && p.i + k >= 0 && p.i + k < nx) copy4(reinterpret_cast<float*>(ps) + k, g + k);
+            else reinterpret_cast<float*>(ps)[k] = 0.f;
           }
         }
-        if (!STORE) *ps = put4(v);
+      }
+    }
+  }
+}
+
+template <int R, bool ALIGNED>
+__device__ __forceinline__ void tile_psi_store(const DevShot& S, float* slab, const TilePos& p, const TilePsi& psi, int rows,
+                                               int row0, unsigned own, int u0, int u1) {
+  const int nx = S.nx, ny = S.ny, P = S.npml;
+  const int64_t pitch = S.pitch;
+  if (!own) return;
+#pragma unroll 1
+  for (int r = 0; r < R; ++r) {
+    const int j = p.j0 + r;
+    if (j < u0 || j >= u1) continue;
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      if (p.strip()) {
+        float v[4];
+        get4(v, psi.x[(f * rows + row0 + r) * p.nxl + p.xslot]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (!(f ? p.xe(k) : p.xh(k)) || !(own >> k & 1)) continue;
+          const int c = p.i + k;
+          const int side = c >= P ? 1 : 0, q = side ? nx - (f ? 1 : 2) - c : c;
+          slab[(f ? S.o_ezx : S.o_hyx) + ((int64_t)side * ny + j) * P + q] = v[k];
+        }
+      }
+      if (p.y && (f ? y_strip_e(j, ny, P) : y_strip_h(j, ny, P))) {
+        const int side = j >= P ? 1 : 0, q = side ? ny - (f ? 1 : 2) - j : j;
+        float* g = slab + (f ? S.o_ezy + ((int64_t)side * P + q) * pitch : ((int64_t)side * (P - 1) + q) * pitch) + p.i;
+        const float4 v = psi.y[(f ? R + 1 + r : r + 1) * 32];
+        if (ALIGNED) {
+          if (p.i >= 0 && p.i < nx) *reinterpret_cast<float4*>(g) = v;
+        } else {
+          const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if ((own >> k & 1) && p.i + k >= 0 && p.i + k < nx) g[k] = w[k];
+        }
       }
     }
   }
