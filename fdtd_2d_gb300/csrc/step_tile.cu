@@ -18,10 +18,13 @@
 //
 // Bytes: 20 x (halo) + 16 per stored cell and 4 steps, 10.1 B per cell-update
 // with R = 7 (the two-step path 18).  Measured on GB300 against that path,
-// Gcell/s: 8192^2 FP32 553 (315), F16 585 (413); 4096^2 457 (249) and 471
-// (281); 2048^2 327 (165).  R = 4 (Jz in registers) 504, 5 491, 6 520, 8 485
-// at 8192^2 FP32.  FP32 moves 5.6 TB/s of tile traffic there, 0.82 of the copy
-// peak; 16-bit storage is bound by its instructions.
+// Gcell/s: 8192^2 FP32 571 (315), F16 610 (413); 4096^2 511 (249) and 513
+// (281); 2048^2 406 (165).  Bound by latency at 16 warps per SM: a 4096^2 pass
+// issues in 49 % of the cycles, DRAM moves 4.2 TB/s (0.62 of the copy peak); the
+// loads of a tile take a third of its time, overlapped with the SM's other CTA.
+// Rows per warp at 8192^2 FP32 when this was chosen: 4 (Jz in registers) 504, 5
+// 491, 6 520, 7 553, 8 485; CTAs of CPML tiles with 5 or 6 rows need the shared
+// memory of two (363, 370).
 #include <algorithm>
 
 #include "internal.h"
@@ -40,12 +43,25 @@ constexpr int kRowsEdge = kREdge * kWarps;
 constexpr int kShapes[] = {7, 5};
 constexpr int kNumShapes = 2;
 
+// Waits until the launches before this one in its stream have ended (this one
+// may have been started beside the last of them) and what they wrote is visible,
+// then lets the next one start.  (After the wait, so that at most two launches
+// overlap.)
+__device__ __forceinline__ void earlier_launches_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Four elements (not by the read-only path, whose loads the compiler may
+// move up across the wait above).
 template <class T>
 __device__ __forceinline__ void load4(float (&d)[4], const T* p, bool in) {
-  if (in) {
-    Sto<T>::ldg4(d, p);
-  } else {
+  if (!in) {
     zero4(d);
+  } else if constexpr (sizeof(T) == 4) {
+    get4(d, *reinterpret_cast<const float4*>(p));
+  } else {
+    Sto<T>::cvt(d, *reinterpret_cast<const uint2*>(p));
   }
 }
 
@@ -78,6 +94,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
   const T* hy = field_ptr_t<T>(S, kHy, 0) + p.i;
   const T* jz = field_ptr_t<T>(S, kJz, 0) + p.i;
   const T* kp = reinterpret_cast<const T*>(S.kp);
+  earlier_launches_done();
   if (!PLAIN) tile_psi_load<R, true>(S, S.psi, p, psi, rows, row0);
   float kv[kCopy ? 1 : R][4], jv[JS && !kCopy ? R : 1][4];
 #pragma unroll
@@ -217,6 +234,26 @@ step_tma_batch_kernel(const DevShot* __restrict__ shots, const int4* __restrict_
   }
 }
 
+// A launch that may start while the one before it in the stream ends; its tiles
+// wait for the earlier launches before they read anything those write
+// (earlier_launches_done).  Saves ~3 us of the ~5 us between two passes: 700^2
+// 4.10 -> 3.46 us per step, 2048^2 11.25 -> 10.3.  (Loading the tables and the
+// points' values before that wait gained nothing more and cost the plain tiles,
+// compiled into the same kernel, 8 % at 8192^2.)
+cudaError_t launch_early(const void* fn, int n_tiles, void** args, size_t smem, cudaStream_t stream) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(n_tiles);
+  cfg.blockDim = dim3(kWarps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 bool lossless(const DevShot& s) { return s.ca == 1.f && s.da == 1.f; }
 
 template <int RP, bool AUX, class T>
@@ -295,7 +332,7 @@ cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, 
   DevShot s = shot;
   TileAux a = aux ? *aux : TileAux{};
   void* args[] = {&s, &a, (void*)&tiles, &n_global, &steps};
-  return cudaLaunchKernel(fn, dim3(n_tiles), dim3(kWarps * 32), args, smem, stream);
+  return launch_early(fn, n_tiles, args, smem, stream);
 }
 
 cudaError_t launch_batch_tile(int shape, bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
@@ -309,7 +346,7 @@ cudaError_t launch_batch_tile(int shape, bool lossless, const DevShot* shots, co
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {&shots, &tiles, &g, &steps, &pass};
-  return cudaLaunchKernel(fn, dim3(n_tiles), dim3(kWarps * 32), args, smem, stream);
+  return launch_early(fn, n_tiles, args, smem, stream);
 }
 
 }  // namespace fdtd2d
