@@ -940,6 +940,20 @@ bool setup_aux(fdtd2d_ctx* c, const std::vector<int32_t>& scan_i, const std::vec
   return true;
 }
 
+// The material-ID medium on chip: run calls of at least kResidentSteps steps of
+// the shots that fit, with the same switches; shorter calls keep the one-step
+// kernels, as do shots whose tracker or probe the kernel cannot record.  At 500 x
+// 1200 with 21 tracker lines 3.54 us per step, the persistent kernel 15.4.
+int setup_resident_material(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
+  for (const char* v : {"FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_KERNEL"})
+    if (std::getenv(v)) return FDTD2D_OK;
+  const int rc = setup_resident(c, device);
+  if (rc || !c->resident) return rc;
+  const std::vector<int32_t> scan(s->rc_scan_i, s->rc_scan_i + c->n_rc), most(s->rc_max_i, s->rc_max_i + c->n_rc);
+  if (!setup_aux(c, scan, most)) c->resident = false;
+  return FDTD2D_OK;
+}
+
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
 // shot whose CPML fits a tile's shared memory.  Measured on GB300 against the two-step path and
 // the persistent kernel, Gcell/s: 1024^2 180 (85), 2048^2 327 (165), 4096^2
@@ -1799,6 +1813,10 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
     CK(cudaMemcpyAsync(c->d_units, units.data(), units.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
   if (c->tma && !member && !c->tile) CK_RC(setup_tmat(c, device));
   if (!member && !solo && !c->tile) CK_RC(setup_persist(c, device));
+  if (!member && c->medium != FDTD2D_MEDIUM_UNIFORM) {
+    CK_RC(setup_resident_material(c, s, device));
+    if (c->resident) std::snprintf(c->kernel_name, sizeof c->kernel_name, "step_persist_kernel<1>/tile<%d>", c->rplan.R);
+  }
   CK(dalloc(c, &c->d_flag, 1));
   CK(cudaStreamSynchronize(c->stream));
 #undef CK
@@ -1828,7 +1846,8 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
     if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ev_m, 0);
     if (e != cudaSuccess) return fail_cuda(c, e);
   }
-  if (c->persist) {
+  const bool on_chip = c->resident && n_last - n_first + 1 >= kResidentSteps;
+  if (c->persist && !on_chip) {
     // all the steps in persistent launches, the tracker and the line probe
     // on their service warps
     PersistAux A{};
@@ -1863,7 +1882,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
     }
     return FDTD2D_OK;
   }
-  if (c->tile) {
+  if (c->tile || on_chip) {
     // launches up to `stop`: until the tracker's history is full, or the line
     // probe's window opens or closes where the kernels do not record it
     for (int32_t n = n_first; n <= n_last;) {
@@ -1876,7 +1895,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
       aux.n0 = n0;
       while (n < stop) {
         int k = stop - n;
-        const bool resident = c->resident && k >= kResidentSteps;
+        const bool resident = c->resident && (k >= kResidentSteps || !c->tile);
         k = std::min(k, resident ? kPersistSteps : kTileSteps);
         cudaEvent_t p0 = prof_mark(c, nullptr, 0, k);
         const DevShot t = tile_view(c, n);

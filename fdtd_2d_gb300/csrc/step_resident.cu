@@ -332,7 +332,7 @@ struct ResPoints {
   }
 };
 
-template <int R, bool LOSSLESS, bool AUX>
+template <int R, bool LOSSLESS, bool AUX, bool MED>
 __device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A, const ResidentPlan& G, int n, int steps, uint64_t* link,
                                              const Waiter& wait, uint32_t tag_add, float4* smem, int* slots) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x;
@@ -358,9 +358,22 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A,
   E.col_in = E.col_out + 2 * rows;
   float4* rest = E.row_in + edge_f4(G.nw * R);
   const int wt = G.nw * 32;                     // threads that step
-  float4* kps = rest + tid;                     // [R][wt]
-  float4* jzs = kps + R * wt;                   // [R][wt] where JS
-  rest += (JS ? 2 : 1) * R * wt;
+  constexpr int kWords = MED ? R + 1 : R;
+  float4* kps = rest + tid;                     // [kWords][wt]
+  float4* jzs = kps + kWords * wt;              // [R][wt] where JS
+  rest += (kWords + (JS ? R : 0)) * wt;
+  MatTables mat;
+  if (MED) {
+    float4* e = rest;
+    float2* h = reinterpret_cast<float2*>(e + 256);
+    for (int t = tid; t < 256; t += threads) {
+      e[t] = __ldg(reinterpret_cast<const float4*>(S.mat_e) + t);
+      h[t] = __ldg(reinterpret_cast<const float2*>(S.mat_h) + t);
+    }
+    mat.e = e;
+    mat.h = h;
+    rest += 256 + 128;
+  }
   float4* point_mem = rest;
   rest += G.point_warps * point_f4(R);
   float* tc = reinterpret_cast<float*>(rest);
@@ -407,12 +420,16 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A,
       for (int q = 0; q < 4; ++q) {
         const int c = p.i + q, j = j0 + r;
         const bool in = work && j < ny && c >= 0 && c < nx;
-        kv[q] = S.kp && in ? __ldg(S.kp + (int64_t)j * pitch + c) : 0.f;
+        kv[q] = !MED && S.kp && in ? __ldg(S.kp + (int64_t)j * pitch + c) : 0.f;
         if (JS) jv[q] = in ? __ldcg(f[kJz] + (int64_t)j * pitch + q) : 0.f;
       }
-      kps[r * wt] = put4(kv);
+      if (!MED) kps[r * wt] = put4(kv);
       if (JS) jzs[r * wt] = put4(jv);
     }
+  }
+  if (MED && work) {
+    for (int r = -1; r < R; ++r)
+      *reinterpret_cast<uint4*>(kps + (r < 0 ? R : r) * wt) = mat_make(S, p.i, j0 + r);
   }
   if (work) tile_psi_load<R, false>(S, S.psi, p, psi, rows, row0);
   copies_done();
@@ -453,7 +470,7 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A,
         s.ez[r + 1][0] = take_l ? z : s.ez[r + 1][0];
         s.ez[r + 1][3] = take_r ? z : s.ez[r + 1][3];
       }
-      tile_step<R, JS, LOSSLESS, decltype(x)::value, decltype(y)::value, float>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, wt, lane);
+      tile_step<R, JS, LOSSLESS, decltype(x)::value, decltype(y)::value, float, MED>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, wt, lane, mat);
       if (pts.state) pts.sources<R, JS>(s, lane);
     }
   };
@@ -495,7 +512,7 @@ __device__ __forceinline__ void resident_run(const DevShot& S, const TileAux& A,
   tile_psi_store<R, false>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, r0, min(r0 + rows, ny - 1));
 }
 
-template <int R, bool LOSSLESS, bool AUX>
+template <int R, bool LOSSLESS, bool AUX, bool MED>
 __global__ void __launch_bounds__(all_warps(R) * 32, 1)
 step_persist_tile_kernel(const __grid_constant__ DevShot S, const __grid_constant__ TileAux A,
                          const __grid_constant__ ResidentPlan G, int n_global, int steps,
@@ -505,16 +522,17 @@ step_persist_tile_kernel(const __grid_constant__ DevShot S, const __grid_constan
   if (threadIdx.x == 0) dead = slots = 0;
   __syncthreads();
   const Waiter wait{&dead, err, wait_ns};
-  resident_run<R, LOSSLESS, AUX>(S, A, G, n_global - S.base_n, steps, link, wait, (uint32_t)tag_add, smem, &slots);
+  resident_run<R, LOSSLESS, AUX, MED>(S, A, G, n_global - S.base_n, steps, link, wait, (uint32_t)tag_add, smem, &slots);
 }
 
 template <int R, bool AUX>
 const void* resident_kernel(const DevShot& s) {
-  return s.ca == 1.f && s.da == 1.f ? (const void*)step_persist_tile_kernel<R, true, AUX>
-                                    : (const void*)step_persist_tile_kernel<R, false, AUX>;
+  return s.ca == 1.f && s.da == 1.f ? (const void*)step_persist_tile_kernel<R, true, AUX, false>
+                                    : (const void*)step_persist_tile_kernel<R, false, AUX, false>;
 }
 template <int R>
 const void* resident_kernel(const DevShot& s, bool aux) {
+  if (s.mat_e) return (const void*)step_persist_tile_kernel<R, false, true, true>;   // (one form: such shots have a tracker)
   return aux ? resident_kernel<R, true>(s) : resident_kernel<R, false>(s);
 }
 const void* resident_kernel(int R, const DevShot& s, bool aux) {
@@ -647,6 +665,7 @@ bool resident_plan(const DevShot& s, const std::vector<int3>& points, int R, int
   }
   f4 += g.point_warps * point_f4(R);
   f4 += 4 * g.nw * 32 + edge_f4(g.nw * R) + (jz_shared(R) ? 2 : 1) * R * g.nw * 32;
+  if (s.mat_e) f4 += g.nw * 32 + 256 + 128;   // the words of the rows below, the tables
   g.smem = f4 * 16;
   if (g.smem + 64 > most) return false;
   g.link_words = 2 * ((int64_t)(edge_bands * g.ns[0] + inner * g.ns[1]) * 2 * kTileCols + 2 * (int64_t)g.nb * g.groups * R);

@@ -289,6 +289,47 @@ __device__ __forceinline__ void tile_psi_store(const DevShot& S, float* slab, co
   }
 }
 
+// The material-ID medium: tables by material in shared memory, and per thread
+// and row one word for 4 cells in place of the drive: their ids in the Hx, Hy and
+// Ez maps, and which of the reference's eight update launches reach them (bit
+// 4 q + k: kernel q, column k).  Row R of the thread's words is the row below.
+// (The one-step kernel reads 3 ids and compares 8 indexes per cell and step; here
+// both are done once per launch, and a step costs one 16-byte read per 4 cells.)
+struct MatTables {
+  const float2* h = nullptr;   // da, db
+  const float4* e = nullptr;   // ca, cb, drive, PEC
+};
+__device__ __forceinline__ uint4 mat_word(const float4* words, int r, int stride) {
+  return *reinterpret_cast<const uint4*>(words + r * stride);
+}
+__device__ __forceinline__ bool mat_covered(const uint4& w, int kernel, int k) { return w.w >> (4 * kernel + k) & 1; }
+
+// The word of columns i .. i+3 of row j (zeros outside the grid).
+__device__ __forceinline__ uint4 mat_make(const DevShot& S, int i, int j) {
+  uint4 w = make_uint4(0, 0, 0, 0);
+  const int nx = S.nx, ny = S.ny, P = S.npml;
+  if (j < 0 || j >= ny) return w;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int c = i + k;
+    if (c < 0 || c >= nx) continue;
+    const int64_t o = (int64_t)j * S.pitch + c;
+    w.x |= (unsigned)__ldg(S.id1 + o) << 8 * k;
+    w.y |= (unsigned)__ldg(S.id2 + o) << 8 * k;
+    w.z |= (unsigned)__ldg(S.id3 + o) << 8 * k;
+    // the reference's thread index of the cell in each launch
+    const int ry = j >= P ? ny - 2 - j : j, rx = c >= P ? nx - 2 - c : c;
+    const long long l[8] = {(long long)j * (nx - 1) + c, (long long)ry * (nx - 1) + c, (long long)j * (nx - 1) + c,
+                            (long long)j * (P - 1) + rx, (long long)(j - 1) * (nx - 2) + (c - 1),
+                            (long long)(j - 1) * (nx - 2) + (c - 1),
+                            (long long)(j - 1) * (P - 1) + ((c >= P ? nx - 1 - c : c) - 1),
+                            (long long)((j >= P ? ny - 1 - j : j) - 1) * (nx - 2) + (c - 1)};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) w.w |= (l[q] < S.cov[q] ? 1u : 0u) << (4 * q + k);
+  }
+  return w;
+}
+
 // One time step of the thread's cells up to Ez, without sources, detectors
 // and the rounding to the storage type; s.ez[0] and s.ez[R+1] hold the rows
 // around the thread's.  X, Y: the tile's and the warp's forms (TilePos).  The
@@ -299,10 +340,12 @@ __device__ __forceinline__ void tile_psi_store(const DevShot& S, float* slab, co
 // ~1800 cycles a row, and the tiles in the corners of the grid set the step
 // time of all.
 // kp: the thread's drive, js its Jz where JS, `stride` float4 from row to row.
-template <int R, bool JS, bool LOSSLESS, bool X, bool Y, class T>
+// MED: the material-ID medium (FP32): kp holds the cells' words.
+template <int R, bool JS, bool LOSSLESS, bool X, bool Y, class T, bool MED = false>
 __device__ __forceinline__ void tile_step(TileRegs<R, JS>& s, const DevShot& S, const Coef<T>& C, const TilePos& p,
                                           const TilePsi& psi, const float* tc, const float* tr, int rows, int row0,
-                                          const float4* kp, float4* js, int stride, int lane) {
+                                          const float4* kp, float4* js, int stride, int lane, const MatTables& M = MatTables()) {
+  static_assert(!MED || (!LOSSLESS && sizeof(T) == 4), "the material medium: FP32, coefficients by cell");
   const int ny = S.ny, P = S.npml;
   const int ts = rows + 1;             // row tables start at row r0 - 1
   const float* trw = tr + row0;        // this warp's: entry r is row j0 - 1 + r
@@ -321,6 +364,23 @@ __device__ __forceinline__ void tile_step(TileRegs<R, JS>& s, const DevShot& S, 
       c = trw[kTcCh * ts + r];
       strip = y_strip_h(p.j0 - 1 + r, ny, P);
     }
+    if constexpr (MED) {
+      const uint4 w = mat_word(kp, r == 0 ? R : r - 1, stride);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 m = M.h[w.x >> 8 * k & 255];
+        const bool in = !X || p.mh(k);
+        float v = tile_h<false>(m.x, s.hx[r][k], m.y, s.ez[r][k], s.ez[r + 1][k], den);
+        v = in && mat_covered(w, kCovHx, k) ? v : s.hx[r][k];
+        if (Y) {
+          const bool add = strip && in && mat_covered(w, kCovHxPml, k);
+          const float q = upd_psi(b, pn[k], c, s.ez[r][k], s.ez[r + 1][k]);
+          v = add ? __fmaf_rn(m.y, q, v) : v;
+          pn[k] = add ? q : pn[k];
+        }
+        s.hx[r][k] = v;
+      }
+    } else
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const bool in = !X || p.mh(k);
@@ -354,6 +414,22 @@ __device__ __forceinline__ void tile_step(TileRegs<R, JS>& s, const DevShot& S, 
     const float er[4] = {s.ez[r + 1][1], s.ez[r + 1][2], s.ez[r + 1][3], e4};
     float (&pn)[4] = pq[r % kBatch];
     if (X) get4(pn, psi.x[(row0 + r) * p.nxl + p.xslot]);
+    if constexpr (MED) {
+      const uint4 w = mat_word(kp, r, stride);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 m = M.h[w.y >> 8 * k & 255];
+        float v = tile_h<false>(m.x, s.hy[r][k], m.y, er[k], s.ez[r + 1][k], dhx[k]);
+        v = (!X || p.mh(k)) && mat_covered(w, kCovHy, k) ? v : s.hy[r][k];
+        if (X) {
+          const bool add = p.xh(k) && mat_covered(w, kCovHyPml, k);
+          const float q = upd_psi(b[k], pn[k], c[k], er[k], s.ez[r + 1][k]);
+          v = add ? __fmaf_rn(m.y, q, v) : v;
+          pn[k] = add ? q : pn[k];
+        }
+        s.hy[r][k] = v;
+      }
+    } else
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       float v = tile_h<LOSSLESS>(C.da, s.hy[r][k], C.db, er[k], s.ez[r + 1][k], dhx[k]);
@@ -403,6 +479,33 @@ __device__ __forceinline__ void tile_step(TileRegs<R, JS>& s, const DevShot& S, 
       yc = trw[kTcCe * ts + r + 1];
       ystrip = y_strip_e(j, ny, P);
     }
+    if constexpr (MED) {
+      const uint4 w = mat_word(kp, r, stride);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 m = M.e[w.z >> 8 * k & 255];   // ca, cb, drive, PEC
+        const bool in = row_in && (!X || p.me(k));
+        const float jo = JS ? jv[k] : jz[k];
+        const float jn = in && mat_covered(w, kCovJz, k) ? upd_j(C.ja, jo, m.z, s.ez[r + 1][k]) : jo;
+        float v = upd_e(m.x, s.ez[r + 1][k], m.y, __fsub_rn(s.hy[r][k], hyl[k]), dex[k], __fsub_rn(s.hx[r][k], s.hx[r + 1][k]), dey, jn);
+        v = m.w != 0.f ? 0.f : v;
+        v = in && mat_covered(w, kCovEz, k) ? v : s.ez[r + 1][k];
+        if (X) {
+          const bool add = row_in && p.xe(k) && mat_covered(w, kCovEzPmlI, k);
+          const float q = upd_psi(b[k], px[k], c[k], s.hy[r][k], hyl[k]);
+          v = add ? __fmaf_rn(m.y, q, v) : v;
+          px[k] = add ? q : px[k];
+        }
+        if (Y) {
+          const bool add = ystrip && in && mat_covered(w, kCovEzPmlJ, k);
+          const float q = upd_psi(yb, py[k], yc, s.hx[r][k], s.hx[r + 1][k]);
+          v = add ? __fmaf_rn(m.y, q, v) : v;
+          py[k] = add ? q : py[k];
+        }
+        if (JS) jv[k] = jn; else jz[k] = jn;
+        s.ez[r + 1][k] = v;
+      }
+    } else
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const bool in = row_in && (!X || p.me(k));

@@ -209,3 +209,65 @@ def test_tracker_and_probe_recorded(gpu, monkeypatch, tmp_path):
     for k in ref:
         assert np.array_equal(ref[k], on_chip[k]), ("on chip", k)
         assert np.array_equal(ref[k], passes[k]), ("passes", k)
+
+
+@pytest.mark.parametrize("rows,imax,jmax", [("2", 60, 45), ("4", 190, 101), ("6", 127, 160), ("8", 250, 333), ("", 250, 600)])
+def test_resident_material(gpu, monkeypatch, tmp_path, rows, imax, jmax):
+    """The material-ID medium on chip: random ids (with the perfect conductor's)
+    in the three maps, coefficients by material, update launches that stop short
+    of their last cells; run calls of 1 to 40 steps, the short ones on the
+    one-step kernels.  The streaming kernel's bits."""
+    import ctypes
+    import re
+    from pathlib import Path
+
+    ini = (Path(__file__).resolve().parent / "golden" / "sphere_fluc_chirp" / "Settings.ini").read_text()
+    for key, val in (("Imax", imax), ("Jmax", jmax), ("Use_Exp_time", "0"), ("Max_time", "90")):
+        ini = re.sub(rf"(?m)^{key}\s*=.*$", f"{key} = {val}", ini)
+    path = tmp_path / "Settings.ini"
+    path.write_text(ini)
+    prob = F.Problem.from_ini(path)
+    s = prob.setup
+    nx, ny, P, n = s.nx, s.ny, s.npml, s.n_materials
+    assert s.medium == F.MEDIUM_MATERIAL_ID
+    rng = np.random.default_rng(nx)
+    keep = []
+
+    def put(name, a):
+        keep.append(a)
+        setattr(s, name, a.ctypes.data_as(type(getattr(s, name))))
+
+    for name in ("id1", "id2", "id3"):
+        put(name, rng.integers(0, n, (ny, nx)).astype(np.int32))
+    for name in ("mat_ca", "mat_da"):
+        put(name, rng.uniform(0.9, 1.0, n).astype(np.float32))
+    for name in ("mat_cb", "mat_db"):
+        put(name, (np.ctypeslib.as_array(getattr(s, name), (n,)) * rng.uniform(0.5, 1.0, n)).astype(np.float32))
+    full = [(nx - 1) * (ny - 1), (nx - 1) * (P - 1), (nx - 1) * (ny - 1), (P - 1) * (ny - 1)]
+    full += [(nx - 2) * (ny - 2), (nx - 2) * (ny - 2), (P - 1) * (ny - 2), (nx - 2) * (P - 1)]
+    s.cover = (ctypes.c_int64 * 8)(*(int(c * f) for c, f in zip(full, rng.uniform(0.6, 1.0, 8))))
+    st = random_state(None, nx, ny, P, rng)
+
+    def stepped():
+        with F.Shot(prob, gpu) as shot:
+            load_state([shot], st)
+            first = 1
+            for c in (1, 9, 3, 8, 12, 7, 40):
+                shot.run(first, first + c - 1)
+                first += c
+            out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+            out.update(shot.traces())
+            out["rc"] = shot.rc() if s.n_rc else np.zeros(1)
+            return shot.kernel_name(), out
+
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE", "FDTD2D_RESIDENT"):
+        monkeypatch.delenv(v, raising=False)
+    if rows:
+        monkeypatch.setenv("FDTD2D_RESIDENT", rows)
+    name, got = stepped()
+    assert name.startswith("step_persist_kernel<1>/tile<" + rows), name
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = stepped()
+    assert name == "step_stream_kernel<1>", name
+    for k in ref:
+        assert np.array_equal(ref[k], got[k]), k
