@@ -869,9 +869,10 @@ DevShot tile_view(const fdtd2d_ctx* c, int n) {
 }
 
 // The whole shot on chip (step_resident.cu) for run calls of at least
-// kResidentSteps steps, wherever it fits (FP32, up to ~1.6 M cells): faster than
-// the tile passes at every size that fits (4.16 against 6.19 us per step at 500 x
-// 3000, 2.87 against 5.12 at 1024^2).  Not for a batch's solo members, whose
+// kResidentSteps steps, wherever it fits (up to ~1.6 M cells, ~1.2 M with 16-bit
+// fields): faster than the tile passes at every size that fits (us per step, FP32:
+// 3.80 against 6.7 at 500 x 3000, 4.27 against 4.58 at 900 x 1600, 2.90 against 4.5
+// at 1024^2; F16: 3.4 against 4.6 at 1024^2, 2.0 against 3.95 at 512^2).  Not for a batch's solo members, whose
 // launches share the GPU.  FDTD2D_RESIDENT=0 (or FDTD2D_PERSIST=0, or FDTD2D_TILE
 // naming the tiles): never; FDTD2D_RESIDENT=R: with R rows per warp only.
 int setup_resident(fdtd2d_ctx* c, int device) {
@@ -956,8 +957,8 @@ int setup_resident_material(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
 
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
 // shot whose CPML fits a tile's shared memory.  Measured on GB300 against the two-step path and
-// the persistent kernel, Gcell/s: 1024^2 180 (85), 2048^2 327 (165), 4096^2
-// 457 (249), 8192^2 553 (315), F16 4096^2 471 (281), 8192^2 585 (413).
+// the persistent kernel, Gcell/s: 1024^2 240 (85), 2048^2 406 (165), 4096^2
+// 511 (249), 8192^2 571 (315), F16 8192^2 610 (413).
 // The compiled shapes are timed at create (a trial reads one buffer set and
 // writes the other, as a step does) and the choice kept per class.
 // FDTD2D_TILE=0: never; FDTD2D_TILE=R: the shape with R rows per warp.  Not
@@ -985,7 +986,7 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
   bool have = forced < 0 && !c->resident && find_choice(key, &ch) && ch.k >= 0 && ch.k < tile_shape_count();
   if (have) note_choice(c, have, ch);
   if (c->resident) {
-    ch.k = 0;
+    ch.k = c->h.store == FDTD2D_STORE_F32 ? 0 : 1;
     have = true;
   }
   if (!have && forced < 0 && c->untimed) {

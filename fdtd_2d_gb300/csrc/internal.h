@@ -315,6 +315,7 @@ struct ResidentPlan {
   int64_t link_words;
 };
 const std::vector<int>& resident_rows();
+const void* resident_kernel16(int R, int store);   // (step_resident16.cu)
 // points: (column, row, PointKind) of the shot's sources and detectors.
 bool resident_plan(const DevShot& s, const std::vector<int3>& points, int R, int device, ResidentPlan* out);
 cudaError_t launch_resident(const DevShot& shot, const ResidentPlan& plan, int n_global, int steps, const TileAux* aux,

@@ -271,3 +271,50 @@ def test_resident_material(gpu, monkeypatch, tmp_path, rows, imax, jmax):
     assert name == "step_stream_kernel<1>", name
     for k in ref:
         assert np.array_equal(ref[k], got[k]), k
+
+
+@pytest.mark.parametrize("rows,nx,ny,P,store,profile,ca,comp", [
+    ("2", 10, 9, 2, 1, 1, 1.0, True), ("2", 253, 97, 12, 2, 1, 0.999, False), ("2", 126, 40, 3, 1, 0, 1.0, False),
+    ("4", 203, 157, 7, 1, 1, 1.0, True), ("4", 500, 400, 40, 2, 3, 0.998, False), ("6", 777, 601, 17, 1, 3, 1.0, False),
+    ("6", 127, 41, 5, 2, 1, 1.0, True), ("6", 1100, 90, 9, 1, 1, 1.0, False), ("", 1000, 900, 20, 2, 3, 1.0, True)])
+def test_resident_16bit_equals_one_row(gpu, monkeypatch, rows, nx, ny, P, store, profile, ca, comp):
+    """The whole shot on chip with 16-bit fields, rounded after every step; Ez
+    detectors alone and with component ones."""
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE", "FDTD2D_RESIDENT"):
+        monkeypatch.delenv(v, raising=False)
+    n = 1 if nx < 40 else 5
+    prob = F.Problem.from_spec(nx=nx, ny=ny, npml=P, n_steps=STEPS, profile=profile, x_lo=nx // 3, x_hi=nx - 3,
+                               x_center=nx / 2, width=nx / 8, grf_rms=0.05, grf_corr=8, ne_peak=2e19, nu=3e9, n_elem=n,
+                               src_i=nx // 2 - 6 if nx > 40 else 4, src_j=ny // 2, src_di=3, src_dj=1, n_det=n,
+                               det_i=nx // 2 - 8 if nx > 40 else 5, det_j=ny // 2 - 2, det_di=2, det_dj=1, storage=store,
+                               field_max=16.0)
+    s = prob.setup
+    s.ca = s.da = ca
+    if comp:
+        s.n_comp, s.comp = s.n_det, s.det
+
+    def stepped(chunks):
+        with F.Shot(prob, gpu) as shot:
+            load_state([shot], st)
+            first = 1
+            for c in chunks:
+                shot.run(first, first + c - 1)
+                first += c
+            out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+            out.update(shot.traces())
+            out["dft"] = shot.dft()
+            return shot.kernel_name(), out
+
+    st = random_state(None, nx, ny, P, np.random.default_rng(nx))
+    if rows:
+        monkeypatch.setenv("FDTD2D_RESIDENT", rows)
+    name, got = stepped(CHUNKS)
+    assert name.startswith("step_persist_kernel<0>/tile<" + rows), name
+    monkeypatch.delenv("FDTD2D_RESIDENT", raising=False)
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv("FDTD2D_TMA", "4,3")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = stepped((STEPS,))
+    assert name == "step_tma_kernel<4,3>", name
+    for k in ref:
+        assert np.array_equal(ref[k], got[k]), k
