@@ -957,8 +957,8 @@ int setup_resident_material(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
 
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
 // shot whose CPML fits a tile's shared memory.  Measured on GB300 against the two-step path and
-// the persistent kernel, Gcell/s: 1024^2 240 (85), 2048^2 406 (165), 4096^2
-// 511 (249), 8192^2 571 (315), F16 8192^2 610 (413).
+// the persistent kernel, Gcell/s: 1024^2 263 (85), 2048^2 445 (165), 4096^2
+// 536 (249), 8192^2 591 (315), F16 4096^2 576 (281), 8192^2 648 (413).
 // The compiled shapes are timed at create (a trial reads one buffer set and
 // writes the other, as a step does) and the choice kept per class.
 // FDTD2D_TILE=0: never; FDTD2D_TILE=R: the shape with R rows per warp.  Not

@@ -275,8 +275,11 @@ cudaError_t launch_rc_steps(const TileAux& A, int ny, int steps, int n_rc, const
                             int j_cut, float level, float* edge, float* cand, int* spd, cudaStream_t stream);
 
 // Several steps per pass on register tiles (step_tile.cu), in shapes that
-// differ in the rows of a plain tile: tiles (flags, c0, r0, u1) of 128 columns
-// from c0 and a band of rows from r0, storing rows up to u1.  A launch reads
+// differ in the rows of a plain tile: tiles (flags, c0, r0, part) of 128 columns
+// from c0 and a band of rows from r0, storing a part of them: plain tiles what
+// their halo leaves up to row `part`, the others the rows and groups of 4 columns
+// in `part` (first row, end row, first group, end group, a byte each, counted from
+// r0 and c0).  A launch reads
 // state n_global-1 from fb[0] and psi, writes state n_global-1+steps (steps <=
 // kTileSteps) to fb[1] and psi + psi_buf.  smem: tile_smem of the shot.
 constexpr int kTileSteps = 4;
@@ -291,7 +294,7 @@ cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, 
                              int steps, const TileAux* aux, cudaStream_t stream);
 // A pass of a batch: every shot in `shots` (FP32) by up to `steps` steps after
 // global step g, shot s by its own steps g + 1 - base_n on, at most to its last
-// one.  tiles: (flags | slot << kTileSlot, c0, r0, u1).  pass: the batch's passes
+// one.  tiles: (flags | slot << kTileSlot, c0, r0, part).  pass: the batch's passes
 // before this one; a shot's state is in fb[q] and psi + q psi_buf, q the parity of
 // its own passes (pass - base_pass).  lossless: CA = DA = 1 in every shot.
 constexpr int kTileSlot = 8;

@@ -18,8 +18,8 @@
 //
 // Bytes: 20 x (halo) + 16 per stored cell and 4 steps, 10.1 B per cell-update
 // with R = 7 (the two-step path 18).  Measured on GB300 against that path,
-// Gcell/s: 8192^2 FP32 571 (315), F16 610 (413); 4096^2 511 (249) and 513
-// (281); 2048^2 406 (165).  Bound by latency at 16 warps per SM: a 4096^2 pass
+// Gcell/s: 8192^2 FP32 591 (315), F16 648 (413); 4096^2 536 (249) and 576
+// (281); 2048^2 445 (165).  Bound by latency at 16 warps per SM: a 4096^2 pass
 // issues in 49 % of the cycles, DRAM moves 4.2 TB/s (0.62 of the copy peak); the
 // loads of a tile take a third of its time, overlapped with the SM's other CTA.
 // Rows per warp at 8192^2 FP32 when this was chosen: 4 (Jz in registers) 504, 5
@@ -65,11 +65,28 @@ __device__ __forceinline__ void load4(float (&d)[4], const T* p, bool in) {
   }
 }
 
+// The part of the grid a tile answers for: rows [r0, r1), and of the thread's
+// columns all (15) or none.  A plain tile's is what its halo leaves; the others
+// read theirs again wherever they need it, for both kinds share the kernel's
+// registers: kept in them, or read for plain tiles too, it took 8192^2 from 114
+// to 123 and 132 us per step.
+struct Part {
+  int r0, r1;
+  unsigned own;
+};
+template <bool PLAIN>
+__device__ __forceinline__ Part tile_part(const int4& tile, const int4* at, int lane, bool in) {
+  if (PLAIN) return {tile.z + kHalo, tile.w, lane >= kHalo / 4 && lane < 32 - kHalo / 4 && in ? 15u : 0u};
+  int w;
+  asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(w) : "l"(&at->w));
+  return {tile.z + (w & 255), tile.z + (w >> 8 & 255), lane >= (w >> 16 & 255) && lane < w >> 24 && in ? 15u : 0u};
+}
+
 template <int R, int NW, bool JS, bool LOSSLESS, bool PLAIN, bool AUX, class T>
-__device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, const int4 tile, int n, int steps, float4* smem) {
+__device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, const int4 tile, const int4* at, int n, int steps, float4* smem) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int rows = NW * R, threads = NW * 32;
-  const int c0 = tile.y, r0 = tile.z, u0 = max(r0 + kHalo, 0), u1 = tile.w;
+  const int c0 = tile.y, r0 = tile.z;
   const int nx = S.nx, ny = S.ny;
   const int64_t pitch = S.pitch;
   const int row0 = warp * R, j0 = r0 + row0;
@@ -133,15 +150,13 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
       if (JS) jzs[r * threads] = put4(jv[JS && !kCopy ? r : 0]);
     }
   }
-  // lanes whose columns are stored
-  const unsigned own = lane >= kHalo / 4 && lane < 32 - kHalo / 4 && p.i < nx ? 15u : 0u;
   int p0 = 0, p1 = 0;
   if (j0 + R > 0 && j0 < ny) {
     p0 = __ldg(S.row_start + max(j0, 0));
     p1 = __ldg(S.row_start + min(j0 + R, ny));
   }
   copies_done();   // (a thread reads only what it copied)
-  const unsigned slots = AUX ? tile_tracked(A, p.i, own) : 0u;
+  const unsigned slots = AUX ? tile_tracked(A, p.i, tile_part<PLAIN>(tile, at, lane, p.i < nx).own) : 0u;
   // the loop in the form the warp needs (its barriers pair across the forms)
   auto loop = [&](auto x, auto y) {
     for (int t = 0; t < steps; ++t) {
@@ -153,8 +168,11 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
       get4(s.ez[0], e[(warp > 0 ? 2 * warp - 1 : 0) * 32 + lane]);
       get4(s.ez[R + 1], e[(warp < NW - 1 ? 2 * warp + 2 : 2 * warp + 1) * 32 + lane]);
       tile_step<R, JS, LOSSLESS, decltype(x)::value, decltype(y)::value, T>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, threads, lane);
-      if (p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, own, u0, u1);
-      if (AUX) tile_record<R, JS>(s, A, slots, p, own, u0, u1, n + t);
+      if (AUX || p1 > p0) {
+        const Part u = tile_part<PLAIN>(tile, at, lane, p.i < nx);
+        if (p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, u.own, u.r0, u.r1);
+        if (AUX) tile_record<R, JS>(s, A, slots, p, u.own, u.r0, u.r1, n + t);
+      }
       tile_round<R, JS, T>(s);
     }
   };
@@ -162,7 +180,8 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
   else if (!p.y) loop(Yes{}, No{});
   else if (!p.x) loop(No{}, Yes{});
   else loop(Yes{}, Yes{});
-  if (own) {
+  const Part u = tile_part<PLAIN>(tile, at, lane, p.i < nx);
+  if (u.own) {
     T* ez_w = field_ptr_t<T>(S, kEz, 1) + p.i;
     T* hx_w = field_ptr_t<T>(S, kHx, 1) + p.i;
     T* hy_w = field_ptr_t<T>(S, kHy, 1) + p.i;
@@ -170,7 +189,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int j = j0 + r;
-      if (j < u0 || j >= u1) continue;
+      if (j < u.r0 || j >= u.r1) continue;
       const int64_t o = (int64_t)j * pitch;
       Sto<T>::stcs4(ez_w + o, s.ez[r + 1]);
       Sto<T>::stcs4(hx_w + o, s.hx[r + 1]);
@@ -184,7 +203,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
       }
     }
   }
-  if (!PLAIN) tile_psi_store<R, true>(S, S.psi + S.psi_buf, p, psi, rows, row0, own, u0, u1);
+  if (!PLAIN) tile_psi_store<R, true>(S, S.psi + S.psi_buf, p, psi, rows, row0, u.own, u.r0, u.r1);
 }
 
 template <int RP>
@@ -199,9 +218,9 @@ step_tmat_kernel(const __grid_constant__ DevShot S, const __grid_constant__ Tile
   const int4 tile = __ldg(tiles + blockIdx.x);
   const int n = n_global - S.base_n;
   if (tile.x & kTilePlain) {
-    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, AUX, T>(S, A, tile, n, steps, smem);
+    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, AUX, T>(S, A, tile, tiles + blockIdx.x, n, steps, smem);
   } else {
-    tile_pass<kREdge, kWarps, false, LOSSLESS, false, AUX, T>(S, A, tile, n, steps, smem);
+    tile_pass<kREdge, kWarps, false, LOSSLESS, false, AUX, T>(S, A, tile, tiles + blockIdx.x, n, steps, smem);
   }
 }
 
@@ -228,9 +247,9 @@ step_tma_batch_kernel(const DevShot* __restrict__ shots, const int4* __restrict_
   if (k <= 0) return;
   const TileAux none{};
   if (tile.x & kTilePlain) {
-    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, false, float>(S, none, tile, n, k, smem);
+    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, false, float>(S, none, tile, tiles + blockIdx.x, n, k, smem);
   } else {
-    tile_pass<kREdge, kWarps, false, LOSSLESS, false, false, float>(S, none, tile, n, k, smem);
+    tile_pass<kREdge, kWarps, false, LOSSLESS, false, false, float>(S, none, tile, tiles + blockIdx.x, n, k, smem);
   }
 }
 
@@ -275,39 +294,87 @@ const void* tile_kernel(int shape, const DevShot& s, bool aux) {
 int tile_shape_count() { return kNumShapes; }
 int tile_shape_rows(int shape) { return kShapes[shape]; }
 
-// Tiles over the grid: plain ones where a whole tile and its halo lie inside
-// the CPML, the others (slower: first) over the rest.
-std::vector<int4> make_tiles(const DevShot& s, int shape) {
-  const int nx = s.nx, ny = s.ny, P = s.npml, ue = kRowsEdge - 2 * kHalo, up = kShapes[shape] * kWarps - 2 * kHalo;
-  std::vector<int4> edge, plain;
-  auto add = [&](std::vector<int4>& v, int f, int ca, int cb, int ra, int rb, int use_r) {
-    for (int r = ra; r < rb; r += use_r)
-      for (int c = ca; c < cb; c += kUse) v.push_back(make_int4(f, c - kHalo, r - kHalo, std::min(r + use_r, rb)));
-  };
-  // plain columns [xa, xb): tiles whose 128 columns have no CPML; plain rows
-  // [ya, yb) likewise (a tile reads one row below its first)
-  const int xa = (P + kHalo + kUse - 1) / kUse * kUse;
-  const int nxp = (nx - P - kHalo - xa) / kUse;
-  const int ya = P + 1 + kHalo, yb = ny - P - kHalo;
-  if (!s.den_uniform || nxp < 1 || yb - ya < up) {
-    add(edge, 0, 0, nx, 0, ny - 1, ue);
-    return edge;
+namespace {
+
+// A column of tiles: it answers for grid columns [a, b), a a multiple of 4, with
+// tiles from column c0 on.  plain: no CPML, no border.
+struct TileColumn {
+  int c0, a, b;
+  bool plain;
+};
+
+// Plain columns (whole: 120 grid columns each), as few as it takes, between a first and a last one on
+// the borders, which need no halo there: up to 124 grid columns each.
+std::vector<TileColumn> tile_columns(const DevShot& s) {
+  const int nx = s.nx, clear = s.npml + kHalo, most = kTileCols - kHalo;
+  std::vector<TileColumn> v;
+  const int n = s.den_uniform ? std::max(0, (nx - 2 * most + kUse - 1) / kUse) : 0, both = nx - n * kUse;
+  if (n < 1 || both < 2 * ((clear + 3) & ~3)) {
+    for (int a = 0, b; a < nx; a = b) {
+      const int c0 = std::max(a - kHalo, 0);
+      b = c0 + kTileCols >= nx ? nx : c0 + most;
+      v.push_back({c0, a, b, false});
+    }
+    return v;
   }
-  const int xb = xa + nxp * kUse;
-  const int yc = ya + (yb - ya) / up * up;   // whole plain tiles only: a short one would read into the strip
-  add(edge, 0, 0, nx, 0, ya, ue);
-  add(edge, 0, 0, nx, yc, ny - 1, ue);
-  add(edge, 0, 0, xa, ya, yc, ue);
-  add(edge, 0, xb, nx, ya, yc, ue);
-  add(plain, kTilePlain, xa, xb, ya, yc, up);
+  int a = std::min(most, (both - clear) & ~3);
+  v.push_back({0, 0, a, false});
+  for (int q = 0; q < n; ++q, a += kUse) v.push_back({a - kHalo, a, a + kUse, true});
+  v.push_back({a - kHalo, a, nx, false});
+  return v;
+}
+
+}  // namespace
+
+// Tiles over the grid: plain ones, whole, where no cell of the tile has CPML, the
+// others (slower: first) over the rest.  Every cell below the last row belongs to
+// one tile.  Tiles on a border have no halo there, so a CPML of 20 cells takes one
+// column of them on each side and 2 to 4 rows, where tiles that began 4 cells
+// outside took 2 or 3 columns and 4 or 5 rows.  us per step, before and now: 2048^2
+// 10.35 and 9.43 (with 5 rows per warp 10.68 and 9.43), 4096^2 32.1 and 31.3, F16
+// 31.9 and 29.1, 2300 x 1531 BF16 8.43 and 8.07, 8192^2 F16 110 and 104.
+std::vector<int4> make_tiles(const DevShot& s, int shape) {
+  const int ny = s.ny, P = s.npml, up = kShapes[shape] * kWarps - 2 * kHalo;
+  std::vector<int4> edge, plain;
+  // plain rows between `top` and `bottom` rows of others: as many as fit, the rest
+  // split so that it takes the fewest tiles (a tile reads one row below its first)
+  const int top0 = P + 1 + kHalo, bottom0 = P + kHalo - 1, n = (ny - 1 - top0 - bottom0) / up;
+  int top = 0, least = 1 << 30;
+  if (n >= 1) {
+    const int rest = ny - 1 - n * up, ue = kRowsEdge - 2 * kHalo, on = kRowsEdge - kHalo;
+    auto count = [&](int r, int first) { return r <= first ? 1 : 1 + (r - first + ue - 1) / ue; };
+    for (int r = top0; r <= rest - bottom0; ++r)
+      if (const int k = count(r, on) + count(rest - r, on - 1); k < least) {
+        least = k;
+        top = r;
+      }
+  }
+  for (const TileColumn& c : tile_columns(s)) {
+    const int lanes = (c.a - c.c0) / 4 << 16 | (c.b - c.c0 + 3) / 4 << 24;
+    auto others = [&](int a, int stop) {
+      while (a < stop) {
+        const int r0 = std::max(a - kHalo, 0), b = std::min(stop, r0 + kRowsEdge >= ny ? ny - 1 : r0 + kRowsEdge - kHalo);
+        edge.push_back(make_int4(0, c.c0, r0, (a - r0) | (b - r0) << 8 | lanes));
+        a = b;
+      }
+    };
+    if (!c.plain || n < 1) {
+      others(0, ny - 1);
+      continue;
+    }
+    others(0, top);
+    others(top + n * up, ny - 1);
+    for (int q = 0; q < n; ++q) plain.push_back(make_int4(kTilePlain, c.c0, top + q * up - kHalo, top + (q + 1) * up));
+  }
   edge.insert(edge.end(), plain.begin(), plain.end());
   return edge;
 }
 
 size_t tile_smem(const DevShot& s, int shape) {
   int nxl = 0, yw = 0;
-  for (int c = 0; c < s.nx; c += kUse) nxl = std::max(nxl, strip_lanes(s, c - kHalo));
-  for (int r = 0; r < s.ny - 1; ++r) yw = std::max(yw, y_warps(s, r - kHalo, kWarps, kREdge));
+  for (const TileColumn& c : tile_columns(s))
+    if (!c.plain) nxl = std::max(nxl, strip_lanes(s, c.c0));
+  for (int r = 0; r < s.ny - 1; ++r) yw = std::max(yw, y_warps(s, r, kWarps, kREdge));
   const size_t ex = 4 * kWarps * 32;
   const size_t edge = ex + kREdge * kWarps * 32 + tile_table_f4(kRowsEdge) + tile_psi_x(kRowsEdge, nxl) +
                       (size_t)yw * (2 * kREdge + 1) * 32;

@@ -318,3 +318,25 @@ def test_resident_16bit_equals_one_row(gpu, monkeypatch, rows, nx, ny, P, store,
     assert name == "step_tma_kernel<4,3>", name
     for k in ref:
         assert np.array_equal(ref[k], got[k]), k
+
+
+@pytest.mark.parametrize("rows,nx,ny,P,ca", [
+    ("7", 128, 60, 5, 1.0), ("7", 129, 33, 6, 0.999), ("5", 248, 32, 9, 1.0), ("7", 249, 131, 12, 1.0), ("7", 371, 107, 23, 1.0),
+    ("7", 372, 108, 24, 1.0), ("5", 500, 149, 30, 0.998), ("7", 502, 210, 52, 1.0), ("7", 613, 163, 20, 1.0), ("5", 490, 185, 2, 1.0)])
+def test_tile_partition(gpu, monkeypatch, rows, nx, ny, P, ca):
+    """Tiles on the borders and plain tiles moved back: one, two and more columns
+    of tiles, widths around them, one and more rows of CPML tiles, points on both
+    sides of every 8th row and column where tiles may meet."""
+    for v in ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_RESIDENT"):
+        monkeypatch.delenv(v, raising=False)
+    n = min((nx - 4) // 8, (ny - 4) // 4) - 1
+    prob = F.Problem.from_spec(nx=nx, ny=ny, npml=P, n_steps=STEPS, profile=1, x_lo=nx // 3, x_hi=nx - 3, ne_peak=2e19, nu=3e9,
+                               n_elem=n, src_i=3, src_j=2, src_di=8, src_dj=4, n_det=n, det_i=4, det_j=3, det_di=8, det_dj=4)
+    prob.setup.ca = prob.setup.da = ca
+    st = random_state(None, nx, ny, P, np.random.default_rng(nx))
+    monkeypatch.setenv("FDTD2D_TILE", rows)
+    name, got = _stepped(gpu, prob, st, CHUNKS)
+    assert name == f"step_tmat_kernel<tile,{rows}>", name
+    ref = _one_row(gpu, monkeypatch, prob, st, STEPS)
+    for k in ref:
+        assert np.array_equal(ref[k], got[k]), k
