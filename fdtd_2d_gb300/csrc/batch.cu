@@ -102,10 +102,6 @@ int fail(fdtd2d_batch* b, cudaError_t e) {
   return e == cudaErrorMemoryAllocation ? FDTD2D_ERR_NOMEM : FDTD2D_ERR_CUDA;
 }
 
-// Shape of the members' plain tiles: 7 rows per warp (8192^2: 560 Gcell/s, 490
-// with 5).
-constexpr int kBatchShape = 0;
-
 // The tile list of every live shot with steps left, tiles with CPML work (the
 // slower ones) of all shots first, uploaded in the stream's order.
 int upload_tiles(fdtd2d_batch* b) {
@@ -377,7 +373,7 @@ static int fdtd2d_batch_run_body(fdtd2d_batch* b, int32_t n_steps) {
       if (rc) return rc;
     }
     const int K = std::min<int>(n_steps, kTileSteps);
-    const cudaError_t e = launch_batch_tile(kBatchShape, b->lossless, b->d_shots, b->d_tiles, b->n_tiles, b->smem, b->g, K,
+    const cudaError_t e = launch_batch_tile(b->lossless, b->d_shots, b->d_tiles, b->n_tiles, b->smem, b->g, K,
                                             b->passes, b->stream);
     if (e != cudaSuccess) return fail(b, e);
     b->g += K;

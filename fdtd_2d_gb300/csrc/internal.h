@@ -298,7 +298,12 @@ cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, 
 // before this one; a shot's state is in fb[q] and psi + q psi_buf, q the parity of
 // its own passes (pass - base_pass).  lossless: CA = DA = 1 in every shot.
 constexpr int kTileSlot = 8;
-cudaError_t launch_batch_tile(int shape, bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
+// Shape of the members' plain tiles: 5 rows per warp, which spill less than 7 in
+// this kernel and leave a smaller last wave; grids so large that 7 are better
+// (8192^2) are solo members.  12 shots of 512 to 1800 cells a side, 128 steps: 4.58
+// ms (7 rows: 4.70); 8 of 700^2 through the server, 500 steps: 8.43 (8.78).
+constexpr int kBatchShape = 1;
+cudaError_t launch_batch_tile(bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
                               int g, int steps, int pass, cudaStream_t stream);
 
 // The whole shot in the SMs' registers for many steps (step_resident.cu): nb

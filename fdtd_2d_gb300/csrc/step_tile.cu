@@ -402,14 +402,12 @@ cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, 
   return launch_early(fn, n_tiles, args, smem, stream);
 }
 
-cudaError_t launch_batch_tile(int shape, bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
+cudaError_t launch_batch_tile(bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
                               int g, int steps, int pass, cudaStream_t stream) {
   if (steps < 1 || steps > kTileSteps) return cudaErrorInvalidValue;
   if (n_tiles <= 0) return cudaSuccess;
-  const void* fn = shape == 0 ? (lossless ? (const void*)step_tma_batch_kernel<Tile<kShapes[0]>, true>
-                                          : (const void*)step_tma_batch_kernel<Tile<kShapes[0]>, false>)
-                              : (lossless ? (const void*)step_tma_batch_kernel<Tile<kShapes[1]>, true>
-                                          : (const void*)step_tma_batch_kernel<Tile<kShapes[1]>, false>);
+  const void* fn = lossless ? (const void*)step_tma_batch_kernel<Tile<kShapes[kBatchShape]>, true>
+                            : (const void*)step_tma_batch_kernel<Tile<kShapes[kBatchShape]>, false>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {&shots, &tiles, &g, &steps, &pass};
