@@ -309,8 +309,7 @@ def run_batched(args, local: int) -> tuple[dict, float]:
            "note": "end to end from host setups: create/upload, all steps, traces + DFT read back; kernel "
                    "choices of every size class timed once before both passes. plain: one shot at a time "
                    "through the single-shot ABI; batch: grids of >= 2^21 cells as solo members (own "
-                   "streams, two-step tensor path, at most 8 stepping at a time), the rest in one "
-                   "persistent launch per step in CUDA-graph blocks of 16"}
+                   "streams, at most 8 stepping at a time), the rest in one launch per four steps"}
     if args.batch_storage != "f32":
         store = {"f16": F.STORE_F16, "bf16": F.STORE_BF16}[args.batch_storage]
         probs16 = [F.Problem.from_spec(**sp, storage=store) for sp in specs]
@@ -592,7 +591,7 @@ def run_ours(args, world, rank, local, dist) -> None:
 
     # roofline of the interior step kernel: algorithmic bytes of one launch
     # (bpc per cell of its region: each field read and written once per
-    # pass, whether a pass advances them one time step or two; the
+    # pass, however many time steps a pass advances them; the
     # persistent kernel's launch makes one pass per step) over its mean
     # event-timed launch duration
     per_launch_s = kt["ms"] / 1e3 / max(kt["launches"], 1)

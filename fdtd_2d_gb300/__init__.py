@@ -475,7 +475,7 @@ def clear_kernel_choices() -> None:
 
 class Batch:
     """Many uniform-medium shots advanced together on one GPU (fdtd2d_batch_*):
-    one persistent launch per time step in CUDA-graph blocks, each shot at its
+    one launch per four time steps over the tiles of all shots, each shot at its
     own step, admission by a device-memory budget."""
 
     def __init__(self, device: int = 0, budget_bytes: int = 0):

@@ -875,18 +875,17 @@ DevShot tile_view(const fdtd2d_ctx* c, int n) {
 // at 1024^2; F16: 3.4 against 4.6 at 1024^2, 2.0 against 3.95 at 512^2).  Not for a batch's solo members, whose
 // launches share the GPU.  FDTD2D_RESIDENT=0 (or FDTD2D_PERSIST=0, or FDTD2D_TILE
 // naming the tiles): never; FDTD2D_RESIDENT=R: with R rows per warp only.
-int setup_resident(fdtd2d_ctx* c, int device) {
+void setup_resident(fdtd2d_ctx* c, int device) {
   const char* env = std::getenv("FDTD2D_RESIDENT");
-  if (c->solo || std::getenv("FDTD2D_PERSIST") || std::getenv("FDTD2D_TILE")) return FDTD2D_OK;
+  if (c->solo || std::getenv("FDTD2D_PERSIST") || std::getenv("FDTD2D_TILE")) return;
   for (const int R : resident_rows()) {
     if (env && std::atoi(env) != R) continue;
     if (!resident_plan(c->h, c->points, R, device, &c->rplan)) continue;
-    const cudaError_t e = dalloc(c, &c->d_link, (size_t)c->rplan.link_words);
-    if (e != cudaSuccess) return fail_cuda(c, e);
-    c->resident = true;
-    break;
+    // (no memory for the exchanged edges: the other paths)
+    if (dalloc(c, &c->d_link, (size_t)c->rplan.link_words) == cudaSuccess) c->resident = true;
+    else cudaGetLastError();
+    return;
   }
-  return FDTD2D_OK;
 }
 
 // The tracker and the line probe on the tile paths (FP32): the kernels record
@@ -945,14 +944,13 @@ bool setup_aux(fdtd2d_ctx* c, const std::vector<int32_t>& scan_i, const std::vec
 // the shots that fit, with the same switches; shorter calls keep the one-step
 // kernels, as do shots whose tracker or probe the kernel cannot record.  At 500 x
 // 1200 with 21 tracker lines 3.54 us per step, the persistent kernel 15.4.
-int setup_resident_material(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
+void setup_resident_material(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
   for (const char* v : {"FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_KERNEL"})
-    if (std::getenv(v)) return FDTD2D_OK;
-  const int rc = setup_resident(c, device);
-  if (rc || !c->resident) return rc;
+    if (std::getenv(v)) return;
+  setup_resident(c, device);
+  if (!c->resident) return;
   const std::vector<int32_t> scan(s->rc_scan_i, s->rc_scan_i + c->n_rc), most(s->rc_max_i, s->rc_max_i + c->n_rc);
   if (!setup_aux(c, scan, most)) c->resident = false;
-  return FDTD2D_OK;
 }
 
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
@@ -978,8 +976,7 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
     const std::vector<int32_t> scan(s->rc_scan_i, s->rc_scan_i + c->n_rc), most(s->rc_max_i, s->rc_max_i + c->n_rc);
     if (!setup_aux(c, scan, most) && c->n_rc > 0) return FDTD2D_OK;   // (the probe alone: single steps in its window)
   }
-  const int rc = setup_resident(c, device);
-  if (rc) return rc;
+  setup_resident(c, device);
   const ChoiceKey key = choice_key(c, device, "tile");
   KernelChoice ch;
   // (a resident shot's tiles serve its short run calls only: not timed)
@@ -1815,7 +1812,7 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
   if (c->tma && !member && !c->tile) CK_RC(setup_tmat(c, device));
   if (!member && !solo && !c->tile) CK_RC(setup_persist(c, device));
   if (!member && c->medium != FDTD2D_MEDIUM_UNIFORM) {
-    CK_RC(setup_resident_material(c, s, device));
+    setup_resident_material(c, s, device);
     if (c->resident) std::snprintf(c->kernel_name, sizeof c->kernel_name, "step_persist_kernel<1>/tile<%d>", c->rplan.R);
   }
   CK(dalloc(c, &c->d_flag, 1));

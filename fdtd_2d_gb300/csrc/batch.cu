@@ -37,9 +37,8 @@ struct Member {
   // its register tiles (a member of the batch kernel) and the passes issued
   std::vector<int4> tiles;
   int32_t passes = 0;
-  // A solo member is a full single shot on its own streams (the tensor path:
-  // two steps per pass where it wins), stepped by fdtd2d_run from the batch's
-  // run calls; `ev` holds the events recorded after its recent run calls on
+  // A solo member is a full single shot on its own streams, stepped by
+  // fdtd2d_run from the batch's run calls; `ev` holds the events recorded after its recent run calls on
   // its stream, oldest first.
   bool solo = false;
   std::vector<cudaEvent_t> ev;
@@ -47,7 +46,7 @@ struct Member {
 };
 
 // Solo members stepped at a time (the oldest admitted first; the others
-// wait): a few two-step chains keep the GPU busy, and every extra one only
+// wait): a few chains of passes keep the GPU busy, and every extra one only
 // adds streams and shares the device among more shots, which delays each.
 // FDTD2D_BATCH_SOLO_ACTIVE overrides it.
 int solo_active() {
@@ -57,7 +56,7 @@ int solo_active() {
 }
 
 // Grids of at least this many cells (2^21, about 1448^2) join a batch as
-// solo members (their own tensor-path launches fill the GPU); smaller ones
+// solo members (their own launches fill the GPU); smaller ones
 // share the batch kernel.  FDTD2D_BATCH_SOLO_CELLS overrides it (0: none
 // solo).
 int64_t solo_cells() {

@@ -246,13 +246,13 @@ const char *fdtd2d_kernel_name(const fdtd2d_ctx *ctx);
 /* ---- Batched and continuous stepping (no counterpart in the reference, which
    runs one shot per process with global state, FDTD_2D_Full/kernel.cu:1928-2818).
    A batch advances many uniform-medium shots (CPML <= 120 cells, no wave-front
-   tracker or line probe) together: one persistent launch per time step, issued
-   in blocks captured as CUDA graphs, each shot at its own step.  Shots can be
+   tracker or line probe) together: one launch per four time steps over the
+   register tiles of all shots, each shot at its own step.  Shots can be
    admitted between fdtd2d_batch_run calls while others are in flight.  A shot
    of at least 2^21 cells (FDTD2D_BATCH_SOLO_CELLS overrides; 0 for none) is
    a solo member instead: a full single shot on its own streams with its own
-   kernel choice (two steps per pass where that wins), stepped from the same
-   run calls; its budget share counts that path's two extra field buffers.
+   kernel choice, stepped from the same run calls; its budget share counts the
+   two extra field buffers that the two-step path would take.
    The batch's kernel steps FP32 fields, so a shot with F16 or BF16 storage
    is a solo member whatever its size.  At most 8 solo members step at a
    time, the oldest admitted first (FDTD2D_BATCH_SOLO_ACTIVE overrides).  A
