@@ -20,11 +20,13 @@
 // with R = 7 (the two-step path 18).  Measured on GB300 against that path,
 // Gcell/s: 8192^2 FP32 591 (315), F16 648 (413); 4096^2 536 (249) and 576
 // (281); 2048^2 445 (165).  Bound by latency at 16 warps per SM: a 4096^2 pass
-// issues in 49 % of the cycles, DRAM moves 4.2 TB/s (0.62 of the copy peak); the
+// issues in 43 % of the cycles, DRAM moves 4.4 TB/s (0.65 of the copy peak); the
 // loads of a tile take a third of its time, overlapped with the SM's other CTA.
-// Rows per warp at 8192^2 FP32 when this was chosen: 4 (Jz in registers) 504, 5
-// 491, 6 520, 7 553, 8 485; CTAs of CPML tiles with 5 or 6 rows need the shared
-// memory of two (363, 370).
+// us per step with 7 / 6 / 5 rows per warp: FP32 8192^2 114 / 119 / 127, 4096^2
+// 31.4 / 32.6 / 33.2, 2048^2 9.8 / 9.6 / 9.4, 1024^2 4.5 / 4.4 / 4.0, F16 8192^2
+// 104 / 125 / 112; 6 is best at few sizes (1400^2 4.9 against 5.0 with 5) and left
+// out.  CTAs of CPML tiles with 5 or 6 rows need the shared memory of two (8192^2:
+// 363 and 370 Gcell/s).
 #include <algorithm>
 
 #include "internal.h"
