@@ -384,6 +384,30 @@ size_t tile_smem(const DevShot& s, int shape) {
   return std::max(edge, plain) * 16;
 }
 
+namespace {
+
+// The most shared memory a tile takes: tile_smem with every lane of the tile in an
+// x strip and every warp in a y strip (a CPML of 120 cells comes to that).
+constexpr size_t most_smem() {
+  size_t most = 0;
+  for (const int rows : kShapes) {
+    const size_t plain = 4 * kWarps * 32 + 2 * (size_t)rows * kWarps * 32;
+    most = most > plain ? most : plain;
+  }
+  const size_t edge = 4 * kWarps * 32 + kREdge * kWarps * 32 + kTcRows * (kTileCols + kRowsEdge + 4) / 4 +
+                      2 * kRowsEdge * 32 + (size_t)kWarps * (2 * kREdge + 1) * 32;
+  return (most > edge ? most : edge) * 16;
+}
+
+// The attribute belongs to the kernel, in every thread that launches it: always
+// set to the same value, so that no thread takes away what another one's launch is
+// about to ask for.
+cudaError_t allow_smem(const void* fn) {
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most_smem());
+}
+
+}  // namespace
+
 bool tile_fits(const DevShot& s, int shape, int device) {
   int most = 0;
   cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -396,7 +420,7 @@ cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, 
   if (steps < 1 || steps > kTileSteps || n_tiles <= 0) return cudaErrorInvalidValue;
   const void* fn = tile_kernel(shape, shot, aux != nullptr);
   if (!fn) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) return e;
   DevShot s = shot;
   TileAux a = aux ? *aux : TileAux{};
@@ -410,7 +434,7 @@ cudaError_t launch_batch_tile(bool lossless, const DevShot* shots, const int4* t
   if (n_tiles <= 0) return cudaSuccess;
   const void* fn = lossless ? (const void*)step_tma_batch_kernel<Tile<kShapes[kBatchShape]>, true>
                             : (const void*)step_tma_batch_kernel<Tile<kShapes[kBatchShape]>, false>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) return e;
   void* args[] = {&shots, &tiles, &g, &steps, &pass};
   return launch_early(fn, n_tiles, args, smem, stream);
