@@ -953,6 +953,95 @@ void setup_resident_material(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
   if (!setup_aux(c, scan, most)) c->resident = false;
 }
 
+// The second stream, for the CPML-band kernel, and the events between the two.
+cudaError_t make_side(fdtd2d_ctx* c) {
+  cudaError_t e = cudaSuccess;
+  for (cudaEvent_t* ev : {&c->ev_t, &c->ev_e, &c->ev_m, &c->ev_a})
+    if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  if (e == cudaSuccess && !c->side) e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
+  return e;
+}
+
+// One-step passes of a tile shot (a run call of one step, the last step of one
+// of 4 m + 1, a step the probe reads) from these many cells on by the tensor
+// kernel's one-step form, the one-row kernel beside it on the CPML bands: a tile
+// reads its halo of 4 cells and pays its prologue whatever the number of steps.
+// us per step in calls of one step, tiles and this form: F16 2900^2 45.5 and 45.4,
+// 4096^2 79.6 and 67.6, 5800^2 153 and 126, 8192^2 296 and 221; BF16 4096^2 81.9 and
+// 68.0; FP32 4096^2 105 and 109, 5800^2 207 and 212, 3000 x 12000 245 and 234, 8192^2
+// 409 and 385.  (Two steps stay one tile pass: F16 8192^2 167 us per step, where the
+// two-step kernel with its two extra field buffers took 162; everywhere else faster.)
+constexpr int64_t kOneStepCells32 = 35000000, kOneStepCells16 = int64_t(1) << 24;
+
+// Whether a tile shot may take that form.  FDTD2D_ONE_STEP=0 (at create): never;
+// =1: at every size it can step.
+bool one_step_wanted(const fdtd2d_ctx* c) {
+  if (const char* env = std::getenv("FDTD2D_ONE_STEP")) return std::atoi(env) != 0;
+  return (int64_t)c->nx * c->ny >= (c->h.store == FDTD2D_STORE_F32 ? kOneStepCells32 : kOneStepCells16);
+}
+
+// Sets it up at its first use; false where it cannot step the shot.
+bool one_step_ready(fdtd2d_ctx* c) {
+  if (c->one_step) return c->one_step > 0;
+  c->one_step = -1;
+  const DevShot& h = c->h;
+  if (!tensor_encoder()) return false;
+  // the shapes the trials of these forms keep most often
+  const int k = tmat_shape_find(4, 4, 2), q = tma_shape_find(2, 2);
+  if (k < 0 || q < 0) return false;
+  const int nx = c->nx, ny = c->ny, P = c->npml, bt = tmat_band_cols(k), b1 = tma_band_cols(q), R = tmat_rows(k);
+  // the interior: rows outside the strips, whole one-row bands of columns; the first
+  // tensor unit of a row range starts `lead` columns left of it, its warps there idle
+  const int ri0 = P, ri1 = ny - P, ci0 = (P + b1 - 1) / b1 * b1, ci1 = ci0 + (nx - P - ci0) / b1 * b1;
+  const int nb = (ci1 - ci0 + bt - 1) / bt, lead = nb * bt - (ci1 - ci0);
+  if (ci1 - ci0 < bt || ny - 2 * P < 4 * R + 2 || !encode_maps(h, nx, ny, tmat_box_cols(k), R, &c->maps)) return false;
+  c->maps_fb0 = h.fb[0];
+  c->tmat_shape = k;
+  c->tma_shape = q;
+  c->tmat_ctas = tmat_resident_ctas(k, h.store, c->device);
+  c->grid_warps = tma_resident_ctas(q, P, h.store, c->device);
+  std::vector<int4> tu;
+  add_units(tu, ci0 - lead, ci1, bt, ri0, ri1, std::min(std::max(1, c->tmat_ctas / nb), (ri1 - ri0) / (2 * R)));
+  for (int4& u : tu)
+    if (u.y < ci0) u.x = (lead / kCols) << 4;
+  const std::vector<int4> eu = edge_units(nx, ny, P, ci0, ci1, ri0, ri1, b1, c->grid_warps);
+  cudaError_t e = make_side(c);
+  if (e == cudaSuccess) e = dalloc(c, &c->d_tunits, tu.size());
+  if (e == cudaSuccess) e = dalloc(c, &c->d_eunits, eu.size());
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(c->d_tunits, tu.data(), tu.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(c->d_eunits, eu.data(), eu.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // the tile passes then
+    return false;
+  }
+  c->n_tunits = (int)tu.size();
+  c->n_eunits = (int)eu.size();
+  c->one_step = 1;
+  return true;
+}
+
+// Step n in that form: after the shot stream's earlier work, and whole when the
+// shot stream goes on.
+cudaError_t launch_one_step(fdtd2d_ctx* c, int32_t n) {
+  TensorMaps m = c->maps;
+  if (c->maps_fb0 != c->h.fb[0]) {   // the tile passes have let the buffers trade places
+    std::swap(m.hj[0], m.hj[1]);
+    std::swap(m.e[0], m.e[1]);
+  }
+  cudaError_t e = cudaEventRecord(c->ev_m, c->stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ev_m, 0);
+  if (e == cudaSuccess)
+    e = launch_step_tmat(c->tmat_shape, c->h, m, c->d_tunits, c->n_tunits, n, c->tmat_ctas, c->d_err, c->stream);
+  if (e == cudaSuccess)
+    e = launch_step_tma(c->tma_shape, c->h, c->d_eunits, c->n_eunits, n, c->grid_warps, c->d_err, c->side);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev_e, c->side);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_e, 0);
+  ++c->launches;
+  return e;
+}
+
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
 // shot whose CPML fits a tile's shared memory.  Measured on GB300 against the two-step path and
 // the persistent kernel, Gcell/s: 1024^2 263 (85), 2048^2 445 (165), 4096^2
@@ -1056,6 +1145,7 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
   c->tile_shape = ch.k;
   c->tile_smem = tile_smem(c->h, ch.k);
   c->tile = true;
+  c->one_step = one_step_wanted(c) ? 0 : -1;
   if (c->resident)
     std::snprintf(c->kernel_name, sizeof c->kernel_name, "step_persist_kernel<0>/tile<%d>", c->rplan.R);
   else
@@ -1102,14 +1192,7 @@ int setup_tmat(fdtd2d_ctx* c, int device) {
   const bool full = full_env && std::strcmp(full_env, "full") == 0;
   DevShot& h = c->h;
   const int nx = c->nx, ny = c->ny, P = c->npml;
-  if (!c->side) {
-    cudaError_t e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_t, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_e, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_m, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_a, cudaEventDisableTiming);
-    if (e != cudaSuccess) return fail_cuda(c, e);
-  }
+  if (const cudaError_t e = make_side(c); e != cudaSuccess) return fail_cuda(c, e);
   // Two-step form: two more field buffers, copies of the first (cells that
   // no kernel writes keep their values in every buffer), its unit counter,
   // and a scratch psi slab for the trials (a trial pair's second step writes
@@ -1895,11 +1978,13 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
         int k = stop - n;
         const bool resident = c->resident && (k >= kResidentSteps || !c->tile);
         k = std::min(k, resident ? kPersistSteps : kTileSteps);
-        cudaEvent_t p0 = prof_mark(c, nullptr, 0, k);
-        const DevShot t = tile_view(c, n);
         const TileAux* a = c->aux ? &aux : nullptr;
+        const bool one = k == 1 && !resident && !a && one_step_ready(c);
+        cudaEvent_t p0 = one ? nullptr : prof_mark(c, nullptr, 0, k);
+        const DevShot t = tile_view(c, n);
         const cudaError_t e =
-            resident ? launch_ordered(c, [&] {
+            one ? launch_one_step(c, n)
+            : resident ? launch_ordered(c, [&] {
               return launch_resident(t, c->rplan, n, k, a, c->d_link, c->d_err, c->wait_ns, c->bar_extra, c->stream);
             })
                      : launch_step_tile(c->tile_shape, t, c->d_tiles, c->n_tiles, c->tile_smem, n, k, a, c->stream);

@@ -72,6 +72,10 @@ struct fdtd2d_ctx {
   int tile_shape = 0, n_tiles = 0;
   size_t tile_smem = 0;
   int4* d_tiles = nullptr;
+  // a tile shot's one-step passes on the tensor kernel, by the fields above (1: set
+  // up, -1: not taken, 0: not looked at yet); maps_fb0: fb[0] when maps were made
+  int one_step = 0;
+  const float* maps_fb0 = nullptr;
   // the tracker and the line probe recorded by the tile kernels: the history
   // holds rc_chunk steps, worked off after them
   bool aux = false;

@@ -6,10 +6,12 @@ import numpy as np
 import pytest
 
 import fdtd_2d_gb300 as F
+from helpers import FIELDS, PSI_FIELDS, load_state, random_state
 
 pytestmark = pytest.mark.gpu
 
-SWITCHES = ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE", "FDTD2D_RESIDENT")
+SWITCHES = ("FDTD2D_KERNEL", "FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_PERSIST", "FDTD2D_TILE", "FDTD2D_RESIDENT",
+            "FDTD2D_ONE_STEP")
 
 
 @pytest.fixture(autouse=True)
@@ -82,3 +84,47 @@ def test_batches_in_two_threads(gpu):
     for a, b in zip(alone, _in_threads(*[lambda p=p: stepped(p) for p in probs])):
         for x, y in zip(a, b):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("nx,ny,P,store,ca", [
+    (800, 90, 3, 0, 1.0), (1283, 333, 17, 0, 0.999), (900, 300, 120, 0, 1.0), (1024, 401, 32, 1, 1.0), (1411, 200, 5, 2, 0.998)])
+def test_one_step_calls(gpu, monkeypatch, nx, ny, P, store, ca):
+    """Run calls that leave a single step to the form for it, between passes of
+    two to four steps after which the buffers have or have not traded places: the
+    one-row kernel's bits in every field, psi array, trace and DFT sum."""
+    chunks = (1, 4, 1, 1, 2, 1, 5, 3, 1, 9, 1)
+    n = sum(chunks)
+    prob = F.Problem.from_spec(nx=nx, ny=ny, npml=P, n_steps=n, profile=1, x_lo=nx // 3, x_hi=nx - 3, ne_peak=2e19, nu=3e9,
+                               n_elem=6, src_i=nx // 2 - 300, src_j=ny // 2, src_di=97, src_dj=1, n_det=9, det_i=P + 4,
+                               det_j=ny // 2 - 3, det_di=(nx - 2 * P) // 10, det_dj=1, storage=store, field_max=16.0)
+    prob.setup.ca = prob.setup.da = ca
+    st = random_state(None, nx, ny, P, np.random.default_rng(nx))
+
+    def stepped(parts):
+        with F.Shot(prob, gpu) as shot:
+            load_state([shot], st)
+            first = 1
+            for c in parts:
+                shot.run(first, first + c - 1)
+                first += c
+            out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+            out["det"], out["dft"] = shot.traces()["det_ez"], shot.dft()
+            shot.synchronize()
+            return shot.kernel_name(), shot.launches(), out
+
+    monkeypatch.setenv("FDTD2D_TILE", "7")
+    monkeypatch.setenv("FDTD2D_ONE_STEP", "0")
+    name, tiles, _ = stepped(chunks)
+    monkeypatch.setenv("FDTD2D_ONE_STEP", "1")
+    name, launches, got = stepped(chunks)
+    assert name == "step_tmat_kernel<tile,7>", name
+    assert launches == tiles + 8   # a second launch for each single step
+    for v in ("FDTD2D_TILE", "FDTD2D_ONE_STEP"):
+        monkeypatch.delenv(v)
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv("FDTD2D_TMA", "4,3")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, _, ref = stepped((n,))
+    assert name == "step_tma_kernel<4,3>", name
+    for k in ref:
+        assert np.array_equal(ref[k], got[k]), k
