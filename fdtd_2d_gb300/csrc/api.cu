@@ -25,6 +25,7 @@
 
 #include <thread>
 
+#include <sys/mman.h>
 #include <sys/stat.h>
 #include <unistd.h>
 
@@ -56,26 +57,46 @@ cudaError_t read_err(fdtd2d_ctx* c, int* err) {
 // Makes the pages of a result buffer present before the device writes them.
 // The copy engine reaches pageable memory through the host's page tables, and
 // a page that was never touched costs it a fault of ~55 us (64 KB pages):
-// 226 ms for an 8192^2 field into a new buffer, 2.9 ms into a present one.
+// 226 ms for an 8192^2 field into a new buffer, 1.4 ms into a present one.
 // Touching them here costs 0.3 us a page (mostly the kernel's clearing), which
-// several threads share for large buffers.  The whole buffer is overwritten
-// by the copy that follows.
+// several threads share where there are many.  Only pages that are not there are
+// touched (the copy that follows overwrites the whole buffer), and none of memory
+// that is not mapped: asking costs less than touching again, 4096^2 into a kept
+// buffer 0.72 ms with every page touched.
 void touch_pages(void* p, size_t bytes) {
   static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  if (bytes < 128 * 1024) return;   // from the heap then, mostly there (asking: 0.7 of the call's 15 us)
+  const uintptr_t first = (uintptr_t)p, base = first & ~(uintptr_t)(page - 1);
+  const size_t n = (first + bytes - base + page - 1) / page;
+  unsigned char few[64];
+  std::vector<unsigned char> many;
+  unsigned char* there = few;
+  if (n > sizeof few) {
+    try {
+      many.resize(n);
+    } catch (...) {
+      return;   // the pages fault in the copy
+    }
+    there = many.data();
+  }
+  if (mincore((void*)base, n * page, there) != 0) return;
   auto part = [=](size_t a, size_t b) {
-    for (size_t o = a; o < b; o += page) static_cast<volatile char*>(p)[o] = 0;
-    if (b > a) static_cast<volatile char*>(p)[b - 1] = 0;
+    for (size_t k = a; k < b; ++k)
+      if (!(there[k] & 1)) *(volatile char*)std::max(first, base + k * page) = 0;
   };
-  const size_t per = size_t(8) << 20;
-  const int n = (int)std::min<size_t>({bytes / per, 8, std::max(1u, std::thread::hardware_concurrency())});
-  if (n <= 1) return part(0, bytes);
+  const size_t missing = n - (size_t)std::count_if(there, there + n, [](unsigned char v) { return v & 1; });
+  if (missing == 0) return;
+  if (missing < 512) return part(0, n);   // (starting threads takes 70 us)
+  // (the number of cores comes from a file, 7 us)
+  static const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
+  const size_t k = std::min(cores, 8u);
   std::vector<std::thread> threads;
   try {
-    for (int k = 1; k < n; ++k) threads.emplace_back(part, bytes / n * k, k + 1 < n ? bytes / n * (k + 1) : bytes);
+    for (size_t t = 1; t < k; ++t) threads.emplace_back(part, n * t / k, n * (t + 1) / k);
   } catch (...) {
     // no more threads to be had: what is left over faults in the copy
   }
-  part(0, bytes / n);
+  part(0, n / k);
   for (std::thread& t : threads) t.join();
 }
 

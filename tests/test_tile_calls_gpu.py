@@ -128,3 +128,37 @@ def test_one_step_calls(gpu, monkeypatch, nx, ny, P, store, ca):
     assert name == "step_tma_kernel<4,3>", name
     for k in ref:
         assert np.array_equal(ref[k], got[k]), k
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 40), (700, 300), (3100, 3000)])
+def test_read_into_kept_new_and_odd_buffers(gpu, nx, ny):
+    """A field read into new pages, pages that are there, some of each, and a buffer
+    that starts inside a page: the same values, nothing outside the buffer touched."""
+    import mmap
+
+    prob = _point_shot(nx, ny, 8, 8)
+    a = np.random.default_rng(nx).standard_normal((ny, nx)).astype(np.float32)
+    n = a.nbytes
+    with F.Shot(prob, gpu) as shot:
+        shot.write_field("ez", a)
+        assert np.array_equal(shot.read_field("ez"), a)
+        for at in (0, 4, 4096 - 8, 70004):
+            mem = mmap.mmap(-1, n + (1 << 18))
+            buf = np.frombuffer(mem, np.uint8)
+            got = buf[at:at + n].view(np.float32)
+            for fill in (0, 3, 7):   # new pages, then present ones; at last every second MB of a new map
+                if fill == 7:
+                    del got, buf
+                    mem = mmap.mmap(-1, n + (1 << 18))
+                    buf = np.frombuffer(mem, np.uint8)
+                    got = buf[at:at + n].view(np.float32)
+                    for m in range(0, n, 2 << 20):
+                        buf[at + m:at + min(m + (1 << 20), n)] = 7
+                elif fill:
+                    buf[:] = fill
+                rc = F._lib().fdtd2d_read_field(shot._h, F.FIELD_EZ, got.ctypes.data_as(F._fp))
+                assert rc == F.OK
+                assert np.array_equal(got, a.ravel())
+                out = 0 if fill == 7 else fill
+                assert (buf[:at] == out).all() and (buf[at + n:] == out).all()
+            del got, buf
