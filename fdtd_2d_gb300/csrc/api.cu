@@ -1064,7 +1064,7 @@ cudaError_t launch_one_step(fdtd2d_ctx* c, int32_t n) {
 }
 
 // Four steps per pass on register tiles (step_tile.cu): every uniform-medium
-// shot whose CPML fits a tile's shared memory.  Measured on GB300 against the two-step path and
+// shot of the staged kernels' CPML depths.  Measured on GB300 against the two-step path and
 // the persistent kernel, Gcell/s: 1024^2 263 (85), 2048^2 445 (165), 4096^2
 // 536 (249), 8192^2 591 (315), F16 4096^2 576 (281), 8192^2 648 (413).
 // The compiled shapes are timed at create (a trial reads one buffer set and
@@ -1078,10 +1078,8 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
     if (std::getenv(v)) return FDTD2D_OK;
   if (const char* v = std::getenv("FDTD2D_PERSIST"); v && std::atoi(v) == 1) return FDTD2D_OK;
   int forced = -1;
-  for (int k = 0; k < tile_shape_count(); ++k) {
-    if (!tile_fits(c->h, k, device)) return FDTD2D_OK;
+  for (int k = 0; k < tile_shape_count(); ++k)
     if (env && std::atoi(env) == tile_shape_rows(k)) forced = k;
-  }
   {
     const std::vector<int32_t> scan(s->rc_scan_i, s->rc_scan_i + c->n_rc), most(s->rc_max_i, s->rc_max_i + c->n_rc);
     if (!setup_aux(c, scan, most) && c->n_rc > 0) return FDTD2D_OK;   // (the probe alone: single steps in its window)

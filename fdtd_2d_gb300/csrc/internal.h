@@ -288,7 +288,6 @@ int tile_shape_count();
 int tile_shape_rows(int shape);   // rows per warp of its plain tiles
 std::vector<int4> make_tiles(const DevShot& s, int shape);
 size_t tile_smem(const DevShot& s, int shape);
-bool tile_fits(const DevShot& s, int shape, int device);
 // aux: null, or what to record (FP32 storage).
 cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
                              int steps, const TileAux* aux, cudaStream_t stream);

@@ -408,13 +408,6 @@ cudaError_t allow_smem(const void* fn) {
 
 }  // namespace
 
-bool tile_fits(const DevShot& s, int shape, int device) {
-  int most = 0;
-  cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  // (Hx and Hy share one scale: the stored-unit arithmetic takes it so)
-  return (s.store == 0 || s.sc[1] == s.sc[2]) && tile_smem(s, shape) <= (size_t)most;
-}
-
 cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
                              int steps, const TileAux* aux, cudaStream_t stream) {
   if (steps < 1 || steps > kTileSteps || n_tiles <= 0) return cudaErrorInvalidValue;

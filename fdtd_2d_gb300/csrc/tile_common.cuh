@@ -39,7 +39,8 @@ __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 0;" ::: "mem
 enum TabCol : int { kTcBh = 0, kTcCh, kTcBe, kTcCe, kTcDe, kTcDh, kTcRows };
 constexpr int kTileCols = 128;
 
-// Coefficients of a shot in stored units.
+// Coefficients of a shot in stored units (Hx and Hy share one scale, as
+// set_storage_scales gives them).
 template <class T>
 struct Coef {
   float da, db, ca, cb, ja, rj, rk;   // upd_h, upd_es, upd_j and the drive's factor
