@@ -1072,11 +1072,8 @@ cudaError_t launch_one_step(fdtd2d_ctx* c, int32_t n) {
 // FDTD2D_TILE=0: never; FDTD2D_TILE=R: the shape with R rows per warp.  Not
 // taken when another path is forced by name.
 int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
+  if (tiles_off()) return FDTD2D_OK;
   const char* env = std::getenv("FDTD2D_TILE");
-  if (env && std::strcmp(env, "0") == 0) return FDTD2D_OK;
-  for (const char* v : {"FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_KERNEL"})
-    if (std::getenv(v)) return FDTD2D_OK;
-  if (const char* v = std::getenv("FDTD2D_PERSIST"); v && std::atoi(v) == 1) return FDTD2D_OK;
   int forced = -1;
   for (int k = 0; k < tile_shape_count(); ++k)
     if (env && std::atoi(env) == tile_shape_rows(k)) forced = k;
@@ -1486,6 +1483,14 @@ int setup_tmat(fdtd2d_ctx* c, int device) {
 }  // namespace
 
 int fdtd2d::validate_setup(const fdtd2d_setup* s) { return validate(s); }
+
+bool fdtd2d::tiles_off() {
+  if (const char* v = std::getenv("FDTD2D_TILE"); v && std::strcmp(v, "0") == 0) return true;
+  for (const char* v : {"FDTD2D_TMA", "FDTD2D_TMAT", "FDTD2D_TB", "FDTD2D_KERNEL"})
+    if (std::getenv(v)) return true;
+  const char* v = std::getenv("FDTD2D_PERSIST");
+  return v && std::atoi(v) == 1;
+}
 
 void fdtd2d::adopt_ctx(fdtd2d_ctx* c, cudaStream_t batch_stream) {
   cudaSetDevice(c->device);

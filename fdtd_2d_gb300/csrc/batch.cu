@@ -166,6 +166,12 @@ void settle(Member& x, const DevShot& s) {
   h.psi_buf = at == slot ? s.psi_buf : -s.psi_buf;
 }
 
+// Room a solo member must find beside its device bytes: the two more field buffers
+// of the two-step path, where a variable sends it there.
+int64_t solo_extra(const fdtd2d_setup* s) {
+  return tiles_off() ? 2 * (int64_t)buffer_floats(s->nx, s->ny) * 4 * store_bytes(s->storage) : 0;
+}
+
 int add_solo(fdtd2d_batch* b, const fdtd2d_setup* s, int64_t bytes, int32_t* shot) {
   int slot = -1;
   for (int k = 0; k < (int)b->m.size(); ++k)
@@ -306,14 +312,12 @@ static int fdtd2d_batch_add_body(fdtd2d_batch* b, const fdtd2d_setup* s, int32_t
   const int64_t bytes = fdtd2d_device_bytes(s);
   if (bytes < 0) return FDTD2D_ERR_INVALID;
   if (b->used + bytes > b->budget) return FDTD2D_ERR_BUDGET;
-  // A large grid goes solo when it fits with the two extra field buffers of
-  // the two-step path.  The batch kernel steps FP32 fields only, so a shot
+  // A large grid goes solo.  The batch kernel steps FP32 fields only, so a shot
   // with 16-bit storage is a solo member whatever its size (the single-shot
-  // path, 16-bit forms included), admitted once those buffers fit too.
-  const int64_t field_buf = (int64_t)buffer_floats(s->nx, s->ny) * 4 * store_bytes(s->storage);
+  // path, 16-bit forms included).
   const int64_t cells = (int64_t)s->nx * s->ny;
   const int64_t sc = solo_cells();
-  const bool fits2 = b->used + bytes + 2 * field_buf <= b->budget;
+  const bool fits2 = b->used + bytes + solo_extra(s) <= b->budget;
   if (s->storage != FDTD2D_STORE_F32) return fits2 ? add_solo(b, s, bytes, shot) : FDTD2D_ERR_BUDGET;
   if (sc > 0 && cells >= sc && fits2) return add_solo(b, s, bytes, shot);
   int slot = -1;
@@ -602,9 +606,8 @@ static int fdtd2d_server_submit_body(fdtd2d_server* s, const fdtd2d_setup* setup
   if (vrc) return vrc;
   const int64_t bytes = fdtd2d_device_bytes(setup);
   if (bytes < 0) return FDTD2D_ERR_INVALID;
-  // could never be admitted (a 16-bit shot also needs its two extra buffers)
-  const int64_t extra = setup->storage == FDTD2D_STORE_F32
-                            ? 0 : 2 * (int64_t)buffer_floats(setup->nx, setup->ny) * 4 * store_bytes(setup->storage);
+  // could never be admitted (a 16-bit shot is a solo member)
+  const int64_t extra = setup->storage == FDTD2D_STORE_F32 ? 0 : solo_extra(setup);
   if (bytes + extra > s->b->budget) return FDTD2D_ERR_BUDGET;
   s->queue.push_back({setup, tag});
   return FDTD2D_OK;

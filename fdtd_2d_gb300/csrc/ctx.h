@@ -127,6 +127,9 @@ int create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ctx** out,
 // The checks fdtd2d_create makes on a setup before it allocates anything
 // (FDTD2D_OK, FDTD2D_ERR_INVALID or FDTD2D_ERR_RANGE).
 int validate_setup(const fdtd2d_setup* s);
+// Whether a variable sends uniform shots past the register tiles, to the paths
+// that may take two more field buffers (the two-step form).
+bool tiles_off();
 // Hand a member shot to the batch's stream: its own stream is released and
 // fdtd2d_run is refused from then on (the batch steps it).
 void adopt_ctx(fdtd2d_ctx* c, cudaStream_t batch_stream);

@@ -251,8 +251,9 @@ const char *fdtd2d_kernel_name(const fdtd2d_ctx *ctx);
    admitted between fdtd2d_batch_run calls while others are in flight.  A shot
    of at least 2^21 cells (FDTD2D_BATCH_SOLO_CELLS overrides; 0 for none) is
    a solo member instead: a full single shot on its own streams with its own
-   kernel choice, stepped from the same run calls; its budget share counts the
-   two extra field buffers that the two-step path would take.
+   kernel choice, stepped from the same run calls.  Where a variable names a
+   path that may take two more field buffers (the two-step path), its admission
+   asks for their room too, and its budget share counts them when it takes them.
    The batch's kernel steps FP32 fields, so a shot with F16 or BF16 storage
    is a solo member whatever its size.  At most 8 solo members step at a
    time, the oldest admitted first (FDTD2D_BATCH_SOLO_ACTIVE overrides).  A
@@ -285,7 +286,7 @@ int fdtd2d_batch_destroy(fdtd2d_batch *b);
 
 /* ---- Serving loop (no counterpart in the reference): shots are queued as they
    arrive, admitted in arrival order while they fit the budget, stepped together
-   in blocks of block_steps launches, and retired as soon as the GPU has
+   in blocks of block_steps time steps, and retired as soon as the GPU has
    finished them (their DFT and Ez traces copied out, their memory released
    behind the queued kernels). ---- */
 typedef struct fdtd2d_server fdtd2d_server;
