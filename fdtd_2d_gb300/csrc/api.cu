@@ -107,8 +107,10 @@ void touch_pages(void* p, size_t bytes) {
 // memory released, or, where the library has a smaller form to fall back to
 // (the two-step path's extra buffers), that the shot still runs.  Normal runs
 // leave it unset.
+//
+// Memory of the context's, as it comes.
 template <class T>
-cudaError_t dalloc(fdtd2d_ctx* c, T** p, size_t count) {
+cudaError_t dalloc_raw(fdtd2d_ctx* c, T** p, size_t count) {
   *p = nullptr;
   if (count == 0) return cudaSuccess;
   if (c->fail_alloc > 0 && ++c->n_alloc == c->fail_alloc) return cudaErrorMemoryAllocation;
@@ -120,7 +122,13 @@ cudaError_t dalloc(fdtd2d_ctx* c, T** p, size_t count) {
   if (e != cudaSuccess) return e;
   c->allocs.push_back(q);
   *p = static_cast<T*>(q);
-  return cudaMemsetAsync(q, 0, count * sizeof(T), c->stream);
+  return cudaSuccess;
+}
+// The same, zeroed.
+template <class T>
+cudaError_t dalloc(fdtd2d_ctx* c, T** p, size_t count) {
+  const cudaError_t e = dalloc_raw(c, p, count);
+  return e != cudaSuccess || count == 0 ? e : cudaMemsetAsync(*p, 0, count * sizeof(T), c->stream);
 }
 
 int pitch_for(int nx) { return row_pitch(nx); }
@@ -341,6 +349,30 @@ int validate(const fdtd2d_setup* s) {
   return FDTD2D_OK;
 }
 
+// Steps from which a run call is worth loading the shot on chip.
+constexpr int kResidentSteps = 8;
+
+// The history of tracked columns on the tile paths: up to 256 steps, 64 MB or the
+// whole shot (0 steps: it cannot be kept, and the tracker takes the other paths).
+struct RcHistory {
+  int n_cols = 0, rows = 0, steps = 0;   // distinct columns, floats per column
+  int64_t bytes() const { return (int64_t)steps * n_cols * rows * 4; }
+};
+RcHistory rc_history(const fdtd2d_setup* s) {
+  RcHistory h;
+  auto column = [&](int k) { return k < s->n_rc ? s->rc_scan_i[k] : s->rc_max_i[k - s->n_rc]; };
+  for (int a = 0; a < 2 * s->n_rc && h.n_cols <= kMaxTracked; ++a) {
+    bool seen = false;
+    for (int b = 0; b < a && !seen; ++b) seen = column(b) == column(a);
+    h.n_cols += !seen;
+  }
+  h.rows = (s->ny + 31) / 32 * 32;
+  if (s->storage != FDTD2D_STORE_F32 || h.n_cols == 0 || h.n_cols > kMaxTracked) return h;
+  const int64_t most = (int64_t(64) << 20) / ((int64_t)h.n_cols * h.rows * 4);
+  if (most >= kResidentSteps) h.steps = (int)std::min<int64_t>({256, most, s->n_steps});
+  return h;
+}
+
 // Split rows [0, ny-1) x column blocks of `cols` into at most `warps` units.
 std::vector<int4> make_units(int shot, int nx, int ny, int warps, int cols = kCols, int min_rows = 8) {
   const int cb = (nx + cols - 1) / cols;
@@ -392,7 +424,13 @@ int64_t fdtd2d_device_bytes(const fdtd2d_setup* s) {
   b += (s->medium == FDTD2D_MEDIUM_UNIFORM) ? (s->ne ? cells * es : 0) : cells * 3;
   b += 2 * 4 * (2 * (P - 1) * pitch + 2 * P * pitch + 2 * s->ny * P * 2);
   b += 4 * (int64_t)s->n_steps * (s->record_traces ? (s->n_det + 3 * s->n_comp) : 0);
+  // (the last term: tables, lists, and on chip the edges its CTAs exchange)
   b += 4 * (int64_t)(s->n_steps + 1) + 16 * (int64_t)s->n_det + (1 << 20);
+  if (s->n_rc > 0 && s->rc_scan_i && s->rc_max_i) {
+    const RcHistory h = rc_history(s);
+    b += h.bytes() + 4 * (int64_t)s->n_rc * (h.steps + s->n_steps + 3);
+  }
+  if (s->line_n > 0) b += 4 * (int64_t)s->line_n * (s->line_last - s->line_first + 1);
   return b;
 }
 
@@ -757,9 +795,6 @@ bool material_as_uniform(const fdtd2d_setup* s, double beta, float* ca, float* c
 constexpr int64_t kPersistMaxCells = int64_t(1) << 22;
 // Steps per persistent launch (a launch of a few tens of ms at most).
 constexpr int kPersistSteps = 4096;
-// Steps from which a run call is worth loading the shot on chip.
-constexpr int kResidentSteps = 8;
-
 // Persistent launches of every shot of this process on a device run one at a
 // time: each waits for the previous one (on whichever stream it ran) and
 // leaves an event for the next.  Two cooperative grids that each fill the
@@ -913,30 +948,28 @@ void setup_resident(fdtd2d_ctx* c, int device) {
 // the tracked columns of every step (a history of up to 64 MB) and the probe's
 // row.  False when they cannot (16-bit storage, too many columns, a probe on the
 // last row, which no tile stores); an allocation that fails is no error.
-bool setup_aux(fdtd2d_ctx* c, const std::vector<int32_t>& scan_i, const std::vector<int32_t>& max_i) {
+bool setup_aux(fdtd2d_ctx* c, const fdtd2d_setup* s) {
   if (c->n_rc == 0 && c->line_n == 0) return true;
   if (c->h.store != FDTD2D_STORE_F32 || (c->line_n > 0 && c->line_j >= c->ny - 1)) return false;
   TileAux a{};
   if (c->n_rc > 0) {
-    std::vector<int> cols(scan_i.begin(), scan_i.end());
-    cols.insert(cols.end(), max_i.begin(), max_i.end());
+    const RcHistory history = rc_history(s);
+    if (history.steps == 0) return false;
+    std::vector<int> cols(s->rc_scan_i, s->rc_scan_i + c->n_rc);
+    cols.insert(cols.end(), s->rc_max_i, s->rc_max_i + c->n_rc);
     std::sort(cols.begin(), cols.end());
     cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
     a.n_cols = (int)cols.size();
-    a.rows = (c->ny + 31) / 32 * 32;
-    const int64_t per = (int64_t)a.n_cols * a.rows * 4;
-    c->rc_chunk = (int)std::min<int64_t>(256, (int64_t(64) << 20) / per);
-    if (a.n_cols > kMaxTracked || c->rc_chunk < kResidentSteps) return false;
+    a.rows = history.rows;
+    c->rc_chunk = history.steps;
     auto slot = [&](int32_t i) { return (int)(std::lower_bound(cols.begin(), cols.end(), (int)i) - cols.begin()); };
     std::vector<int> all(cols);   // columns, then each line's slots
-    for (const int32_t i : scan_i) all.push_back(slot(i));
-    for (const int32_t i : max_i) all.push_back(slot(i));
+    for (int l = 0; l < c->n_rc; ++l) all.push_back(slot(s->rc_scan_i[l]));
+    for (int l = 0; l < c->n_rc; ++l) all.push_back(slot(s->rc_max_i[l]));
     int* d = nullptr;
-    void* hist = nullptr;
     cudaError_t e = dalloc(c, &d, all.size());
     if (e == cudaSuccess) e = dalloc(c, &c->d_cand, (size_t)c->rc_chunk * c->n_rc);
-    if (e == cudaSuccess) e = cudaMallocAsync(&hist, (size_t)c->rc_chunk * per, c->stream);
-    if (e == cudaSuccess) c->allocs.push_back(hist);
+    if (e == cudaSuccess) e = dalloc_raw(c, &a.hist, (size_t)history.bytes() / 4);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -946,7 +979,6 @@ bool setup_aux(fdtd2d_ctx* c, const std::vector<int32_t>& scan_i, const std::vec
     a.cols = d;
     c->d_scan_slot = d + a.n_cols;
     c->d_max_slot = c->d_scan_slot + c->n_rc;
-    a.hist = static_cast<float*>(hist);
   }
   if (c->line_n > 0) {
     a.line_n = c->line_n;
@@ -970,8 +1002,7 @@ void setup_resident_material(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
     if (std::getenv(v)) return;
   setup_resident(c, device);
   if (!c->resident) return;
-  const std::vector<int32_t> scan(s->rc_scan_i, s->rc_scan_i + c->n_rc), most(s->rc_max_i, s->rc_max_i + c->n_rc);
-  if (!setup_aux(c, scan, most)) c->resident = false;
+  if (!setup_aux(c, s)) c->resident = false;
 }
 
 // The second stream, for the CPML-band kernel, and the events between the two.
@@ -1077,10 +1108,7 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
   int forced = -1;
   for (int k = 0; k < tile_shape_count(); ++k)
     if (env && std::atoi(env) == tile_shape_rows(k)) forced = k;
-  {
-    const std::vector<int32_t> scan(s->rc_scan_i, s->rc_scan_i + c->n_rc), most(s->rc_max_i, s->rc_max_i + c->n_rc);
-    if (!setup_aux(c, scan, most) && c->n_rc > 0) return FDTD2D_OK;   // (the probe alone: single steps in its window)
-  }
+  if (!setup_aux(c, s) && c->n_rc > 0) return FDTD2D_OK;   // (the probe alone: single steps in its window)
   setup_resident(c, device);
   const ChoiceKey key = choice_key(c, device, "tile");
   KernelChoice ch;

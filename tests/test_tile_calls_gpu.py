@@ -162,3 +162,70 @@ def test_read_into_kept_new_and_odd_buffers(gpu, nx, ny):
                 out = 0 if fill == 7 else fill
                 assert (buf[:at] == out).all() and (buf[at + n:] == out).all()
             del got, buf
+
+
+def _tracker_shot(n_steps, lines):
+    """A 500 x 300 shot with so many tracker lines, its scan columns beside its maximum columns."""
+    prob = _point_shot(500, 300, 10, n_steps)
+    s = prob.setup
+    scan = np.arange(100, 100 + 7 * lines, 7, dtype=np.int32)
+    most = scan + np.int32(3)
+    prob.keep = (scan, most)
+    s.n_rc, s.rc_level, s.rc_j_cut, s.rc_edge0 = lines, 0.07, 40, 1e-3
+    if lines:
+        s.rc_scan_i, s.rc_max_i = (a.ctypes.data_as(type(s.rc_scan_i)) for a in (scan, most))
+    return prob
+
+
+@pytest.mark.parametrize("n_steps", [10, 400])
+def test_tracker_memory_is_counted(gpu, n_steps):
+    """device_bytes counts the columns a tracker shot keeps, which are no more than
+    its steps need."""
+    from test_failure_gpu import _pool_used_bytes
+
+    held, said = [], []
+    for lines in (0, 12):
+        prob = _tracker_shot(n_steps, lines)
+        base = _pool_used_bytes(gpu)
+        if base is None:
+            pytest.skip("no CUDA runtime library to ask")
+        with F.Shot(prob, gpu) as shot:
+            assert shot.kernel_name().startswith("step_persist_kernel<0>/tile<")
+            held.append(_pool_used_bytes(gpu) - base)
+            said.append(prob.device_bytes())
+    history = min(n_steps, 256) * 24 * 320 * 4
+    assert history <= held[1] - held[0] <= history + 100_000
+    assert 0 <= said[1] - said[0] - (held[1] - held[0]) + 8192 <= 100_000   # (allocations are rounded up to 512 B each)
+
+
+def test_tracker_allocation_failures(gpu, monkeypatch):
+    """Every allocation of a tracker shot fails in turn: out of memory, or the same
+    rows on a path that needs less."""
+    prob = _tracker_shot(60, 12)
+    st = random_state(None, 500, 300, 10, np.random.default_rng(1))
+
+    def stepped():
+        with F.Shot(prob, gpu) as shot:
+            load_state([shot], st)
+            shot.run(1, 60)
+            return [shot.rc(), shot.traces()["det_ez"], shot.read_field("ez")], shot.kernel_name()
+
+    ref, name = stepped()
+    assert name.startswith("step_persist_kernel<0>/tile<") and ref[0].max() > 0
+    names, in_a_row = set(), 0
+    for k in range(1, 200):
+        monkeypatch.setenv("FDTD2D_TEST_FAIL_ALLOC", str(k))
+        try:
+            got, name = stepped()
+        except F.FdtdError as e:
+            assert e.status == F.ERR_NOMEM, (k, e)
+            in_a_row = 0
+            continue
+        for a, b in zip(ref, got):
+            assert np.array_equal(a, b), (k, name)
+        names.add(name)
+        in_a_row = in_a_row + 1 if name.startswith("step_persist_kernel<0>/tile<") else 0
+        if in_a_row == 3:
+            break
+    assert in_a_row == 3
+    assert any(not n.startswith("step_persist_kernel<0>/tile<") for n in names), names
