@@ -104,7 +104,8 @@ void touch_pages(void* p, size_t bytes) {
 // allocation a context makes reports cudaErrorMemoryAllocation without
 // allocating, so a test can walk every allocation of fdtd2d_create and check
 // that each failure comes back as FDTD2D_ERR_NOMEM with the context's other
-// memory released, or, where the library has a smaller form to fall back to
+// memory released (a batch's add counts its tile list, in host memory, as the one
+// after them), or, where the library has a smaller form to fall back to
 // (the two-step path's extra buffers), that the shot still runs.  Normal runs
 // leave it unset.
 //
@@ -113,7 +114,7 @@ template <class T>
 cudaError_t dalloc_raw(fdtd2d_ctx* c, T** p, size_t count) {
   *p = nullptr;
   if (count == 0) return cudaSuccess;
-  if (c->fail_alloc > 0 && ++c->n_alloc == c->fail_alloc) return cudaErrorMemoryAllocation;
+  if (c->fail_here()) return cudaErrorMemoryAllocation;
   void* q = nullptr;
   // Stream-ordered allocation from the device's pool: a shot's memory is
   // released with cudaFreeAsync behind its last kernel, so retiring a batch

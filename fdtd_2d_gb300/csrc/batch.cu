@@ -11,7 +11,9 @@
 //
 // Host-side state changes (admit, finish, remove) take effect between passes:
 // the tile list is rebuilt on the host and uploaded in the order of the batch's
-// stream before the next pass; nothing waits for the device.
+// stream before the next pass.  Two lists can be on their way: the host waits for
+// the device only when a third change follows while the first one's list is still
+// behind queued passes.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -332,21 +334,30 @@ static int fdtd2d_batch_add_body(fdtd2d_batch* b, const fdtd2d_setup* s, int32_t
   const int rc = create_ctx(s, b->device, true, &c);   // uploads on its own stream
   if (rc) return rc;
   adopt_ctx(c, b->stream);
+  c->h.base_n = b->g;
+  c->h.base_pass = b->passes;
+  // nothing of the batch's changes before all that can fail has been done
   Member& x = b->m[slot];
+  cudaError_t e = cudaSuccess;
+  try {
+    if (c->fail_here()) throw std::bad_alloc();
+    x.tiles = make_tiles(c->h, kBatchShape);
+    b->h_shots[slot] = c->h;
+    cudaSetDevice(b->device);
+    e = cudaMemcpyAsync(b->d_shots + slot, &b->h_shots[slot], sizeof(DevShot), cudaMemcpyHostToDevice, b->stream);
+  } catch (const std::bad_alloc&) {
+    e = cudaErrorMemoryAllocation;
+  }
+  if (e != cudaSuccess) {
+    fdtd2d_destroy(c);
+    return fail(b, e);
+  }
   x.ctx = c;
   x.bytes = bytes;
   x.base = b->g;
   x.live = true;
   x.done = false;
   x.passes = 0;
-  c->h.base_n = b->g;
-  c->h.base_pass = b->passes;
-  x.tiles = make_tiles(c->h, kBatchShape);
-  b->h_shots[slot] = c->h;
-  cudaSetDevice(b->device);
-  cudaError_t e = cudaMemcpyAsync(b->d_shots + slot, &b->h_shots[slot], sizeof(DevShot), cudaMemcpyHostToDevice,
-                                  b->stream);
-  if (e != cudaSuccess) return fail(b, e);
   b->used += bytes;
   b->dirty = true;
   *shot = slot;

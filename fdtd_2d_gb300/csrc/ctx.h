@@ -111,8 +111,9 @@ struct fdtd2d_ctx {
   int line_n = 0, line_i0 = 0, line_j = 0, line_first = 0, line_last = -1;
   float* d_line = nullptr;
   std::vector<void*> allocs;
-  // test parameter: the fail_alloc-th device allocation fails (0: none)
+  // test parameter: the fail_alloc-th allocation fails (0: none)
   int fail_alloc = 0, n_alloc = 0;
+  bool fail_here() { return fail_alloc > 0 && ++n_alloc == fail_alloc; }
 };
 
 namespace fdtd2d {

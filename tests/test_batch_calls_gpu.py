@@ -50,3 +50,42 @@ def test_solo_member_needs_what_it_holds(gpu, monkeypatch, nx, ny, store):
             with pytest.raises(F.FdtdError) as e:
                 srv.submit(p, 6)
             assert e.value.status == F.ERR_BUDGET
+
+
+def test_add_that_fails_leaves_no_member(gpu, monkeypatch):
+    """Every allocation of an add fails in turn (its tile list the last of them): out
+    of memory, nothing charged, no member left that later passes would step; the
+    members before and after it give a single shot's results."""
+    import numpy as np
+
+    probs = [_shot(300, 200), _shot(260, 220)]
+    alone = []
+    for p in probs:
+        with F.Shot(p, gpu) as shot:
+            shot.run(1, 24)
+            alone.append((shot.traces()["det_ez"], shot.dft()))
+    failed = 0
+    with F.Batch(gpu) as b:
+        first = b.add(probs[0])
+        b.run(3)
+        free = b.free_bytes()
+        for k in range(1, 200):
+            monkeypatch.setenv("FDTD2D_TEST_FAIL_ALLOC", str(k))
+            try:
+                i = b.add(probs[1])
+            except F.FdtdError as e:
+                assert e.status == F.ERR_NOMEM, (k, e)
+                assert b.free_bytes() == free, k
+                failed = k
+                continue
+            b.remove(i)
+            break
+        monkeypatch.delenv("FDTD2D_TEST_FAIL_ALLOC")
+        assert failed == k - 1 >= 8
+        second = b.add(probs[1])
+        assert second == first + 1          # the slot of the failed ones
+        b.run(24)
+        b.synchronize()
+        for i, (tr, dft) in zip((first, second), alone):
+            assert b.finished(i)
+            assert np.array_equal(b.shot(i).traces()["det_ez"], tr) and np.array_equal(b.shot(i).dft(), dft)
