@@ -183,11 +183,18 @@ def profile_traffic(kernel: str, cells: int) -> float | None:
     return float(m.group(1)) if m else None
 
 
+def launch_passes(kernel: str, steps: int) -> int:
+    """Passes over the fields of a launch that advances them `steps` time steps:
+    the grid-barrier kernel reads and writes them once per step, every other one
+    (the on-chip kernel and the tile passes too) once per launch."""
+    return steps if kernel.startswith("step_persist") and "/tile<" not in kernel else 1
+
+
 def workload_config(args) -> dict:
     bpc = BYTES_PER_CELL if getattr(args, "storage", "f32") == "f32" else 18
-    touched = bpc * args.size * args.size   # bytes one time step reads and writes
-    l2 = (f"no flush: {touched / 1e9:.2g} GB touched per time step >> 129 MB L2" if touched > 4 * 129e6 else
-          f"no flush: {touched / 1e6:.3g} MB touched per time step, L2-resident (a small-grid case, not the "
+    touched = bpc * args.size * args.size   # bytes one pass over the fields reads and writes
+    l2 = (f"no flush: {touched / 1e9:.2g} GB touched per pass >> 129 MB L2" if touched > 4 * 129e6 else
+          f"no flush: {touched / 1e6:.3g} MB touched per pass, L2-resident (a small-grid case, not the "
           "HBM-bound workload)")
     return {"workload": f"{args.size}x{args.size} TMz phased-array reflectometry shot: 32-cell CPML, "
                         "tanh x GRF plasma, nu 2e9/s, 16 elements at 50 GHz steered 15 deg, 16 Ez "
@@ -455,16 +462,17 @@ def run_precision(args, local: int) -> dict:
                 kt = shot.step_kernel_time()
                 shot.time_step_kernel(False)
                 val = cells * K * S / (ms / 1e3) / 1e9
-                two = kt["steps"] == 2
                 # 16-bit Ez, Hx, Hy, Jz read and written and the drive read once
-                # per launch: 18 B per cell of the launch's region, for the one
-                # or two time steps the launch advances
+                # per pass: 18 B per cell of the launch's region, for all the
+                # time steps the pass advances
+                per_cell = 18 * launch_passes(shot.kernel_name(), kt["steps"])
+                per_update = per_cell / max(kt["steps"], 1)
                 per_launch = kt["ms"] / 1e3 / max(kt["launches"], 1)
-                kgbs = 18 * kt["cells"] / per_launch / 1e9
-                entry.update({"value": val, "unit": UNIT, "bytes_per_cell_update": 9 if two else 18,
-                              "step_rate_gbs": (9 if two else 18) * val,
+                kgbs = per_cell * kt["cells"] / per_launch / 1e9
+                entry.update({"value": val, "unit": UNIT, "bytes_per_cell_update": per_update,
+                              "step_rate_gbs": per_update * val,
                               "interior_kernel": {"achieved_gbs": kgbs, "frac": kgbs / peak,
-                                                  "bytes_per_cell_per_launch": 18, "steps_per_launch": kt["steps"],
+                                                  "bytes_per_cell_per_launch": per_cell, "steps_per_launch": kt["steps"],
                                                   "mean_launch_us": per_launch * 1e6},
                               "ok_finite": shot.check_finite()})
         if store == F.STORE_F32:
@@ -497,8 +505,8 @@ def run_precision(args, local: int) -> dict:
                    "dft_phase_err_rad": phase_err(shot.dft(), o_dft)}
         out.setdefault(name, {})["vs_fp64_oracle_384x320_1500_steps"] = res
     out["note"] = ("F16: Ez, Hx, Hy, Jz and the drive map stored as FP16 with a power-of-two scale per array; "
-                   "BF16 the same without scales; 18 B per cell-update per pass (FP32: 36), 9 (18) when a pass "
-                   "advances two time steps; arithmetic FP32, DFT FP64; errors vs FP32 over the whole "
+                   "BF16 the same without scales; 18 B per cell and pass (FP32: 36), whatever the time steps "
+                   "a pass advances; arithmetic FP32, DFT FP64; errors vs FP32 over the whole "
                    f"{n_err}-step shot")
     return out
 
@@ -591,12 +599,10 @@ def run_ours(args, world, rank, local, dist) -> None:
 
     # roofline of the interior step kernel: algorithmic bytes of one launch
     # (bpc per cell of its region: each field read and written once per
-    # pass, however many time steps a pass advances them; the
-    # persistent kernel's launch makes one pass per step) over its mean
+    # pass, however many time steps a pass advances them) over its mean
     # event-timed launch duration
     per_launch_s = kt["ms"] / 1e3 / max(kt["launches"], 1)
-    passes = kt["steps"] if kernel.startswith("step_persist") else 1
-    alg_bytes = bpc * kt["cells"] * passes
+    alg_bytes = bpc * kt["cells"] * launch_passes(kernel, kt["steps"])
     achieved = alg_bytes / per_launch_s / 1e9
     step_gbs = bpc * cells / ((ms / 1e3) / (K * S)) / 1e9   # bpc per cell-update at the whole-step rate
     peaks = measured_peaks()
@@ -676,7 +682,7 @@ def run_ours(args, world, rank, local, dist) -> None:
                              "step_rate_gbs_at_36_b_per_cell_update": step_gbs,
                              "note": "achieved: the interior kernel alone (event-timed on its stream); "
                                      "step_rate: whole steps at bpc per cell-update, above the copy peak "
-                                     "when a launch advances its cells two steps"},
+                                     "when a launch advances its cells several steps"},
                 "e2e": e2e, "cpu_baseline": cpu, "gpu_launches": int(launches), "clocks": clk,
                 "finite": ok, "precision": precision, "batched": batched, "serving": serving}
         print(json.dumps(line), flush=True)
