@@ -89,3 +89,41 @@ def test_add_that_fails_leaves_no_member(gpu, monkeypatch):
         for i, (tr, dft) in zip((first, second), alone):
             assert b.finished(i)
             assert np.array_equal(b.shot(i).traces()["det_ez"], tr) and np.array_equal(b.shot(i).dft(), dft)
+
+
+def test_batch_of_lossy_and_lossless_shots(gpu):
+    """Members of lossy and lossless media and of different lengths, one with
+    denominators that vary everywhere, so that the passes' kernel changes as members end
+    and join: a single shot's bits."""
+    import numpy as np
+
+    probs = []
+    for k, (nx, ny, n, ca) in enumerate([(300, 200, 37, 1.0), (410, 260, 22, 0.998), (260, 333, 50, 1.0), (390, 180, 64, 0.999)]):
+        p = F.Problem.from_spec(nx=nx, ny=ny, npml=8 + k, n_steps=n, profile=1, x_lo=nx // 2, x_hi=nx - 8, ne_peak=2e19,
+                                src_i=nx // 2, src_j=ny // 2, det_i=nx // 2 + 3, det_j=ny // 2)
+        p.setup.ca = p.setup.da = ca
+        if k == 2:
+            a = np.ctypeslib.as_array(p.setup.den_ey, (ny - 1,))
+            a *= np.random.default_rng(3).uniform(0.8, 1.0, ny - 1).astype(np.float32)
+        probs.append(p)
+    fields = ("ez", "hx", "hy", "jz")
+
+    def outputs(shot):
+        return [shot.traces()["det_ez"], shot.dft()] + [shot.read_field(f) for f in fields]
+
+    alone = []
+    for p in probs:
+        with F.Shot(p, gpu) as shot:
+            shot.run(1, p.n_steps)
+            alone.append(outputs(shot))
+    with F.Batch(gpu) as b:
+        ids = [b.add(p) for p in probs[:3]]
+        b.run(13)
+        ids.append(b.add(probs[3]))
+        for k in (1, 6, 10, 3, 44):
+            b.run(k)
+        b.synchronize()
+        for i, ref in zip(ids, alone):
+            assert b.finished(i)
+            for x, y in zip(outputs(b.shot(i)), ref):
+                assert np.array_equal(x, y)

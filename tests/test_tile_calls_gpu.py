@@ -229,3 +229,93 @@ def test_tracker_allocation_failures(gpu, monkeypatch):
             break
     assert in_a_row == 3
     assert any(not n.startswith("step_persist_kernel<0>/tile<") for n in names), names
+
+
+def _outputs(gpu, prob, st, chunks):
+    with F.Shot(prob, gpu) as shot:
+        load_state([shot], st)
+        first = 1
+        for c in chunks:
+            shot.run(first, first + c - 1)
+            first += c
+        out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+        out["det"], out["dft"] = shot.traces()["det_ez"], shot.dft()
+        if prob.setup.n_rc:
+            out["rc"] = shot.rc()
+        shot.synchronize()
+        return shot.kernel_name(), out
+
+
+def _same(ref, got):
+    for k in ref:
+        assert np.array_equal(ref[k], got[k], equal_nan=np.asarray(ref[k]).dtype.kind in "fc"), k
+
+
+FORMS = [("FDTD2D_TILE", "7"), ("FDTD2D_TILE", "5"), ("FDTD2D_RESIDENT", "2"), ("FDTD2D_RESIDENT", "4"), ("FDTD2D_RESIDENT", "6"),
+         ("FDTD2D_RESIDENT", "8")]
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: f[0][7:] + f[1])
+@pytest.mark.parametrize("nx,ny,P,store,ca", [(700, 300, 9, 0, 1.0), (700, 300, 9, 0, 0.999), (500, 223, 21, 1, 1.0), (390, 180, 4, 2, 0.998)])
+def test_denominators_that_vary(gpu, monkeypatch, form, nx, ny, P, store, ca):
+    """Curl denominators that vary outside the CPML too: no plain tile, every warp in
+    the form with tables, tiles without a strip lane.  The one-row kernel's bits."""
+    if form == ("FDTD2D_RESIDENT", "8") and store:
+        pytest.skip("16-bit fields take at most 6 rows")
+    chunks = (1, 4, 3, 8, 2, 9)
+    n = sum(chunks)
+    prob = F.Problem.from_spec(nx=nx, ny=ny, npml=P, n_steps=n, profile=1, x_lo=nx // 3, x_hi=nx - 3, ne_peak=2e19, nu=3e9,
+                               n_elem=5, src_i=nx // 2 - 6, src_j=ny // 2, src_di=3, src_dj=1, n_det=6, det_i=nx // 2 - 8,
+                               det_j=ny // 2 - 2, det_di=2, det_dj=1, storage=store, field_max=16.0)
+    s = prob.setup
+    s.ca = s.da = ca
+    rng = np.random.default_rng(nx)
+    for name, m in (("den_ex", nx - 1), ("den_hx", nx - 1), ("den_ey", ny - 1), ("den_hy", ny - 1)):
+        a = np.ctypeslib.as_array(getattr(s, name), (m,))
+        a *= rng.uniform(0.8, 1.0, m).astype(np.float32)
+    st = random_state(None, nx, ny, P, rng)
+    monkeypatch.setenv(*form)
+    name, got = _outputs(gpu, prob, st, chunks)
+    assert name.endswith("%s>" % form[1]) and "tile" in name, name
+    monkeypatch.delenv(form[0])
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv("FDTD2D_TMA", "4,3")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = _outputs(gpu, prob, st, (n,))
+    assert name == "step_tma_kernel<4,3>", name
+    _same(ref, got)
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: f[0][7:] + f[1])
+@pytest.mark.parametrize("store,ca,lines", [(0, 1.0, 0), (0, 0.999, 12), (1, 1.0, 0), (2, 0.999, 0)])
+def test_special_values(gpu, monkeypatch, form, store, ca, lines):
+    """NaN, infinities, values near both ends of the range and signed zeros in the
+    fields and in psi, with the tracker reading some: they spread as in the kernels of
+    one step (FP32: the streaming one, which runs the tracker; 16-bit: the one-row one)."""
+    if form == ("FDTD2D_RESIDENT", "8") and store:
+        pytest.skip("16-bit fields take at most 6 rows")
+    chunks = (1, 4, 3, 8, 2, 12)
+    n = sum(chunks)
+    nx, ny, P = 500, 300, 10
+    prob = _tracker_shot(n, lines) if lines else _point_shot(nx, ny, P, n, storage=store, field_max=16.0, profile=1, x_lo=200, x_hi=490,
+                                                             ne_peak=2e19)
+    prob.setup.ca = prob.setup.da = ca
+    rng = np.random.default_rng(7)
+    st = random_state(None, nx, ny, P, rng)
+    for w in FIELDS + PSI_FIELDS:
+        flat = st[w].reshape(-1)
+        at = rng.choice(flat.size, 12, replace=False)
+        flat[at] = np.array([np.nan, np.inf, -np.inf, 3e38, -3e38, 1e-40, -1e-40, 0.0, -0.0, 1e-38, 6e4, -6e4], np.float32)
+    monkeypatch.setenv(*form)
+    name, got = _outputs(gpu, prob, st, chunks)
+    assert name.endswith("%s>" % form[1]) and "tile" in name, name
+    monkeypatch.delenv(form[0])
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv(*(("FDTD2D_KERNEL", "stream") if store == 0 else ("FDTD2D_TMA", "4,3")))
+    name, ref = _outputs(gpu, prob, st, (n,))
+    assert name == ("step_stream_kernel<0>" if store == 0 else "step_tma_kernel<4,3>"), name
+    assert not np.isfinite(ref[F.FIELD_EZ]).all() and np.isfinite(ref[F.FIELD_EZ]).any()
+    if lines:
+        assert ref["rc"].max() > 0
+    _same(ref, got)
