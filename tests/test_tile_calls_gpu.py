@@ -319,3 +319,23 @@ def test_special_values(gpu, monkeypatch, form, store, ca, lines):
     if lines:
         assert ref["rc"].max() > 0
     _same(ref, got)
+
+
+def test_production_shot_on_tiles(gpu, monkeypatch):
+    """The 8192^2 production shot from a random state on the path it takes by default
+    (register tiles, a single step on the tensor kernel among them): the bits of the
+    two-step path, which the production tests hold against the FP64 oracle."""
+    chunks = (9, 1, 12)
+    n = sum(chunks)
+    prob = F.Problem.from_spec(F.production_spec(n_steps=n))
+    st = {}
+    rng = np.random.default_rng(5)
+    for w in FIELDS + PSI_FIELDS:
+        a = rng.standard_normal(F.field_shape(w, prob.nx, prob.ny, prob.setup.npml), dtype=np.float32)
+        st[w] = a * np.float32({F.FIELD_HX: 1 / 377.0, F.FIELD_HY: 1 / 377.0}.get(w, 1.0 if w in FIELDS else 1e-3))
+    name, got = _outputs(gpu, prob, st, chunks)
+    assert name.startswith("step_tmat_kernel<tile,"), name
+    monkeypatch.setenv("FDTD2D_TB", "1")
+    name, ref = _outputs(gpu, prob, st, (n,))
+    assert name.startswith("step_tmat2_kernel<"), name
+    _same(ref, got)
