@@ -2064,7 +2064,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
         c->launches += 3;
       }
       if (e == cudaSuccess && probe && c->step >= c->line_first && c->step <= c->line_last) {
-        e = launch_line(field_ptr(c->h, kEz, c->step & 1), c->pitch, c->line_j, c->line_i0, c->line_n,
+        e = launch_line(c->h, c->step & 1, c->line_j, c->line_i0, c->line_n,
                         c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
         ++c->launches;
       }
@@ -2121,15 +2121,14 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
     }
     if (e != cudaSuccess) return fail_cuda(c, e);
     ++c->launches;
-    const float* ez_now = field_ptr(c->h, kEz, n & 1);
     if (c->n_rc > 0) {
-      e = launch_rc(ez_now, c->pitch, c->ny, c->n_rc, c->d_rc_scan, c->d_rc_max, c->rc_j_cut,
-                    c->rc_level, c->d_edge, c->d_spd + (size_t)(n - 1) * c->n_rc, c->stream);
+      e = launch_rc(c->h, n & 1, c->n_rc, c->d_rc_scan, c->d_rc_max, c->rc_j_cut, c->rc_level, c->d_edge,
+                    c->d_spd + (size_t)(n - 1) * c->n_rc, c->stream);
       if (e != cudaSuccess) return fail_cuda(c, e);
       ++c->launches;
     }
     if (c->line_n > 0 && n >= c->line_first && n <= c->line_last) {
-      e = launch_line(ez_now, c->pitch, c->line_j, c->line_i0, c->line_n,
+      e = launch_line(c->h, n & 1, c->line_j, c->line_i0, c->line_n,
                       c->d_line + (size_t)(n - c->line_first) * c->line_n, c->stream);
       if (e != cudaSuccess) return fail_cuda(c, e);
       ++c->launches;

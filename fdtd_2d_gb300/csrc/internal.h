@@ -339,14 +339,13 @@ cudaError_t build_source_tables(float* src_val, double2* twiddle, const float* e
                                 double scale, double f0, double beta_half, double src_pi,
                                 double dft_fdt, cudaStream_t stream);
 
-// Wave-front tracker for one step: one CTA per line (see fdtd2d_setup.n_rc).
-cudaError_t launch_rc(const float* ez, int64_t pitch, int ny, int n_rc, const int* scan_i,
-                      const int* max_i, int j_cut, float level, float* edge, int* spd_row,
-                      cudaStream_t stream);
+// Wave-front tracker for one step, on Ez of field buffer `buf`: one CTA per line (see
+// fdtd2d_setup.n_rc).
+cudaError_t launch_rc(const DevShot& s, int buf, int n_rc, const int* scan_i, const int* max_i, int j_cut, float level,
+                      float* edge, int* spd_row, cudaStream_t stream);
 
-// Copy n cells of row j starting at column i0 into dst.
-cudaError_t launch_line(const float* ez, int64_t pitch, int j, int i0, int n, float* dst,
-                        cudaStream_t stream);
+// Copy Ez of n cells of row j starting at column i0, of field buffer `buf`, into dst.
+cudaError_t launch_line(const DevShot& s, int buf, int j, int i0, int n, float* dst, cudaStream_t stream);
 
 // Count non-finite values in n floats (atomic count into *flag).
 cudaError_t launch_nonfinite(const float* a, int64_t n, int* flag, cudaStream_t stream);

@@ -526,12 +526,24 @@ cudaError_t build_source_tables(float* src_val, double2* twiddle, const float* e
   return cudaGetLastError();
 }
 
+// The value of a stored element, and a call with a value of the shot's element type.
+__device__ __forceinline__ float stored(float v, float) { return v; }
+template <class T>
+__device__ __forceinline__ float stored(T v, float sc) { return __fmul_rn(static_cast<float>(v), sc); }
+template <class Call>
+void by_store(const DevShot& s, const Call& call) {
+  if (s.store == 0) call(0.f);
+  else if (s.store == 1) call(__half());
+  else call(__nv_bfloat16());
+}
+
 // Dev_RCcalc (FDTD_2D_Full/kernel.cu:968-1044) as one CTA per line.  The
 // reference walks each column serially with one thread (O(ny) dependent
 // loads); here the column max and the downward scan are block reductions.
 // The scan result is the largest j in [1, ny-3] where |Ez| is not below the
 // edge level, which is where the reference's do-while from j = ny-2 stops.
-__global__ void __launch_bounds__(1024) rc_kernel(const float* __restrict__ ez, int64_t pitch, int ny,
+template <class T>
+__global__ void __launch_bounds__(1024) rc_kernel(const T* __restrict__ ez, float sc, int64_t pitch, int ny,
                                                   const int* __restrict__ scan_i, const int* __restrict__ max_i,
                                                   int j_cut, float level, float* __restrict__ edge,
                                                   int* __restrict__ spd_row) {
@@ -541,24 +553,24 @@ __global__ void __launch_bounds__(1024) rc_kernel(const float* __restrict__ ez, 
   __shared__ float s_edge;
   const int l = blockIdx.x;
   const int im = max_i[l], is = scan_i[l];
-  const int tid = threadIdx.x, T = blockDim.x;
-  const int lane = tid & 31, w = tid >> 5, nw = T >> 5;
-  // The scan column's first kPer*T rows are loaded beside the max column, so
+  const int tid = threadIdx.x, threads = blockDim.x;
+  const int lane = tid & 31, w = tid >> 5, nw = threads >> 5;
+  // The scan column's first kPer*threads rows are loaded beside the max column, so
   // both columns' loads are in flight together.
   float sv[kPer];
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
-    const int j = 1 + tid + k * T;
-    sv[k] = j <= ny - 3 ? fabsf(ez[(int64_t)j * pitch + is]) : 0.f;
+    const int j = 1 + tid + k * threads;
+    sv[k] = j <= ny - 3 ? fabsf(stored(ez[(int64_t)j * pitch + is], sc)) : 0.f;
   }
   float m = -INFINITY;
 #pragma unroll 4
-  for (int j = j_cut + tid; j < ny - 2; j += T) m = fmaxf(m, ez[(int64_t)j * pitch + im]);
+  for (int j = j_cut + tid; j < ny - 2; j += threads) m = fmaxf(m, stored(ez[(int64_t)j * pitch + im], sc));
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (lane == 0) s_max[w] = m;
   __syncthreads();
   if (tid == 0) {
-    float temp = ez[im];  // Dev_FindMax starts from row 0
+    float temp = stored(ez[im], sc);  // Dev_FindMax starts from row 0
     for (int k = 0; k < nw; ++k)
       if (s_max[k] > temp) temp = s_max[k];
     const float cand = temp * level;
@@ -572,11 +584,11 @@ __global__ void __launch_bounds__(1024) rc_kernel(const float* __restrict__ ez, 
   int best = 0;
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
-    const int j = 1 + tid + k * T;
+    const int j = 1 + tid + k * threads;
     if (j <= ny - 3 && !(sv[k] < e)) best = max(best, j);
   }
-  for (int j = 1 + tid + kPer * T; j <= ny - 3; j += T)
-    if (!(fabsf(ez[(int64_t)j * pitch + is]) < e)) best = max(best, j);
+  for (int j = 1 + tid + kPer * threads; j <= ny - 3; j += threads)
+    if (!(fabsf(stored(ez[(int64_t)j * pitch + is], sc)) < e)) best = max(best, j);
   for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
   if (lane == 0) s_best[w] = best;
   __syncthreads();
@@ -587,10 +599,13 @@ __global__ void __launch_bounds__(1024) rc_kernel(const float* __restrict__ ez, 
   }
 }
 
-cudaError_t launch_rc(const float* ez, int64_t pitch, int ny, int n_rc, const int* scan_i,
-                      const int* max_i, int j_cut, float level, float* edge, int* spd_row,
-                      cudaStream_t stream) {
-  rc_kernel<<<n_rc, 1024, 0, stream>>>(ez, pitch, ny, scan_i, max_i, j_cut, level, edge, spd_row);
+cudaError_t launch_rc(const DevShot& s, int buf, int n_rc, const int* scan_i, const int* max_i, int j_cut, float level,
+                      float* edge, int* spd_row, cudaStream_t stream) {
+  by_store(s, [&](auto t) {
+    using T = decltype(t);
+    rc_kernel<T><<<n_rc, 1024, 0, stream>>>(field_ptr_t<T>(s, kEz, buf), s.sc[0], s.pitch, s.ny, scan_i, max_i, j_cut, level, edge,
+                                            spd_row);
+  });
   return cudaGetLastError();
 }
 
@@ -673,15 +688,18 @@ cudaError_t launch_rc_steps(const TileAux& A, int ny, int steps, int n_rc, const
   return cudaGetLastError();
 }
 
-__global__ void line_kernel(const float* __restrict__ ez, int64_t pitch, int j, int i0, int n,
+template <class T>
+__global__ void line_kernel(const T* __restrict__ ez, float sc, int64_t pitch, int j, int i0, int n,
                             float* __restrict__ dst) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-    dst[t] = ez[(int64_t)j * pitch + i0 + t];
+    dst[t] = stored(ez[(int64_t)j * pitch + i0 + t], sc);
 }
 
-cudaError_t launch_line(const float* ez, int64_t pitch, int j, int i0, int n, float* dst,
-                        cudaStream_t stream) {
-  line_kernel<<<(n + 255) / 256, 256, 0, stream>>>(ez, pitch, j, i0, n, dst);
+cudaError_t launch_line(const DevShot& s, int buf, int j, int i0, int n, float* dst, cudaStream_t stream) {
+  by_store(s, [&](auto t) {
+    using T = decltype(t);
+    line_kernel<T><<<(n + 255) / 256, 256, 0, stream>>>(field_ptr_t<T>(s, kEz, buf), s.sc[0], s.pitch, j, i0, n, dst);
+  });
   return cudaGetLastError();
 }
 

@@ -339,3 +339,44 @@ def test_production_shot_on_tiles(gpu, monkeypatch):
     name, ref = _outputs(gpu, prob, st, (n,))
     assert name.startswith("step_tmat2_kernel<"), name
     _same(ref, got)
+
+
+@pytest.mark.parametrize("store", [F.STORE_F32, F.STORE_F16, F.STORE_BF16])
+@pytest.mark.parametrize("lines,probe", [(12, None), (0, 150), (12, 299)])
+def test_tracker_and_probe_of_every_storage(gpu, store, lines, probe):
+    """Tracker rows and probe samples against the ones formed from the fields read
+    after every step, in each storage type (one probe on the grid's last row)."""
+    n = 40
+    prob = _tracker_shot(n, lines)
+    s = prob.setup
+    s.storage, s.field_max = store, 16.0
+    if probe is not None:
+        s.line_n, s.line_i0, s.line_j, s.line_first, s.line_last = 300, 50, probe, 11, 31
+    st = random_state(None, 500, 300, 10, np.random.default_rng(1))
+    with F.Shot(prob, gpu) as shot:
+        load_state([shot], st)
+        for a, b in ((1, 9), (10, 12), (13, n)):
+            shot.run(a, b)
+        rows = shot.rc() if lines else None
+        line = shot.line(11, 31) if probe is not None else None
+        ez = shot.read_field("ez")
+    want_rows, want_line = [], []
+    with F.Shot(prob, gpu) as shot:
+        load_state([shot], st)
+        edge = np.full(lines, s.rc_edge0, np.float32)
+        for k in range(1, n + 1):
+            shot.run(k, k)
+            e = shot.read_field("ez")
+            if 11 <= k <= 31 and probe is not None:
+                want_line.append(e[probe, 50:350])
+            if lines:
+                scan, most = prob.keep
+                top = np.maximum(e[0, most], e[s.rc_j_cut:298, most].max(axis=0))
+                edge = np.maximum(edge, top * np.float32(s.rc_level))
+                hit = ~(np.abs(e[1:298, scan]) < edge)
+                want_rows.append(np.where(hit, np.arange(1, 298)[:, None], 0).max(axis=0))
+    assert np.array_equal(ez, e)
+    if lines:
+        assert np.array_equal(rows, np.array(want_rows)) and rows.max() > 0
+    if probe is not None:
+        assert np.array_equal(line, np.array(want_line)) and np.abs(line).max() > 0
