@@ -1152,7 +1152,7 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
   t.dft = nullptr;
   for (int k = 0; k < tile_shape_count(); ++k) {
     if (!timed && k != ch.k) continue;
-    const std::vector<int4> tiles = make_tiles(c->h, k);
+    const std::vector<int4> tiles = make_tiles(c->h, k, c->points);
     int4* d = nullptr;
     e = dalloc(c, &d, tiles.size());
     if (e == cudaSuccess)

@@ -341,7 +341,7 @@ static int fdtd2d_batch_add_body(fdtd2d_batch* b, const fdtd2d_setup* s, int32_t
   cudaError_t e = cudaSuccess;
   try {
     if (c->fail_here()) throw std::bad_alloc();
-    x.tiles = make_tiles(c->h, kBatchShape);
+    x.tiles = make_tiles(c->h, kBatchShape, c->points);
     b->h_shots[slot] = c->h;
     cudaSetDevice(b->device);
     e = cudaMemcpyAsync(b->d_shots + slot, &b->h_shots[slot], sizeof(DevShot), cudaMemcpyHostToDevice, b->stream);

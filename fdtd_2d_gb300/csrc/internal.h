@@ -283,10 +283,11 @@ cudaError_t launch_rc_steps(const TileAux& A, int ny, int steps, int n_rc, const
 // state n_global-1 from fb[0] and psi, writes state n_global-1+steps (steps <=
 // kTileSteps) to fb[1] and psi + psi_buf.  smem: tile_smem of the shot.
 constexpr int kTileSteps = 4;
-enum TileFlags : int { kTilePlain = 1 };   // no CPML and no border in the tile
+enum TileFlags : int { kTilePlain = 1, kTilePoints = 2 };   // no CPML and no border in the tile; sources or detectors
 int tile_shape_count();
 int tile_shape_rows(int shape);   // rows per warp of its plain tiles
-std::vector<int4> make_tiles(const DevShot& s, int shape);
+// points: (column, row, PointKind) of the shot's sources and detectors, by row.
+std::vector<int4> make_tiles(const DevShot& s, int shape, const std::vector<int3>& points);
 size_t tile_smem(const DevShot& s, int shape);
 // aux: null, or what to record (FP32 storage).
 cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,

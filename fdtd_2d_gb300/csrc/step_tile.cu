@@ -84,7 +84,8 @@ __device__ __forceinline__ Part tile_part(const int4& tile, const int4* at, int 
   return {tile.z + (w & 255), tile.z + (w >> 8 & 255), lane >= (w >> 16 & 255) && lane < w >> 24 && in ? 15u : 0u};
 }
 
-template <int R, int NW, bool JS, bool LOSSLESS, bool PLAIN, bool AUX, class T>
+// POINTS: there are sources or detectors in the tile.
+template <int R, int NW, bool JS, bool LOSSLESS, bool PLAIN, bool POINTS, bool AUX, class T>
 __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, const int4 tile, const int4* at, int n, int steps, float4* smem) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int rows = NW * R, threads = NW * 32;
@@ -153,7 +154,7 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
     }
   }
   int p0 = 0, p1 = 0;
-  if (j0 + R > 0 && j0 < ny) {
+  if (POINTS && (tile.x & kTilePoints) && j0 + R > 0 && j0 < ny) {
     p0 = __ldg(S.row_start + max(j0, 0));
     p1 = __ldg(S.row_start + min(j0 + R, ny));
   }
@@ -170,9 +171,9 @@ __device__ __forceinline__ void tile_pass(const DevShot& S, const TileAux& A, co
       get4(s.ez[0], e[(warp > 0 ? 2 * warp - 1 : 0) * 32 + lane]);
       get4(s.ez[R + 1], e[(warp < NW - 1 ? 2 * warp + 2 : 2 * warp + 1) * 32 + lane]);
       tile_step<R, JS, LOSSLESS, decltype(x)::value, decltype(y)::value, T>(s, S, C, p, psi, tc, tr, rows, row0, kps, jzs, threads, lane);
-      if (AUX || p1 > p0) {
+      if (AUX || (POINTS && p1 > p0)) {
         const Part u = tile_part<PLAIN>(tile, at, lane, p.i < nx);
-        if (p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, u.own, u.r0, u.r1);
+        if (POINTS && p1 > p0) tile_points<R, JS, T>(s, S, p, p0, p1, n + t, u.own, u.r0, u.r1, lane);
         if (AUX) tile_record<R, JS>(s, A, slots, p, u.own, u.r0, u.r1, n + t);
       }
       tile_round<R, JS, T>(s);
@@ -213,17 +214,36 @@ struct Tile {
   static constexpr int kRows = RP;
 };
 
+// Plain tiles with points, in FP32 in a function of their own: their code in the
+// kernel took registers of the loop of the plain tiles without any (8192^2 112.8 us per
+// step, 114.4 with it, 126 with the points in the one loop; with 16-bit fields the call
+// is the slower of the two, F16 103.3 against 103.6 and 104.5).
+template <class Shape, bool LOSSLESS, bool AUX, class T>
+__device__ __noinline__ void points_pass(const DevShot& S, const TileAux& A, const int4 tile, const int4* at, int n, int steps, float4* smem) {
+  tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, true, AUX, T>(S, A, tile, at, n, steps, smem);
+}
+
+// A tile in its form.
+template <class Shape, bool LOSSLESS, bool AUX, class T>
+__device__ __forceinline__ void any_tile(const DevShot& S, const TileAux& A, const int4 tile, const int4* at, int n, int steps, float4* smem) {
+  if (!(tile.x & kTilePlain)) {
+    tile_pass<kREdge, kWarps, false, LOSSLESS, false, true, AUX, T>(S, A, tile, at, n, steps, smem);
+  } else if (!(tile.x & kTilePoints)) {
+    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, false, AUX, T>(S, A, tile, at, n, steps, smem);
+  } else if constexpr (sizeof(T) == 4) {
+    points_pass<Shape, LOSSLESS, AUX, T>(S, A, tile, at, n, steps, smem);
+  } else {
+    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, true, AUX, T>(S, A, tile, at, n, steps, smem);
+  }
+}
+
 template <class Shape, bool LOSSLESS, bool AUX, class T>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 step_tmat_kernel(const __grid_constant__ DevShot S, const __grid_constant__ TileAux A, const int4* __restrict__ tiles, int n_global, int steps) {
   extern __shared__ float4 smem[];
   const int4 tile = __ldg(tiles + blockIdx.x);
   const int n = n_global - S.base_n;
-  if (tile.x & kTilePlain) {
-    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, AUX, T>(S, A, tile, tiles + blockIdx.x, n, steps, smem);
-  } else {
-    tile_pass<kREdge, kWarps, false, LOSSLESS, false, AUX, T>(S, A, tile, tiles + blockIdx.x, n, steps, smem);
-  }
+  any_tile<Shape, LOSSLESS, AUX, T>(S, A, tile, tiles + blockIdx.x, n, steps, smem);
 }
 
 // The same for the shots of a batch: the tile's shot from a device array, its
@@ -248,11 +268,7 @@ step_tma_batch_kernel(const DevShot* __restrict__ shots, const int4* __restrict_
   const int n = g + 1 - S.base_n, k = min(steps, S.n_steps - n + 1);
   if (k <= 0) return;
   const TileAux none{};
-  if (tile.x & kTilePlain) {
-    tile_pass<Shape::kRows, kWarps, true, LOSSLESS, true, false, float>(S, none, tile, tiles + blockIdx.x, n, k, smem);
-  } else {
-    tile_pass<kREdge, kWarps, false, LOSSLESS, false, false, float>(S, none, tile, tiles + blockIdx.x, n, k, smem);
-  }
+  any_tile<Shape, LOSSLESS, false, float>(S, none, tile, tiles + blockIdx.x, n, k, smem);
 }
 
 // A launch that may start while the one before it in the stream ends; its tiles
@@ -335,7 +351,7 @@ std::vector<TileColumn> tile_columns(const DevShot& s) {
 // outside took 2 or 3 columns and 4 or 5 rows.  us per step, before and now: 2048^2
 // 10.35 and 9.43 (with 5 rows per warp 10.68 and 9.43), 4096^2 32.1 and 31.3, F16
 // 31.9 and 29.1, 2300 x 1531 BF16 8.43 and 8.07, 8192^2 F16 110 and 104.
-std::vector<int4> make_tiles(const DevShot& s, int shape) {
+std::vector<int4> make_tiles(const DevShot& s, int shape, const std::vector<int3>& points) {
   const int ny = s.ny, P = s.npml, up = kShapes[shape] * kWarps - 2 * kHalo;
   std::vector<int4> edge, plain;
   // plain rows between `top` and `bottom` rows of others: as many as fit, the rest
@@ -369,6 +385,13 @@ std::vector<int4> make_tiles(const DevShot& s, int shape) {
     for (int q = 0; q < n; ++q) plain.push_back(make_int4(kTilePlain, c.c0, top + q * up - kHalo, top + (q + 1) * up));
   }
   edge.insert(edge.end(), plain.begin(), plain.end());
+  // the tiles that hold points, halo included
+  for (int4& t : edge) {
+    const int rows = t.x & kTilePlain ? kShapes[shape] * kWarps : kRowsEdge;
+    auto q = std::lower_bound(points.begin(), points.end(), t.z, [](const int3& p, int row) { return p.y < row; });
+    for (; q != points.end() && q->y < t.z + rows && !(t.x & kTilePoints); ++q)
+      if (q->x >= t.y && q->x < t.y + kTileCols) t.x |= kTilePoints;
+  }
   return edge;
 }
 

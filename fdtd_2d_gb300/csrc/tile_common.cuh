@@ -561,32 +561,52 @@ inline int y_warps(const DevShot& s, int r0, int warps, int R) {
   return n;
 }
 
-// Sources, then detectors, of the thread's rows at step n (points [p0, p1) of
-// the shot's table are those of the warp's rows).  Detectors record in the
-// columns of the mask `own` and rows [u0, u1), the ones this tile answers for.
+// Sources, then detectors, of the warp's rows at step n (points [p0, p1) of the
+// shot's table are those of its rows, a row's sources before its detectors, the
+// sources of a cell in the order in which they are subtracted).  Detectors record in
+// the columns of the mask `own` and rows [u0, u1), the ones this tile answers for.
+//
+// 32 points at a time, one per lane, which loads and stores what belongs to its point
+// (its entry, the source's value, the detector's trace and sum) beside the others; the
+// cells' values come and go by shuffle.  A point at a time, its loads one after
+// another, took 0.1 to 0.4 us a step for each point of a warp's rows.  us per step then
+// and now: 16 sources and detectors along y, 700^2 6.0 and 3.7; 40 along x, 1500^2 30
+// and 8.8; 40 x 40 detectors, 512^2 90 and 7.4; 400 sources along x, 1500^2 75 and 17.
 template <int R, bool JS, class T>
 __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S, const TilePos& p, int p0, int p1, int n,
-                                            unsigned own, int u0, int u1) {
+                                            unsigned own, int u0, int u1, int lane) {
   constexpr bool sc = sizeof(T) == 2;
-  for (int q = p0; q < p1; ++q) {
-    const int4 pt = __ldg(S.pts + q);
-    const int k = pt.x - p.i, r = pt.w - p.j0;
-    if (k < 0 || k > 3) continue;
-    const int at = r * 4 + k;
-    float e = 0.f;
-#pragma unroll
-    for (int t = 0; t < 4 * R; ++t)
-      if (t == at) e = s.ez[t / 4 + 1][t % 4];
-    if (pt.y == kPointSource) {
-      const float v = __ldg(S.src_val + (int64_t)n * S.n_src + pt.z);
-      e = __fsub_rn(e, sc ? __fmul_rn(v, S.isc[0]) : v);
+  const int c0 = p.i - 4 * lane;
+#pragma unroll 1
+  for (int q0 = p0; q0 < p1; q0 += 32) {
+    int4 pt = make_int4(c0 - 1, 0, 0, 0);
+    if (q0 + lane < p1) pt = __ldg(S.pts + q0 + lane);
+    const int x = pt.x - c0;
+    const bool in = x >= 0 && x < kTileCols, src = in && pt.y == kPointSource;
+    if (!__any_sync(kFull, in)) continue;
+    const int at = in ? x >> 2 : 0, slot = (pt.w - p.j0) * 4 + (x & 3);
+    float v = 0.f;
+    if (src) v = __ldg(S.src_val + (int64_t)n * S.n_src + pt.z);
+    if (sc) v = __fmul_rn(v, S.isc[0]);
+    for (unsigned m = __ballot_sync(kFull, src); m; m &= m - 1) {
+      const int k = __ffs(m) - 1;
+      const int owner = __shfl_sync(kFull, at, k), cell = __shfl_sync(kFull, slot, k), to = owner == lane ? cell : -1;
+      const float w = __shfl_sync(kFull, v, k);
 #pragma unroll
       for (int t = 0; t < 4 * R; ++t)
-        if (t == at) s.ez[t / 4 + 1][t % 4] = e;
-    } else if (!(own >> k & 1) || pt.w < u0 || pt.w >= u1) {
-      continue;
-    } else if (pt.y == kPointDetEz) {
-      if (sc) e = __fmul_rn(e, S.sc[0]);
+        if (t == to) s.ez[t / 4 + 1][t % 4] = __fsub_rn(s.ez[t / 4 + 1][t % 4], w);
+    }
+    const unsigned owned = __shfl_sync(kFull, own, at);
+    const bool det = in && !src && pt.w >= u0 && pt.w < u1 && (owned >> (x & 3) & 1);
+    if (!__any_sync(kFull, det)) continue;
+    float e = 0.f;
+#pragma unroll
+    for (int t = 0; t < 4 * R; ++t) {
+      const float z = __shfl_sync(kFull, s.ez[t / 4 + 1][t % 4], at);
+      e = t == slot ? z : e;
+    }
+    if (sc) e = __fmul_rn(e, S.sc[0]);
+    if (det && pt.y == kPointDetEz) {
       if (S.record) S.trace[(int64_t)(n - 1) * S.n_det + pt.z] = e;
       if (S.dft) {
         const double2 tw = __ldg(S.twiddle + n);
@@ -595,15 +615,22 @@ __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S
         acc.y = fma(-(double)e, tw.y, acc.y);
         S.dft[pt.z] = acc;
       }
-    } else if (S.record) {
+    }
+    const bool comp = det && pt.y == kPointDetComp;
+    if (S.record && __any_sync(kFull, comp)) {
       float hxv = 0.f, hyv = 0.f;
 #pragma unroll
-      for (int t = 0; t < 4 * R; ++t)
-        if (t == at) { hxv = s.hx[t / 4 + 1][t % 4]; hyv = s.hy[t / 4][t % 4]; }
-      float* dst = S.ctrace + ((int64_t)(n - 1) * S.n_comp + pt.z) * 3;
-      dst[0] = sc ? __fmul_rn(e, S.sc[0]) : e;
-      dst[1] = sc ? __fmul_rn(hxv, S.sc[1]) : hxv;
-      dst[2] = sc ? __fmul_rn(hyv, S.sc[2]) : hyv;
+      for (int t = 0; t < 4 * R; ++t) {
+        const float a = __shfl_sync(kFull, s.hx[t / 4 + 1][t % 4], at), b = __shfl_sync(kFull, s.hy[t / 4][t % 4], at);
+        hxv = t == slot ? a : hxv;
+        hyv = t == slot ? b : hyv;
+      }
+      if (comp) {
+        float* dst = S.ctrace + ((int64_t)(n - 1) * S.n_comp + pt.z) * 3;
+        dst[0] = e;
+        dst[1] = sc ? __fmul_rn(hxv, S.sc[1]) : hxv;
+        dst[2] = sc ? __fmul_rn(hyv, S.sc[2]) : hyv;
+      }
     }
   }
 }

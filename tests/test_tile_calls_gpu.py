@@ -380,3 +380,59 @@ def test_tracker_and_probe_of_every_storage(gpu, store, lines, probe):
         assert np.array_equal(rows, np.array(want_rows)) and rows.max() > 0
     if probe is not None:
         assert np.array_equal(line, np.array(want_line)) and np.abs(line).max() > 0
+
+
+@pytest.mark.parametrize("form", [("FDTD2D_TILE", "7"), ("FDTD2D_TILE", "5"), ("FDTD2D_RESIDENT", "4")], ids=lambda f: f[0][7:] + f[1])
+@pytest.mark.parametrize("store", [0, 1, 2])
+@pytest.mark.parametrize("kind", ["rows", "block", "cell", "spread", "strips"])
+def test_many_points(gpu, monkeypatch, form, store, kind):
+    """More points than lanes in a warp's rows: lines of sources and detectors along x, a
+    block of detectors, many sources and detectors in one cell (subtracted in their
+    order), points all over the grid, points in the CPML; component detectors beside
+    them.  The one-row kernel's bits."""
+    chunks = (1, 4, 3, 8)
+    n, nx, ny, P = sum(chunks), 420, 300, 12
+    prob = _point_shot(nx, ny, P, n, storage=store, field_max=16.0, profile=1, x_lo=200, x_hi=400, ne_peak=2e19, n_elem=90)
+    s = prob.setup
+    rng = np.random.default_rng(9)
+    at = {"rows": lambda q: (30 + 4 * q % 360, 150 + q % 2), "block": lambda q: (200 + q % 13, 140 + q // 13),
+          "cell": lambda q: (211, 150), "spread": lambda q: (int(rng.integers(1, nx - 1)), int(rng.integers(1, ny - 1))),
+          "strips": lambda q: (1 + q % (P + 3), 1 + q // (P + 3))}[kind]
+
+    def points(count):
+        a = (type(s.det[0]) * count)()
+        for q in range(count):
+            a[q].i, a[q].j = at(q)
+        return a
+
+    prob.keep = src, det, comp = points(s.n_src), points(230), points(70)
+    s.src, s.det, s.comp, s.n_det, s.n_comp = src, det, comp, len(det), len(comp)
+    phase = np.ctypeslib.as_array(s.src_phase_deg, (s.n_src,))
+    phase += rng.uniform(0, 360, s.n_src)   # sources of different values, so that their order shows
+    st = random_state(None, nx, ny, P, rng)
+
+    def stepped(parts):
+        name, out = _outputs(gpu, prob, st, parts)
+        return name, out
+
+    def all_traces(parts):
+        with F.Shot(prob, gpu) as shot:
+            load_state([shot], st)
+            first = 1
+            for c in parts:
+                shot.run(first, first + c - 1)
+                first += c
+            return shot.traces()
+
+    monkeypatch.setenv(*form)
+    name, got = stepped(chunks)
+    got.update(all_traces(chunks))
+    assert "tile" in name, name
+    monkeypatch.delenv(form[0])
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv("FDTD2D_TMA", "4,3")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = stepped((n,))
+    ref.update(all_traces((n,)))
+    assert name == "step_tma_kernel<4,3>", name
+    _same(ref, got)
