@@ -1027,6 +1027,9 @@ cudaError_t make_side(fdtd2d_ctx* c) {
 // 68.0; FP32 4096^2 105 and 109, 5800^2 207 and 212, 3000 x 12000 245 and 234, 8192^2
 // 409 and 385.  (Two steps stay one tile pass: F16 8192^2 167 us per step, where the
 // two-step kernel with its two extra field buffers took 162; everywhere else faster.)
+// Every step of a 16-bit shot of that size whose curl denominators vary outside the CPML
+// goes that way: all its tiles take the form with tables, 4 rows per warp.  BF16 2900^2
+// 42.2 in passes and 44.4, 4096^2 82.2 and 68, 8192^2 311 and 221; FP32 8192^2 272 and 385.
 constexpr int64_t kOneStepCells32 = 35000000, kOneStepCells16 = int64_t(1) << 24;
 
 // Whether a tile shot may take that form.  FDTD2D_ONE_STEP=0 (at create): never;
@@ -2035,7 +2038,9 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
         const bool resident = c->resident && (k >= kResidentSteps || !c->tile);
         k = std::min(k, resident ? kPersistSteps : kTileSteps);
         const TileAux* a = c->aux ? &aux : nullptr;
-        const bool one = k == 1 && !resident && !a && one_step_ready(c);
+        const bool single = k == 1 || (!c->h.den_uniform && c->h.store != FDTD2D_STORE_F32);
+        const bool one = single && !resident && !a && one_step_ready(c);
+        if (one) k = 1;
         cudaEvent_t p0 = one ? nullptr : prof_mark(c, nullptr, 0, k);
         const DevShot t = tile_view(c, n);
         const cudaError_t e =

@@ -436,3 +436,23 @@ def test_many_points(gpu, monkeypatch, form, store, kind):
     ref.update(all_traces((n,)))
     assert name == "step_tma_kernel<4,3>", name
     _same(ref, got)
+
+
+def test_varying_denominators_step_by_step(gpu, monkeypatch):
+    """A 16-bit shot with varying denominators goes a step at a time where single
+    steps have a form of their own; in passes elsewhere.  The same bits."""
+    nx, ny, P, n = 1100, 300, 9, 22
+    prob = _point_shot(nx, ny, P, n, storage=F.STORE_F16, field_max=16.0)
+    a = np.ctypeslib.as_array(prob.setup.den_ey, (ny - 1,))
+    a *= np.random.default_rng(3).uniform(0.8, 1.0, ny - 1).astype(np.float32)
+    st = random_state(None, nx, ny, P, np.random.default_rng(2))
+    monkeypatch.setenv("FDTD2D_TILE", "5")
+    out = []
+    for one in ("0", "1"):
+        monkeypatch.setenv("FDTD2D_ONE_STEP", one)
+        out.append(_outputs(gpu, prob, st, (1, 13, 8))[1])
+        with F.Shot(prob, gpu) as shot:
+            before = shot.launches()
+            shot.run(1, 8)
+            assert shot.launches() - before == (16 if one == "1" else 2)   # two launches a step, one per pass of four
+    _same(*out)
