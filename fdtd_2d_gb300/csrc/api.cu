@@ -2024,20 +2024,24 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
   }
   if (c->tile || on_chip) {
     // launches up to `stop`: until the tracker's history is full, or the line
-    // probe's window opens or closes where the kernels do not record it
+    // probe's window opens or closes where the kernels do not record it.  A single
+    // step records nothing: what it leaves is read from the fields (two launches
+    // less and no scattered columns: us per call, 100 tracker lines at 2048^2 78 and
+    // 41, one line at 500 x 300 21.4 and 16.4).
     for (int32_t n = n_first; n <= n_last;) {
       int32_t stop = n_last + 1;
       const bool probe = c->line_n > 0 && !c->aux;
       if (probe && n <= c->line_last && stop > c->line_first) stop = n < c->line_first ? c->line_first : n + 1;
       if (c->n_rc > 0) stop = (int32_t)std::min<int64_t>(stop, (int64_t)n + c->rc_chunk);
       const int32_t n0 = n;
+      const bool lone = c->tile && stop - n == 1 && (c->n_rc > 0 || one_step_ready(c));
       TileAux aux = c->taux;
       aux.n0 = n0;
       while (n < stop) {
         int k = stop - n;
         const bool resident = c->resident && (k >= kResidentSteps || !c->tile);
         k = std::min(k, resident ? kPersistSteps : kTileSteps);
-        const TileAux* a = c->aux ? &aux : nullptr;
+        const TileAux* a = c->aux && !lone ? &aux : nullptr;
         const bool single = k == 1 || (!c->h.den_uniform && c->h.store != FDTD2D_STORE_F32);
         const bool one = single && !resident && !a && one_step_ready(c);
         if (one) k = 1;
@@ -2063,12 +2067,16 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
         c->step = n - 1;
       }
       cudaError_t e = cudaSuccess;
-      if (c->n_rc > 0) {
+      if (c->n_rc > 0 && lone) {
+        e = launch_rc(c->h, n0 & 1, c->n_rc, c->d_rc_scan, c->d_rc_max, c->rc_j_cut, c->rc_level, c->d_edge,
+                      c->d_spd + (size_t)(n0 - 1) * c->n_rc, c->one_step <= 0, c->stream);
+        ++c->launches;
+      } else if (c->n_rc > 0) {
         e = launch_rc_steps(aux, c->ny, n - n0, c->n_rc, c->d_scan_slot, c->d_max_slot, c->rc_j_cut, c->rc_level, c->d_edge,
                             c->d_cand, c->d_spd + (size_t)(n0 - 1) * c->n_rc, c->stream);
         c->launches += 3;
       }
-      if (e == cudaSuccess && probe && c->step >= c->line_first && c->step <= c->line_last) {
+      if (e == cudaSuccess && (probe || (c->line_n > 0 && lone)) && c->step >= c->line_first && c->step <= c->line_last) {
         e = launch_line(c->h, c->step & 1, c->line_j, c->line_i0, c->line_n,
                         c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
         ++c->launches;
@@ -2128,7 +2136,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
     ++c->launches;
     if (c->n_rc > 0) {
       e = launch_rc(c->h, n & 1, c->n_rc, c->d_rc_scan, c->d_rc_max, c->rc_j_cut, c->rc_level, c->d_edge,
-                    c->d_spd + (size_t)(n - 1) * c->n_rc, c->stream);
+                    c->d_spd + (size_t)(n - 1) * c->n_rc, false, c->stream);
       if (e != cudaSuccess) return fail_cuda(c, e);
       ++c->launches;
     }

@@ -341,9 +341,10 @@ cudaError_t build_source_tables(float* src_val, double2* twiddle, const float* e
                                 double dft_fdt, cudaStream_t stream);
 
 // Wave-front tracker for one step, on Ez of field buffer `buf`: one CTA per line (see
-// fdtd2d_setup.n_rc).
+// fdtd2d_setup.n_rc).  early: the launch may start while the tile pass before it in the
+// stream ends.
 cudaError_t launch_rc(const DevShot& s, int buf, int n_rc, const int* scan_i, const int* max_i, int j_cut, float level,
-                      float* edge, int* spd_row, cudaStream_t stream);
+                      float* edge, int* spd_row, bool early, cudaStream_t stream);
 
 // Copy Ez of n cells of row j starting at column i0, of field buffer `buf`, into dst.
 cudaError_t launch_line(const DevShot& s, int buf, int j, int i0, int n, float* dst, cudaStream_t stream);

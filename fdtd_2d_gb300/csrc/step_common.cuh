@@ -233,4 +233,13 @@ __device__ __forceinline__ void hx_row(const DevShot& S, const MediumRow<MEDIUM>
   }
 }
 
+// Waits until the launches before this one in its stream have ended (this one
+// may have been started beside the last of them) and what they wrote is visible,
+// then lets the next one start.  (After the wait, so that at most two launches
+// overlap.)
+__device__ __forceinline__ void earlier_launches_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 }  // namespace fdtd2d

@@ -537,13 +537,30 @@ void by_store(const DevShot& s, const Call& call) {
   else call(__nv_bfloat16());
 }
 
+// A launch that may start while the one before it in the stream ends, where `early`
+// (its kernel begins with earlier_launches_done and reads what that one wrote by plain
+// pointers: const __restrict__ ones let the compiler read ahead of the wait).
+template <class... P, class... A>
+cudaError_t launch_early(bool early, dim3 grid, int threads, cudaStream_t stream, void (*kernel)(P...), A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Dev_RCcalc (FDTD_2D_Full/kernel.cu:968-1044) as one CTA per line.  The
 // reference walks each column serially with one thread (O(ny) dependent
 // loads); here the column max and the downward scan are block reductions.
 // The scan result is the largest j in [1, ny-3] where |Ez| is not below the
 // edge level, which is where the reference's do-while from j = ny-2 stops.
 template <class T>
-__global__ void __launch_bounds__(1024) rc_kernel(const T* __restrict__ ez, float sc, int64_t pitch, int ny,
+__global__ void __launch_bounds__(1024) rc_kernel(const T* ez, float sc, int64_t pitch, int ny,
                                                   const int* __restrict__ scan_i, const int* __restrict__ max_i,
                                                   int j_cut, float level, float* __restrict__ edge,
                                                   int* __restrict__ spd_row) {
@@ -553,6 +570,7 @@ __global__ void __launch_bounds__(1024) rc_kernel(const T* __restrict__ ez, floa
   __shared__ float s_edge;
   const int l = blockIdx.x;
   const int im = max_i[l], is = scan_i[l];
+  earlier_launches_done();
   const int tid = threadIdx.x, threads = blockDim.x;
   const int lane = tid & 31, w = tid >> 5, nw = threads >> 5;
   // The scan column's first kPer*threads rows are loaded beside the max column, so
@@ -600,13 +618,14 @@ __global__ void __launch_bounds__(1024) rc_kernel(const T* __restrict__ ez, floa
 }
 
 cudaError_t launch_rc(const DevShot& s, int buf, int n_rc, const int* scan_i, const int* max_i, int j_cut, float level,
-                      float* edge, int* spd_row, cudaStream_t stream) {
+                      float* edge, int* spd_row, bool early, cudaStream_t stream) {
+  cudaError_t e = cudaSuccess;
   by_store(s, [&](auto t) {
     using T = decltype(t);
-    rc_kernel<T><<<n_rc, 1024, 0, stream>>>(field_ptr_t<T>(s, kEz, buf), s.sc[0], s.pitch, s.ny, scan_i, max_i, j_cut, level, edge,
-                                            spd_row);
+    e = launch_early(early, dim3(n_rc), 1024, stream, rc_kernel<T>, field_ptr_t<T>(s, kEz, buf), s.sc[0], s.pitch, s.ny, scan_i, max_i,
+                     j_cut, level, edge, spd_row);
   });
-  return cudaGetLastError();
+  return e;
 }
 
 // The tracker over many steps at once, from the columns the tile kernels
@@ -619,6 +638,7 @@ __global__ void __launch_bounds__(256) rc_max_steps_kernel(const TileAux A, int 
   __shared__ float s_max[8];
   const int l = blockIdx.x, t = blockIdx.y, tid = threadIdx.x;
   const float* col = A.hist + ((int64_t)t * A.n_cols + max_slot[l]) * A.rows;
+  earlier_launches_done();
   float m = -INFINITY;
 #pragma unroll 4
   for (int j = j_cut + tid; j < ny - 2; j += 256) m = fmaxf(m, col[j]);
@@ -633,11 +653,12 @@ __global__ void __launch_bounds__(256) rc_max_steps_kernel(const TileAux A, int 
   }
 }
 __global__ void __launch_bounds__(256) rc_scan_steps_kernel(const TileAux A, int ny, const int* __restrict__ scan_slot,
-                                                            const float* __restrict__ cand, const float* __restrict__ edge,
+                                                            const float* cand, const float* edge,
                                                             int* __restrict__ spd) {
   __shared__ float s_max[8];
   __shared__ int s_best[8];
   const int l = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, n_rc = gridDim.x;
+  earlier_launches_done();
   float e = edge[l];
   for (int q = tid; q <= t; q += 256) {
     const float c = cand[q * n_rc + l];
@@ -664,7 +685,8 @@ __global__ void __launch_bounds__(256) rc_scan_steps_kernel(const TileAux A, int
     spd[t * n_rc + l] = best;
   }
 }
-__global__ void rc_edge_steps_kernel(const float* __restrict__ cand, int steps, int n_rc, float* edge) {
+__global__ void rc_edge_steps_kernel(const float* cand, int steps, int n_rc, float* edge) {
+  earlier_launches_done();
   for (int l = threadIdx.x >> 5; l < n_rc; l += blockDim.x >> 5) {
     float e = edge[l];
     for (int q = threadIdx.x & 31; q < steps; q += 32) {
@@ -682,10 +704,10 @@ __global__ void rc_edge_steps_kernel(const float* __restrict__ cand, int steps, 
 cudaError_t launch_rc_steps(const TileAux& A, int ny, int steps, int n_rc, const int* scan_slot, const int* max_slot,
                             int j_cut, float level, float* edge, float* cand, int* spd, cudaStream_t stream) {
   const dim3 grid(n_rc, steps);
-  rc_max_steps_kernel<<<grid, 256, 0, stream>>>(A, ny, max_slot, j_cut, level, cand);
-  rc_scan_steps_kernel<<<grid, 256, 0, stream>>>(A, ny, scan_slot, cand, edge, spd);
-  rc_edge_steps_kernel<<<1, 1024, 0, stream>>>(cand, steps, n_rc, edge);
-  return cudaGetLastError();
+  cudaError_t e = launch_early(true, grid, 256, stream, rc_max_steps_kernel, A, ny, max_slot, j_cut, level, cand);
+  if (e == cudaSuccess) e = launch_early(true, grid, 256, stream, rc_scan_steps_kernel, A, ny, scan_slot, cand, edge, spd);
+  if (e == cudaSuccess) e = launch_early(true, dim3(1), 1024, stream, rc_edge_steps_kernel, cand, steps, n_rc, edge);
+  return e;
 }
 
 template <class T>

@@ -45,15 +45,6 @@ constexpr int kRowsEdge = kREdge * kWarps;
 constexpr int kShapes[] = {7, 5};
 constexpr int kNumShapes = 2;
 
-// Waits until the launches before this one in its stream have ended (this one
-// may have been started beside the last of them) and what they wrote is visible,
-// then lets the next one start.  (After the wait, so that at most two launches
-// overlap.)
-__device__ __forceinline__ void earlier_launches_done() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // Four elements (not by the read-only path, whose loads the compiler may
 // move up across the wait above).
 template <class T>

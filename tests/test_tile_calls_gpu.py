@@ -456,3 +456,42 @@ def test_varying_denominators_step_by_step(gpu, monkeypatch):
             shot.run(1, 8)
             assert shot.launches() - before == (16 if one == "1" else 2)   # two launches a step, one per pass of four
     _same(*out)
+
+
+@pytest.mark.parametrize("one", ["0", "1"])
+def test_single_steps_of_a_tracker_shot(gpu, monkeypatch, one):
+    """Run calls of one step, whose tracker rows and probe samples come from the fields,
+    between longer ones, whose history the passes keep; on the tiles and on the form
+    for single steps.  The streaming kernel's rows, samples and fields."""
+    nx, ny, P, n = 900, 300, 10, 60
+    prob = _point_shot(nx, ny, P, n)
+    s = prob.setup
+    scan = np.arange(100, 100 + 37 * 20, 37, dtype=np.int32)
+    prob.keep = scan, scan[::-1].copy()
+    s.n_rc, s.rc_level, s.rc_j_cut, s.rc_edge0 = 20, 0.07, 40, 1e-3
+    s.rc_scan_i, s.rc_max_i = (a.ctypes.data_as(type(s.rc_scan_i)) for a in prob.keep)
+    s.line_n, s.line_i0, s.line_j, s.line_first, s.line_last = 500, 50, 140, 3, 40
+    st = random_state(None, nx, ny, P, np.random.default_rng(4))
+
+    def stepped(chunks):
+        with F.Shot(prob, gpu) as shot:
+            load_state([shot], st)
+            first = 1
+            for c in chunks:
+                shot.run(first, first + c - 1)
+                first += c
+            out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+            out["rc"], out["line"], out["det"] = shot.rc(), shot.line(3, 40), shot.traces()["det_ez"]
+            return shot.kernel_name(), out
+
+    monkeypatch.setenv("FDTD2D_TILE", "7")
+    monkeypatch.setenv("FDTD2D_ONE_STEP", one)
+    name, got = stepped((1, 1, 1, 4, 1, 9, 1, 20, 1, 1, 17, 3))
+    assert name == "step_tmat_kernel<tile,7>", name
+    monkeypatch.delenv("FDTD2D_TILE")
+    monkeypatch.setenv("FDTD2D_KERNEL", "stream")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = stepped((n,))
+    assert name == "step_stream_kernel<0>", name
+    assert ref["rc"].max() > 0
+    _same(ref, got)
