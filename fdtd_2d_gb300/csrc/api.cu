@@ -950,11 +950,12 @@ void setup_resident(fdtd2d_ctx* c, int device) {
 
 // The tracker and the line probe on the tile paths (FP32): the kernels record
 // the tracked columns of every step (a history of up to 64 MB) and the probe's
-// row.  False when they cannot (16-bit storage, too many columns, a probe on the
-// last row, which no tile stores); an allocation that fails is no error.
+// row (not the last one, which no step changes: run_body copies it).  False when they
+// cannot (16-bit storage, too many columns); an allocation that fails is no error.
 bool setup_aux(fdtd2d_ctx* c, const fdtd2d_setup* s) {
-  if (c->n_rc == 0 && c->line_n == 0) return true;
-  if (c->h.store != FDTD2D_STORE_F32 || (c->line_n > 0 && c->line_j >= c->ny - 1)) return false;
+  const bool line = c->line_n > 0 && !c->line_still;
+  if (c->n_rc == 0 && !line) return true;
+  if (c->h.store != FDTD2D_STORE_F32) return false;
   TileAux a{};
   if (c->n_rc > 0) {
     const RcHistory history = rc_history(s);
@@ -984,7 +985,7 @@ bool setup_aux(fdtd2d_ctx* c, const fdtd2d_setup* s) {
     c->d_scan_slot = d + a.n_cols;
     c->d_max_slot = c->d_scan_slot + c->n_rc;
   }
-  if (c->line_n > 0) {
+  if (line) {
     a.line_n = c->line_n;
     a.line_j = c->line_j;
     a.line_i0 = c->line_i0;
@@ -1851,6 +1852,7 @@ int fdtd2d::create_ctx(const fdtd2d_setup* s, int device, bool member, fdtd2d_ct
   if (s->line_n > 0) {
     c->line_n = s->line_n; c->line_i0 = s->line_i0; c->line_j = s->line_j;
     c->line_first = s->line_first; c->line_last = s->line_last;
+    c->line_still = s->line_j == ny - 1;
     CK(dalloc(c, &c->d_line, (size_t)(s->line_last - s->line_first + 1) * s->line_n));
   }
 
@@ -2030,7 +2032,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
     // 41, one line at 500 x 300 21.4 and 16.4).
     for (int32_t n = n_first; n <= n_last;) {
       int32_t stop = n_last + 1;
-      const bool probe = c->line_n > 0 && !c->aux;
+      const bool line = c->line_n > 0 && !c->line_still, probe = line && !c->aux;
       if (probe && n <= c->line_last && stop > c->line_first) stop = n < c->line_first ? c->line_first : n + 1;
       if (c->n_rc > 0) stop = (int32_t)std::min<int64_t>(stop, (int64_t)n + c->rc_chunk);
       const int32_t n0 = n;
@@ -2076,9 +2078,11 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
                             c->d_cand, c->d_spd + (size_t)(n0 - 1) * c->n_rc, c->stream);
         c->launches += 3;
       }
-      if (e == cudaSuccess && (probe || (c->line_n > 0 && lone)) && c->step >= c->line_first && c->step <= c->line_last) {
-        e = launch_line(c->h, c->step & 1, c->line_j, c->line_i0, c->line_n,
-                        c->d_line + (size_t)(c->step - c->line_first) * c->line_n, c->stream);
+      // the probe's rows of the steps just made: of the last one, or all alike
+      const int32_t l0 = c->line_still ? std::max(n0, c->line_first) : c->step, l1 = std::min(c->step, c->line_last);
+      if (e == cudaSuccess && (c->line_still || probe || (line && lone)) && l0 >= c->line_first && l0 <= l1) {
+        e = launch_line(c->h, c->step & 1, c->line_j, c->line_i0, c->line_n, l1 - l0 + 1,
+                        c->d_line + (size_t)(l0 - c->line_first) * c->line_n, c->stream);
         ++c->launches;
       }
       if (e != cudaSuccess) return fail_cuda(c, e);
@@ -2141,7 +2145,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
       ++c->launches;
     }
     if (c->line_n > 0 && n >= c->line_first && n <= c->line_last) {
-      e = launch_line(c->h, n & 1, c->line_j, c->line_i0, c->line_n,
+      e = launch_line(c->h, n & 1, c->line_j, c->line_i0, c->line_n, 1,
                       c->d_line + (size_t)(n - c->line_first) * c->line_n, c->stream);
       if (e != cudaSuccess) return fail_cuda(c, e);
       ++c->launches;

@@ -109,6 +109,7 @@ struct fdtd2d_ctx {
   int *d_rc_scan = nullptr, *d_rc_max = nullptr, *d_spd = nullptr;
   float* d_edge = nullptr;
   int line_n = 0, line_i0 = 0, line_j = 0, line_first = 0, line_last = -1;
+  bool line_still = false;   // on the last row, which no step changes
   float* d_line = nullptr;
   std::vector<void*> allocs;
   // test parameter: the fail_alloc-th allocation fails (0: none)

@@ -346,8 +346,9 @@ cudaError_t build_source_tables(float* src_val, double2* twiddle, const float* e
 cudaError_t launch_rc(const DevShot& s, int buf, int n_rc, const int* scan_i, const int* max_i, int j_cut, float level,
                       float* edge, int* spd_row, bool early, cudaStream_t stream);
 
-// Copy Ez of n cells of row j starting at column i0, of field buffer `buf`, into dst.
-cudaError_t launch_line(const DevShot& s, int buf, int j, int i0, int n, float* dst, cudaStream_t stream);
+// Copy Ez of n cells of row j starting at column i0, of field buffer `buf`, into each of
+// `rows` rows of dst.
+cudaError_t launch_line(const DevShot& s, int buf, int j, int i0, int n, int rows, float* dst, cudaStream_t stream);
 
 // Count non-finite values in n floats (atomic count into *flag).
 cudaError_t launch_nonfinite(const float* a, int64_t n, int* flag, cudaStream_t stream);

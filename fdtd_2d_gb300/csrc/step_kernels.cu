@@ -711,16 +711,19 @@ cudaError_t launch_rc_steps(const TileAux& A, int ny, int steps, int n_rc, const
 }
 
 template <class T>
-__global__ void line_kernel(const T* __restrict__ ez, float sc, int64_t pitch, int j, int i0, int n,
+__global__ void line_kernel(const T* __restrict__ ez, float sc, int64_t pitch, int j, int i0, int n, int rows,
                             float* __restrict__ dst) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-    dst[t] = stored(ez[(int64_t)j * pitch + i0 + t], sc);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const float v = stored(ez[(int64_t)j * pitch + i0 + t], sc);
+    for (int r = blockIdx.y; r < rows; r += gridDim.y) dst[(int64_t)r * n + t] = v;
+  }
 }
 
-cudaError_t launch_line(const DevShot& s, int buf, int j, int i0, int n, float* dst, cudaStream_t stream) {
+cudaError_t launch_line(const DevShot& s, int buf, int j, int i0, int n, int rows, float* dst, cudaStream_t stream) {
   by_store(s, [&](auto t) {
     using T = decltype(t);
-    line_kernel<T><<<(n + 255) / 256, 256, 0, stream>>>(field_ptr_t<T>(s, kEz, buf), s.sc[0], s.pitch, j, i0, n, dst);
+    line_kernel<T><<<dim3((n + 255) / 256, std::min(rows, 1024)), 256, 0, stream>>>(field_ptr_t<T>(s, kEz, buf), s.sc[0], s.pitch,
+                                                                                    j, i0, n, rows, dst);
   });
   return cudaGetLastError();
 }
