@@ -1118,7 +1118,8 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
     if (env && std::atoi(env) == tile_shape_rows(k)) forced = k;
   if (!setup_aux(c, s) && c->n_rc > 0) return FDTD2D_OK;   // (the probe alone: single steps in its window)
   setup_resident(c, device);
-  const ChoiceKey key = choice_key(c, device, "tile");
+  c->tile_few = tile_few(c->h, c->points);
+  const ChoiceKey key = choice_key(c, device, c->tile_few ? "tile" : "tile many");
   KernelChoice ch;
   // (a resident shot's tiles serve its short run calls only: not timed)
   bool have = forced < 0 && !c->resident && find_choice(key, &ch) && ch.k >= 0 && ch.k < tile_shape_count();
@@ -1170,7 +1171,7 @@ int setup_tile(fdtd2d_ctx* c, const fdtd2d_setup* s, int device) {
       for (int r = 0; r <= reps && e == cudaSuccess; ++r) {
         if (r == 1) e = cudaEventRecord(e0, c->stream);
         if (e == cudaSuccess)
-          e = launch_step_tile(k, t, d, (int)tiles.size(), smem, t.base_n + 1, steps, nullptr, c->stream);
+          e = launch_step_tile(k, c->tile_few, t, d, (int)tiles.size(), smem, t.base_n + 1, steps, nullptr, c->stream);
       }
       if (e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
       if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -2054,7 +2055,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
             : resident ? launch_ordered(c, [&] {
               return launch_resident(t, c->rplan, n, k, a, c->d_link, c->d_err, c->wait_ns, c->bar_extra, c->stream);
             })
-                     : launch_step_tile(c->tile_shape, t, c->d_tiles, c->n_tiles, c->tile_smem, n, k, a, c->stream);
+                     : launch_step_tile(c->tile_shape, c->tile_few, t, c->d_tiles, c->n_tiles, c->tile_smem, n, k, a, c->stream);
         if (p0) prof_mark(c, p0, (int64_t)c->nx * c->ny, k);
         if (e != cudaSuccess) return fail_cuda(c, e);
         ++c->launches;

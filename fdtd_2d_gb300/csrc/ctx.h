@@ -69,6 +69,7 @@ struct fdtd2d_ctx {
   int bar_extra = 0;
   // several steps per pass on register tiles (step_tile.cu)
   bool tile = false;
+  bool tile_few = false;      // by the kernel for few points
   int tile_shape = 0, n_tiles = 0;
   size_t tile_smem = 0;
   int4* d_tiles = nullptr;

@@ -289,8 +289,11 @@ int tile_shape_rows(int shape);   // rows per warp of its plain tiles
 // points: (column, row, PointKind) of the shot's sources and detectors, by row.
 std::vector<int4> make_tiles(const DevShot& s, int shape, const std::vector<int3>& points);
 size_t tile_smem(const DevShot& s, int shape);
-// aux: null, or what to record (FP32 storage).
-cudaError_t launch_step_tile(int shape, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
+// Whether the shot's kernel is the one for few points.
+bool tile_few(const DevShot& s, const std::vector<int3>& points);
+const void* tile_kernel_few(int shape, bool lossless, bool aux);   // (step_tile_few.cu)
+// few: tile_few's answer.  aux: null, or what to record (FP32 storage).
+cudaError_t launch_step_tile(int shape, bool few, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
                              int steps, const TileAux* aux, cudaStream_t stream);
 // A pass of a batch: every shot in `shots` (FP32) by up to `steps` steps after
 // global step g, shot s by its own steps g + 1 - base_n on, at most to its last

@@ -585,8 +585,17 @@ __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S
     const bool in = x >= 0 && x < kTileCols, src = in && pt.y == kPointSource;
     if (!__any_sync(kFull, in)) continue;
     const int at = in ? x >> 2 : 0, slot = (pt.w - p.j0) * 4 + (x & 3);
+    const unsigned owned = __shfl_sync(kFull, own, at);
+    const bool det = in && !src && pt.w >= u0 && pt.w < u1 && (owned >> (x & 3) & 1);
+    const bool sum = det && pt.y == kPointDetEz && S.dft;
+    // everything the points need from memory is asked for together
     float v = 0.f;
+    double2 tw = make_double2(0., 0.), acc = tw;
     if (src) v = __ldg(S.src_val + (int64_t)n * S.n_src + pt.z);
+    if (sum) {
+      tw = __ldg(S.twiddle + n);
+      acc = S.dft[pt.z];
+    }
     if (sc) v = __fmul_rn(v, S.isc[0]);
     for (unsigned m = __ballot_sync(kFull, src); m; m &= m - 1) {
       const int k = __ffs(m) - 1;
@@ -596,8 +605,6 @@ __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S
       for (int t = 0; t < 4 * R; ++t)
         if (t == to) s.ez[t / 4 + 1][t % 4] = __fsub_rn(s.ez[t / 4 + 1][t % 4], w);
     }
-    const unsigned owned = __shfl_sync(kFull, own, at);
-    const bool det = in && !src && pt.w >= u0 && pt.w < u1 && (owned >> (x & 3) & 1);
     if (!__any_sync(kFull, det)) continue;
     float e = 0.f;
 #pragma unroll
@@ -606,15 +613,11 @@ __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S
       e = t == slot ? z : e;
     }
     if (sc) e = __fmul_rn(e, S.sc[0]);
-    if (det && pt.y == kPointDetEz) {
-      if (S.record) S.trace[(int64_t)(n - 1) * S.n_det + pt.z] = e;
-      if (S.dft) {
-        const double2 tw = __ldg(S.twiddle + n);
-        double2 acc = S.dft[pt.z];
-        acc.x = fma((double)e, tw.x, acc.x);
-        acc.y = fma(-(double)e, tw.y, acc.y);
-        S.dft[pt.z] = acc;
-      }
+    if (det && pt.y == kPointDetEz && S.record) S.trace[(int64_t)(n - 1) * S.n_det + pt.z] = e;
+    if (sum) {
+      acc.x = fma((double)e, tw.x, acc.x);
+      acc.y = fma(-(double)e, tw.y, acc.y);
+      S.dft[pt.z] = acc;
     }
     const bool comp = det && pt.y == kPointDetComp;
     if (S.record && __any_sync(kFull, comp)) {
@@ -631,6 +634,52 @@ __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S
         dst[1] = sc ? __fmul_rn(hxv, S.sc[1]) : hxv;
         dst[2] = sc ? __fmul_rn(hyv, S.sc[2]) : hyv;
       }
+    }
+  }
+}
+
+// The same, a point at a time by the thread that holds its cell: its loads wait for one
+// another, but the tiles without points keep more of their registers (tile_few).
+template <int R, bool JS, class T>
+__device__ __forceinline__ void tile_few_points(TileRegs<R, JS>& s, const DevShot& S, const TilePos& p, int p0, int p1, int n,
+                                            unsigned own, int u0, int u1) {
+  constexpr bool sc = sizeof(T) == 2;
+  for (int q = p0; q < p1; ++q) {
+    const int4 pt = __ldg(S.pts + q);
+    const int k = pt.x - p.i, r = pt.w - p.j0;
+    if (k < 0 || k > 3) continue;
+    const int at = r * 4 + k;
+    float e = 0.f;
+#pragma unroll
+    for (int t = 0; t < 4 * R; ++t)
+      if (t == at) e = s.ez[t / 4 + 1][t % 4];
+    if (pt.y == kPointSource) {
+      const float v = __ldg(S.src_val + (int64_t)n * S.n_src + pt.z);
+      e = __fsub_rn(e, sc ? __fmul_rn(v, S.isc[0]) : v);
+#pragma unroll
+      for (int t = 0; t < 4 * R; ++t)
+        if (t == at) s.ez[t / 4 + 1][t % 4] = e;
+    } else if (!(own >> k & 1) || pt.w < u0 || pt.w >= u1) {
+      continue;
+    } else if (pt.y == kPointDetEz) {
+      if (sc) e = __fmul_rn(e, S.sc[0]);
+      if (S.record) S.trace[(int64_t)(n - 1) * S.n_det + pt.z] = e;
+      if (S.dft) {
+        const double2 tw = __ldg(S.twiddle + n);
+        double2 acc = S.dft[pt.z];
+        acc.x = fma((double)e, tw.x, acc.x);
+        acc.y = fma(-(double)e, tw.y, acc.y);
+        S.dft[pt.z] = acc;
+      }
+    } else if (S.record) {
+      float hxv = 0.f, hyv = 0.f;
+#pragma unroll
+      for (int t = 0; t < 4 * R; ++t)
+        if (t == at) { hxv = s.hx[t / 4 + 1][t % 4]; hyv = s.hy[t / 4][t % 4]; }
+      float* dst = S.ctrace + ((int64_t)(n - 1) * S.n_comp + pt.z) * 3;
+      dst[0] = sc ? __fmul_rn(e, S.sc[0]) : e;
+      dst[1] = sc ? __fmul_rn(hxv, S.sc[1]) : hxv;
+      dst[2] = sc ? __fmul_rn(hyv, S.sc[2]) : hyv;
     }
   }
 }

@@ -495,3 +495,54 @@ def test_single_steps_of_a_tracker_shot(gpu, monkeypatch, one):
     assert name == "step_stream_kernel<0>", name
     assert ref["rc"].max() > 0
     _same(ref, got)
+
+
+@pytest.mark.parametrize("rows", ["7", "5"])
+@pytest.mark.parametrize("lines,ca", [(0, 1.0), (0, 0.999), (12, 1.0), (12, 0.998)])
+def test_few_points(gpu, monkeypatch, rows, lines, ca):
+    """A source, a detector and a component detector every 16 rows, in plain tiles, on
+    their borders and in the CPML: the kernel for few points gives the streaming one's
+    bits, with the tracker and without."""
+    chunks = (1, 4, 3, 8)
+    n, nx, ny, P = sum(chunks), 500, 300, 10
+    prob = _tracker_shot(n, lines)
+    s = prob.setup
+    s.ca = s.da = ca
+    count = 18
+
+    def points(i0):
+        a = (type(s.det[0]) * count)()
+        for q in range(count):
+            a[q].i, a[q].j = (i0 + 27 * q) % (nx - 2) + 1, 3 + 16 * q
+        return a
+
+    src = points(60)
+    phase, prob.keep2 = np.random.default_rng(1).uniform(0, 360, count), [src]
+    s.src, s.n_src, s.src_phase_deg = src, count, phase.ctypes.data_as(type(s.src_phase_deg))
+    s.det, s.n_det = prob.keep2.append(points(60)) or prob.keep2[-1], count
+    s.comp, s.n_comp = prob.keep2.append(points(61)) or prob.keep2[-1], count
+    st = random_state(None, nx, ny, P, np.random.default_rng(3))
+
+    def stepped(parts):
+        with F.Shot(prob, gpu) as shot:
+            load_state([shot], st)
+            first = 1
+            for c in parts:
+                shot.run(first, first + c - 1)
+                first += c
+            out = {w: shot.read_field(w) for w in FIELDS + PSI_FIELDS}
+            out.update(shot.traces())
+            out["dft"] = shot.dft()
+            if lines:
+                out["rc"] = shot.rc()
+            return shot.kernel_name(), out
+
+    monkeypatch.setenv("FDTD2D_TILE", rows)
+    name, got = stepped(chunks)
+    assert name == f"step_tmat_kernel<tile,{rows}>", name
+    monkeypatch.delenv("FDTD2D_TILE")
+    monkeypatch.setenv("FDTD2D_KERNEL", "stream")
+    monkeypatch.setenv("FDTD2D_PERSIST", "0")
+    name, ref = stepped((n,))
+    assert name == "step_stream_kernel<0>", name
+    _same(ref, got)
