@@ -137,8 +137,10 @@ void gaussian_random_field(std::vector<float>& g, int nx, int ny, double corr, u
   }
   std::vector<float> tmp((size_t)wx * ny);
   // Each output sums k[d] * input over d = 0 .. 2R in that order; the loops
-  // run d outside and the columns inside (contiguous, vectorisable), one
+  // run d outside and the columns inside (contiguous, vectorised), one
   // accumulator per column, which keeps every output's order of additions.
+  // (Not vectorised, their time depended on where the linker put them: 777 x 1301
+  // 11.3 or 17.7 ms on 16 Arm cores.)
   // pass 1: along y
 #pragma omp parallel
   {
@@ -149,7 +151,9 @@ void gaussian_random_field(std::vector<float>& g, int nx, int ny, double corr, u
       for (int d = 0; d <= 2 * R; ++d) {
         const double kd = k[(size_t)d];
         const float* src = &w[(size_t)(j + d) * wx];
-        for (int i = 0; i < wx; ++i) acc[(size_t)i] += kd * src[i];
+        double* to = acc.data();
+#pragma omp simd
+        for (int i = 0; i < wx; ++i) to[i] += kd * src[i];
       }
       for (int i = 0; i < wx; ++i) tmp[(size_t)j * wx + i] = (float)acc[(size_t)i];
     }
@@ -165,7 +169,9 @@ void gaussian_random_field(std::vector<float>& g, int nx, int ny, double corr, u
       const float* row = &tmp[(size_t)j * wx];
       for (int d = 0; d <= 2 * R; ++d) {
         const double kd = k[(size_t)d];
-        for (int i = 0; i < nx; ++i) acc[(size_t)i] += kd * row[i + d];
+        double* to = acc.data();
+#pragma omp simd
+        for (int i = 0; i < nx; ++i) to[i] += kd * row[i + d];
       }
       for (int i = 0; i < nx; ++i) g[(size_t)j * nx + i] = (float)(acc[(size_t)i] * norm);
     }
