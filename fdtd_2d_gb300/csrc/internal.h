@@ -291,7 +291,7 @@ std::vector<int4> make_tiles(const DevShot& s, int shape, const std::vector<int3
 size_t tile_smem(const DevShot& s, int shape);
 // Whether the shot's kernel is the one for few points.
 bool tile_few(const DevShot& s, const std::vector<int3>& points);
-const void* tile_kernel_few(int shape, bool lossless, bool aux);   // (step_tile_few.cu)
+const void* tile_kernel_few(int shape, int store, bool lossless, bool aux);   // (step_tile_few.cu)
 // few: tile_few's answer.  aux: null, or what to record (FP32 storage).
 cudaError_t launch_step_tile(int shape, bool few, const DevShot& shot, const int4* tiles, int n_tiles, size_t smem, int n_global,
                              int steps, const TileAux* aux, cudaStream_t stream);

@@ -95,7 +95,7 @@ const void* tile_kernel(const DevShot& s, bool aux) {
        : s.store == 1 ? tile_kernel<RP, false, __half>(s) : tile_kernel<RP, false, __nv_bfloat16>(s);
 }
 const void* tile_kernel(int shape, bool few, const DevShot& s, bool aux) {
-  if (few) return tile_kernel_few(shape, lossless(s), aux);
+  if (few) return tile_kernel_few(shape, s.store, lossless(s), aux);
   return shape == 0 ? tile_kernel<kShapes[0]>(s, aux) : tile_kernel<kShapes[1]>(s, aux);
 }
 
@@ -226,10 +226,11 @@ cudaError_t allow_smem(const void* fn) {
 // FP32 shots with at most 4 points in any 8 rows of 128 columns (an array of sources
 // and detectors every 5 rows along y): us per step with tile_few_points and tile_points,
 // 1400^2 5.16 and 5.30, 2048^2 9.51 and 9.73, 8192^2 113.7 and 114.5; an array with an
-// element in every row 2048^2 9.98 and 9.74.  16-bit shots go by tile_points always:
-// 2300 x 1531 BF16 8.07 and 7.7, 4096^2 F16 29.7 and 29.7, 8192^2 F16 103.8 and 104.5.
+// element in every row 2048^2 9.98 and 9.74.  F16 shots too from 4e7 cells on (3300^2
+// 20.7 and 20.7, 5000^2 41.9 and 41.7, 8192^2 104.2 and 104.9), BF16 ones never (4096^2
+// 31.5 and 30.9 at the better shape, 8192^2 110.1 and 109.9).
 bool tile_few(const DevShot& s, const std::vector<int3>& points) {
-  if (s.store != 0) return false;
+  if (s.store == 2 || (s.store == 1 && (int64_t)s.nx * s.ny < 40000000)) return false;
   std::map<std::pair<int, int>, int> blocks;
   for (const int3& p : points)
     if (++blocks[{p.y / 8, p.x / kTileCols}] > 4) return false;

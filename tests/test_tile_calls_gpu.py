@@ -546,3 +546,23 @@ def test_few_points(gpu, monkeypatch, rows, lines, ca):
     name, ref = stepped((n,))
     assert name == "step_stream_kernel<0>", name
     _same(ref, got)
+
+
+def test_few_points_f16_large(gpu, monkeypatch):
+    """The F16 kernel for few points, which the largest grids take: the one-row
+    kernel's bits."""
+    nx, ny, n = 8000, 5010, 9
+    prob = _point_shot(nx, ny, 20, n, storage=F.STORE_F16, field_max=16.0, profile=1, x_lo=nx // 2, x_hi=nx - 20, ne_peak=2e19)
+    rng = np.random.default_rng(6)
+    st = {w: rng.standard_normal(F.field_shape(w, nx, ny, 20), dtype=np.float32) for w in FIELDS}
+    st[F.FIELD_HX] /= np.float32(377)
+    st[F.FIELD_HY] /= np.float32(377)
+    monkeypatch.setenv("FDTD2D_TILE", "7")
+    name, got = _outputs(gpu, prob, st, (4, 2, 3))
+    assert name == "step_tmat_kernel<tile,7>", name
+    monkeypatch.delenv("FDTD2D_TILE")
+    monkeypatch.setenv("FDTD2D_TMAT", "0")
+    monkeypatch.setenv("FDTD2D_TMA", "4,3")
+    name, ref = _outputs(gpu, prob, st, (n,))
+    assert name == "step_tma_kernel<4,3>", name
+    _same(ref, got)
