@@ -351,8 +351,8 @@ int validate(const fdtd2d_setup* s) {
 
 // Steps from which a run call loads the shot on chip.  (Loading and storing it, and
 // starting the launch, take ~15 us at 512^2 and ~30 at 1024^2: us per step in calls of
-// 8 / 9 / 12 steps 3.8 / 3.5 / 3.1 and 6.3 / 6.0 / 5.2, in tile passes of four 3.6 and
-// 4.6; 500 x 3000 with a tracker 11.3 / 10.5 / 9.0 and 16.1.  So grids near the largest
+// 8 / 9 / 12 steps 3.8 / 3.6 / 3.1 and 6.2 / 5.9 / 5.1, in tile passes of four 3.6 and
+// 4.6; 500 x 3000 with a tracker 10.4 / 9.8 / 8.4 and 10.6.  So grids near the largest
 // that fit gain from about 20 steps on only.)
 constexpr int kResidentSteps = 8;
 
@@ -2030,7 +2030,7 @@ static int run_body(fdtd2d_ctx* c, int32_t n_first, int32_t n_last) {
     // probe's window opens or closes where the kernels do not record it.  A single
     // step records nothing: what it leaves is read from the fields (two launches
     // less and no scattered columns: us per call, 100 tracker lines at 2048^2 78 and
-    // 41, one line at 500 x 300 21.4 and 16.4).
+    // 39, one line at 500 x 300 21.4 and 12.8).
     for (int32_t n = n_first; n <= n_last;) {
       int32_t stop = n_last + 1;
       const bool line = c->line_n > 0 && !c->line_still, probe = line && !c->aux;

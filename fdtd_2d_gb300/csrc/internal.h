@@ -303,10 +303,10 @@ cudaError_t launch_step_tile(int shape, bool few, const DevShot& shot, const int
 constexpr int kTileSlot = 8;
 // Shape of the members' plain tiles: 5 rows per warp, which spill less than 7 in
 // this kernel and leave a smaller last wave.  us per step of n members with 5 / 7
-// rows: 60 of 512^2 55.0 / 56.1, 4 of 700^2 6.6 / 7.0, 40 of 1024^2 108.5 / 111.9, 1
-// of 1440^2 5.9 / 6.5, 24 of 1440^2 (50 M cells; members stay below 2^21 each) 114.5 /
-// 118.9, 40 of 512 to 1440 cells a side 103.7 / 108.0.  A single grid of such a size is
-// better with 7 (4096^2 31.4 / 33.7): its CPML tiles are few, a batch's are a third.
+// rows: 60 of 512^2 53.8 / 54.2, 4 of 700^2 6.4 / 7.0, 40 of 1024^2 106.0 / 107.4, 1
+// of 1440^2 5.7 / 6.2, 24 of 1440^2 (50 M cells; members stay below 2^21 each) 112.4 /
+// 113.4, 40 of 512 to 1440 cells a side 101.9 / 103.5.  A single grid of such a size is
+// better with 7 (4096^2 33.1 / 31.4): its CPML tiles are few, a batch's are a third.
 constexpr int kBatchShape = 1;
 cudaError_t launch_batch_tile(bool lossless, const DevShot* shots, const int4* tiles, int n_tiles, size_t smem,
                               int g, int steps, int pass, cudaStream_t stream);
