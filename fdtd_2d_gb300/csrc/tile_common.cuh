@@ -571,7 +571,7 @@ inline int y_warps(const DevShot& s, int r0, int warps, int R) {
 // cells' values come and go by shuffle.  A point at a time, its loads one after
 // another, took 0.1 to 0.4 us a step for each point of a warp's rows.  us per step then
 // and now: 16 sources and detectors along y, 700^2 6.0 and 3.7; 40 along x, 1500^2 30
-// and 8.8; 40 x 40 detectors, 512^2 90 and 7.4; 400 sources along x, 1500^2 75 and 17.
+// and 9.0; 40 x 40 detectors, 512^2 90 and 8.3; 400 sources along x, 1500^2 75 and 17.
 template <int R, bool JS, class T>
 __device__ __forceinline__ void tile_points(TileRegs<R, JS>& s, const DevShot& S, const TilePos& p, int p0, int p1, int n,
                                             unsigned own, int u0, int u1, int lane) {
